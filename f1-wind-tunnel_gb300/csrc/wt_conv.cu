@@ -2,23 +2,19 @@
 // 5th-generation tensor cores (tcgen05, kind::f16 with BF16 operands, FP32
 // accumulation in tensor memory).
 //
-// One kernel, three operand gathers:
 //   FWD    D[m][co]        = sum_k A[m][k] B[co][k],  A[m][(t,ci)]  = x[m + off(t)][ci],  B = w[co][(t,ci)]
 //   DGRAD  D[m][ci]        = sum_k A[m][k] B[ci][k],  A[m][(t,co)]  = dy[m - off(t)][co], B = wt[ci][(t,co)]
 //   WGRAD  D[(t,ci)][co]   = sum_m A[(t,ci)][m] B[co][m], A = x[m + off(t)][ci], B = dy[m][co]
 // (m a voxel of the batch's grid, out-of-grid neighbours read as zero).
 //
-// CTA: 128 threads, a 128 x N tile (N <= 128).  The K dimension runs in
-// slices of 64 through two shared-memory stages: all threads gather a slice of
-// A (128 rows) and B (N rows) into the canonical K-major, non-swizzled
-// core-matrix layout (8 rows x 16 bytes per core matrix; core matrices adjacent
-// along K 128 B apart, along M/N 1024 B apart), one thread issues four
-// tcgen05.mma (K = 16 each) and commits them to the stage's mbarrier, and the
-// next slice is gathered into the other stage meanwhile.  The accumulator
-// (128 lanes x N FP32 columns) lives in tensor memory; the epilogue reads it
-// with tcgen05.ld (warp w owns lanes 32w..32w+31).  Every mbarrier wait is
-// bounded: on expiry the kernel raises g_conv_error, still waits (bounded) for
-// its own MMAs, frees its tensor memory and returns.
+// FWD and DGRAD (conv_rows_kernel): a block holds one input tile with its halo in
+// shared memory and runs all 27 taps on it; a tap is a shift of the matrix
+// descriptor's start address, so every input value is fetched once per tile
+// instead of once per tap.  WGRAD (conv_gemm_kernel) gathers K slices.
+// The accumulators live in tensor memory; the epilogues read them with
+// tcgen05.ld (warp w owns lanes 32w..32w+31).  Every mbarrier wait is bounded:
+// on expiry the kernel raises g_conv_error, still waits (bounded) for its own
+// MMAs, frees its tensor memory and returns.
 #include <atomic>
 #include <cuda_bf16.h>
 #include <stdint.h>
@@ -337,6 +333,344 @@ __global__ void __launch_bounds__(NTHREADS, 1) conv_gemm_kernel(GemmArgs p) {
   }
 }
 
+// ---------------------------------------------------------------------------
+// FWD / DGRAD: the input tile with its halo stays in shared memory for all taps.
+//
+// Rows.  The grid's (batch item, z, y) rows are numbered in one sequence with a
+// zero row after each plane and a zero plane after each batch item, so that a
+// tap's dz and dy are one fixed distance in that numbering and out-of-grid
+// neighbours fall on zeros.  A block computes 16 such rows by 8 XG voxels along x:
+// XG matrix tiles of M = 128 (16 rows x 8 voxels), N = nt output channels each.
+// Shared memory holds, per group of 8 input channels (a plane), nrows x W voxels
+// of 16 bytes: 8 voxels along x are one core matrix (128 B contiguous), the 16
+// rows of a tile are the M groups (stride = row pitch), the planes the K groups.
+// A tap only moves the descriptor's start address (by 16 B along x, by rows along
+// y and z).  The rows a tile needs are either one run (short planes) or three
+// bands, one per dz.
+//
+// Measured, the network's 12 distinct layers at batch 16 / 1 (us in all): forward
+// 1675 -> 395 / 782 -> 144 (launch-bound), data gradient 1530 -> 394, against the
+// gather of 27 x the input per tile; the deepest chain (K = 3456, 72 voxels) 166 ->
+// 17.  What bounds it now: an MMA of M 128 with N 16 takes 39 cycles (64 with N
+// 128), so the narrow layers use a few per cent of the tensor pipe, and the halo
+// (3.4 x the input at 24 x 24 planes).
+//
+// K order is the gather's: taps in order, channels in order, 16 per MMA, so the
+// sums have the same bits whatever the tiling.  A channel count of 8 puts two taps
+// in one MMA (FWD); other odd plane counts, and DGRAD with 8, pair their last plane
+// with a plane of zeros.  Weights come in stages of `ups` MMAs of K through a ring of
+// D stages (cp.async).
+struct RowArgs {
+  const __nv_bfloat16* a;  // FWD x, DGRAD dy
+  const __nv_bfloat16* b;  // FWD w, DGRAD wt: [N][taps][C]
+  const float* bias;
+  void* out;               // FWD bf16 y[M][N], DGRAD f32 dx[M][N]
+  uint32_t C, N, K, taps;  // input channels, output channels, taps * C
+  uint32_t d, h, w, M;     // grid (one batch item) and voxels in all
+  uint32_t hp, dp, rows;   // rows per plane and planes per item with their zero row / plane; rows in all
+  uint32_t cg, planes;     // channel groups; planes in shared memory (the last one zero if cg is odd)
+  uint32_t W, nrows, pitch;  // shared-memory tile: voxels per row, rows, bytes per plane
+  uint32_t halo, run;      // 1 for 27 taps; 1 when the rows are one run
+  uint32_t band0, zstep;   // shared-memory row of tile row 0 for dz = -1, and from one dz to the next
+  uint32_t ctiles;         // tiles along x
+  uint32_t nt, units, ups, upt;  // N per block; MMAs of K; MMAs per stage; MMAs per tap where K is padded per tap, else 0
+  uint32_t depth;            // stages in the weight ring
+  uint32_t cg_magic;       // ceil(2^16 / cg)
+  int relu, vec;           // vec: out is 16-byte aligned and N a multiple of 8
+  uint32_t stage_wait;
+};
+
+constexpr uint32_t ROW_TILE = 16, ROW_ROWS = 3 * (ROW_TILE + 2), ROW_HEAD = 512;  // ROW_HEAD: barriers, slot, ROW_ROWS row voxels
+// Bytes of the head and of the MMAs' tables.
+__host__ __device__ constexpr uint32_t row_tables(uint32_t units) { return (ROW_HEAD + (units + 3) / 4 * 4 * 12 + 127) / 128 * 128; }
+
+__device__ __forceinline__ void cp16(uint32_t dst, const void* src, bool ok) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16u : 0u) : "memory");
+}
+// Voxel index of x position 0 of numbered row R, or -1 for a zero row.
+__device__ __forceinline__ int32_t row_voxel(const RowArgs& p, int64_t R) {
+  if (R < 0 || R >= (int64_t)p.rows) return -1;
+  const uint32_t r = (uint32_t)R, q = r / p.hp, y = r - q * p.hp, b = q / p.dp, z = q - b * p.dp;
+  if (y >= p.h || z >= p.d) return -1;
+  return (int32_t)(((b * p.d + z) * p.h + y) * p.w);  // fewer than 2^31 voxels (+ a row's padding: checked on the host)
+}
+
+// Threads: eight warps load (and later run the epilogue), a ninth issues the MMAs.
+// Stage st of the weights goes to ring slot st % depth once the MMAs of stage
+// st - depth are done (done[slot], committed by the issuing lane); full[slot]
+// completes when its copies have landed, and the issuing warp makes them visible to
+// the tensor cores.  At most two stages of MMAs are in flight.
+constexpr uint32_t ROW_LOADERS = 256, ROW_THREADS = ROW_LOADERS + 32, ROW_DEPTH_MAX = 16;
+
+// mbar_wait that also ends when the block has been told to stop.
+__device__ __forceinline__ bool mbar_wait_or(uint32_t bar, uint32_t parity, const volatile uint32_t* stop) {
+  if (mbar_wait(bar, parity, 1)) return true;
+  for (uint32_t i = 0; i < WAIT_LIMIT && !*stop; i += 16)
+    if (mbar_wait(bar, parity, 16)) return true;
+  return false;
+}
+
+__device__ __forceinline__ void mma_bf16(uint32_t tmem, uint64_t ad, uint64_t bd, uint32_t idesc, uint32_t acc) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
+      "l"(ad), "l"(bd), "r"(idesc), "r"(acc)
+      : "memory");
+}
+
+template <int MODE, int XG>
+__global__ void __launch_bounds__(ROW_THREADS) conv_rows_kernel(RowArgs p) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  // barriers, the tensor-memory slot and the stop flag; the voxel of each tile row;
+  // the MMAs' input descriptors (low words) and weight columns; the input planes;
+  // the weight ring
+  uint64_t* const full = reinterpret_cast<uint64_t*>(smem);
+  uint64_t* const done = full + ROW_DEPTH_MAX;
+  uint32_t* const tmem_slot = reinterpret_cast<uint32_t*>(smem + 256);
+  uint32_t* const stop = tmem_slot + 1;
+  int32_t* const rowvox = reinterpret_cast<int32_t*>(smem + 272);
+  uint32_t* const adesc = reinterpret_cast<uint32_t*>(smem + ROW_HEAD);
+  const uint32_t units4 = (p.units + 3) & ~3u;
+  int32_t* const kcol = reinterpret_cast<int32_t*>(adesc + units4);
+  const uint32_t sa_ofs = row_tables(p.units);
+  const uint32_t sa = smem_u32(smem) + sa_ofs, sb = sa + p.planes * p.pitch;
+  const uint32_t t = threadIdx.x, warp = __shfl_sync(0xffffffffu, t >> 5, 0), lane = t & 31u;
+  const uint32_t x0 = (blockIdx.x % p.ctiles) * XG * 8u, r0 = (blockIdx.x / p.ctiles) * ROW_TILE;
+  const uint32_t n0 = blockIdx.y * p.nt;
+  const uint32_t nst = (p.units + p.ups - 1) / p.ups, depth = p.depth;
+  const uint32_t rowp = p.W * 16u, blbo = p.nt * 16u + 16u, stage_bytes = 2u * p.ups * blbo;
+  const uint32_t cols = XG * p.nt <= 32 ? 32u : XG * p.nt <= 64 ? 64u : XG * p.nt <= 128 ? 128u : XG * p.nt <= 256 ? 256u : 512u;
+  const uint32_t groups = min((uint32_t)XG, (p.w - x0 + 7u) / 8u);
+
+  if (t < p.nrows) {
+    int64_t R;
+    if (p.run) R = (int64_t)r0 - (p.band0 + p.zstep) + t;
+    else R = (int64_t)r0 + ((int64_t)(t / (ROW_TILE + 2)) - 1) * p.hp + (t % (ROW_TILE + 2)) - 1;
+    rowvox[t] = row_voxel(p, R);
+  }
+  if (warp == ROW_LOADERS / 32) {
+    if (lane == 0) {
+      for (uint32_t i = 0; i < depth; i++) {
+        mbar_init(smem_u32(&full[i]), ROW_LOADERS);
+        mbar_init(smem_u32(&done[i]), 1);
+      }
+      *stop = 0u;
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncwarp();
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(cols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  } else if (p.planes > p.cg) {
+    for (uint32_t i = t * 16u; i < p.pitch; i += ROW_LOADERS * 16u)
+      *reinterpret_cast<uint4*>(smem + sa_ofs + p.cg * p.pitch + i) = make_uint4(0u, 0u, 0u, 0u);
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  // per MMA: its input descriptor's low word (start address, K stride) and the weight
+  // columns of its two K halves (-1: zeros)
+  for (uint32_t u = t; u < p.units; u += ROW_THREADS) {
+    uint32_t tap, g = 0, lbo = p.pitch;
+    int32_t k0 = (int32_t)(16u * u), k1 = k0 + 8;
+    if (p.upt) {
+      tap = u / p.upt;
+      g = 2u * (u - tap * p.upt);
+      k0 = (int32_t)((tap * p.cg + g) * 8u);
+      k1 = g + 1 < p.cg ? k0 + 8 : -1;
+    } else if (p.cg == 1) {
+      tap = 2u * u;
+    } else {
+      tap = u / (p.cg >> 1);
+      g = 2u * (u - tap * (p.cg >> 1));
+    }
+    auto tap_off = [&](uint32_t tp) -> uint32_t {
+      const int sg = (MODE == FWD) ? 1 : -1;
+      const int dz = sg * tap_dz(tp, p.taps), dy = sg * tap_dy(tp, p.taps), dx = sg * tap_dx(tp, p.taps);
+      return (p.band0 + (uint32_t)(dz + (int)p.halo) * p.zstep + (uint32_t)dy) * rowp + (uint32_t)((int)p.halo + dx) * 16u;
+    };
+    const uint32_t off = tap_off(tap);
+    if (!p.upt && p.cg == 1 && tap + 1 < p.taps) lbo = tap_off(tap + 1) - off;
+    adesc[u] = ((sa + g * p.pitch + off) >> 4) | ((lbo >> 4) << 16);
+    kcol[2 * u] = k0;
+    kcol[2 * u + 1] = k1 < (int32_t)p.K ? k1 : -1;
+  }
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *tmem_slot;
+
+  bool ok = true;
+  if (warp == ROW_LOADERS / 32) {
+    // One elected lane issues from unrolled code on tabulated descriptors: an MMA then
+    // takes its own 39 (N 16) to 64 (N 128) cycles.  (With the taps' arithmetic or a
+    // loop over the x groups between the MMAs, each took 160-260.)
+    const uint32_t idesc = idesc_bf16(BM, p.nt);
+    const uint64_t ahi = (uint64_t)((rowp >> 4) | (1u << 14)) << 32, bhi = (uint64_t)((128u >> 4) | (1u << 14)) << 32;
+    uint32_t elected;
+    asm volatile("{\n .reg .pred q;\n elect.sync _|q, 0xffffffff;\n selp.u32 %0, 1, 0, q;\n}\n" : "=r"(elected));
+    uint32_t slot = 0, phase = 0, tslot = 0, tphase = 0;  // tslot, tphase: of stage kt - 2
+    for (uint32_t kt = 0; kt < nst; kt++) {
+      if (kt >= 2) {  // MMAs of stage kt-2 done
+        ok = mbar_wait(smem_u32(&done[tslot]), tphase, p.stage_wait);
+        if (++tslot == depth) {
+          tslot = 0;
+          tphase ^= 1u;
+        }
+      }
+      ok = ok && mbar_wait_or(smem_u32(&full[slot]), phase, stop);
+      if (!__all_sync(0xffffffffu, ok)) {
+        ok = false;
+        if (elected) *reinterpret_cast<volatile uint32_t*>(stop) = 1u;
+        // the MMAs issued so far still end before the tensor memory is freed
+        if (kt > 0) {
+          const uint32_t last = slot ? slot - 1 : depth - 1;
+          mbar_wait(smem_u32(&done[last]), slot ? phase : phase ^ 1u, WAIT_LIMIT);
+        }
+        break;
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      if (elected) {
+        const uint32_t u0 = kt * p.ups, u1 = min(p.units, u0 + p.ups), bstep = 2u * blbo >> 4;
+        uint32_t blo = ((sb + slot * stage_bytes) >> 4) | ((blbo >> 4) << 16);
+        for (uint32_t u = u0; u < u1; u += 4) {
+          const uint4 a4 = *reinterpret_cast<const uint4*>(adesc + u);
+          const uint32_t al[4] = {a4.x, a4.y, a4.z, a4.w};
+#pragma unroll
+          for (uint32_t i = 0; i < 4; i++) {
+            if (i == 0 || u + i < u1) {
+              const uint64_t ad = ahi | al[i], bd = bhi | (blo + i * bstep);
+#pragma unroll
+              for (uint32_t xg = 0; xg < XG; xg++)  // x groups past the grid: their columns are not read
+                mma_bf16(tmem + xg * p.nt, ad + xg * 8u, bd, idesc, u + i);
+            }
+          }
+          blo += 4u * bstep;
+        }
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                         smem_u32(&done[slot]))
+                     : "memory");
+      }
+      __syncwarp();
+      if (++slot == depth) {
+        slot = 0;
+        phase ^= 1u;
+      }
+    }
+    if (ok) {
+      const uint32_t last = slot ? slot - 1 : depth - 1;
+      ok = mbar_wait(smem_u32(&done[last]), slot ? phase : phase ^ 1u, WAIT_LIMIT);
+    }
+  } else {
+    // the input tile: 16-byte chunks, channels fastest
+    const uint32_t per_row = p.W * p.cg, q = ROW_LOADERS / per_row, rem = ROW_LOADERS - q * per_row;
+    uint32_t r = t / per_row, e = t - r * per_row;
+#pragma unroll 4
+    for (uint32_t i = t; i < p.nrows * per_row; i += ROW_LOADERS) {
+      const int32_t v0 = rowvox[r];
+      const uint32_t xx = (e * p.cg_magic) >> 16, g = e - xx * p.cg;
+      const uint32_t x = x0 + xx - p.halo;  // wraps below 0: past the grid
+      const bool in = v0 >= 0 && x < p.w && (uint32_t)v0 + x < p.M;
+      cp16(sa + g * p.pitch + (r * p.W + xx) * 16u, in ? p.a + (size_t)((uint32_t)v0 + x) * p.C + g * 8u : p.a, in);
+      r += q;
+      e += rem;
+      if (e >= per_row) {
+        e -= per_row;
+        r++;
+      }
+    }
+    // Weights: thread t copies K half t & (halves - 1) of every stage for its rows.
+    const uint32_t halves = 2u * p.ups, hf = t & (halves - 1u), nstep = ROW_LOADERS / halves;  // halves: 8, 16 or 32
+    const uint32_t dst0 = sb + hf * blbo;
+    uint32_t slot = 0, phase = 1;
+    for (uint32_t st = 0; st < nst; st++) {
+      if (st >= depth && !mbar_wait_or(smem_u32(&done[slot]), phase, stop)) {
+        *reinterpret_cast<volatile uint32_t*>(stop) = 1u;
+        ok = false;
+        break;
+      }
+      const uint32_t u2 = st * halves + hf;
+      const int32_t k = u2 < 2u * p.units ? kcol[u2] : -1;
+      const __nv_bfloat16* const src = p.b + (size_t)n0 * p.K + (k < 0 ? 0 : k);
+      for (uint32_t n = t / halves; n < p.nt; n += nstep) {
+        const bool in = k >= 0 && n0 + n < p.N;
+        cp16(dst0 + slot * stage_bytes + n * 16u, in ? src + (size_t)n * p.K : p.b, in);
+      }
+      // arrives once all copies of this thread so far (with stage 0, the input tile's too) have landed
+      asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&full[slot])) : "memory");
+      if (++slot == depth) {
+        slot = 0;
+        phase ^= 1u;
+      }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+  }
+  __syncwarp();
+  ok = __syncthreads_and(ok);
+  if (!ok && t == 0) atomicExch(&g_conv_error, 1);
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+
+  // ---- epilogue: lane = voxel (t & 7) of row (t & 127) >> 3 of the tile, 16 columns
+  // per tcgen05.ld; the two halves of the loading warps take them in turn
+  if (ok && warp < ROW_LOADERS / 32) {
+    const uint32_t row = r0 + ((t & 127u) >> 3), taddr = tmem + (((warp & 3u) * 32u) << 16);
+    const int32_t v0 = row_voxel(p, row);
+    const uint32_t per = p.nt / 16u, total = groups * per;
+    for (uint32_t c = warp >> 2; c < total; c += 2) {
+      __syncwarp();
+      const uint32_t xg = c / per, c0 = 16u * (c - xg * per), x = x0 + 8u * xg + (t & 7u);
+      uint32_t r[16];
+      asm volatile(
+          "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+          : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+            "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+          : "r"(taddr + xg * p.nt + c0)
+          : "memory");
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      if (v0 < 0 || x >= p.w || (uint32_t)v0 + x >= p.M) continue;
+      const size_t o = (size_t)((uint32_t)v0 + x) * p.N;
+#pragma unroll
+      for (int hh = 0; hh < 2; hh++) {  // 8 columns at a time
+        const uint32_t col = n0 + c0 + 8u * hh;
+        if (col >= p.N) break;  // N is a multiple of 8
+        if constexpr (MODE == FWD) {
+          __nv_bfloat16 v[8];
+#pragma unroll
+          for (int j = 0; j < 8; j++) {
+            float f = __uint_as_float(r[8 * hh + j]);
+            if (p.bias) f += __ldg(p.bias + col + j);
+            if (p.relu) f = fmaxf(f, 0.0f);
+            v[j] = __float2bfloat16_rn(f);
+          }
+          __nv_bfloat16* const y = reinterpret_cast<__nv_bfloat16*>(p.out) + o + col;
+          if (p.vec) {
+            uint4 w;
+            memcpy(&w, v, 16);
+            *reinterpret_cast<uint4*>(y) = w;
+          } else {
+#pragma unroll
+            for (int j = 0; j < 8; j++) y[j] = v[j];
+          }
+        } else {
+          float* const dx = reinterpret_cast<float*>(p.out) + o + col;
+          if (p.vec) {
+            *reinterpret_cast<uint4*>(dx) = make_uint4(r[8 * hh], r[8 * hh + 1], r[8 * hh + 2], r[8 * hh + 3]);
+            *reinterpret_cast<uint4*>(dx + 4) = make_uint4(r[8 * hh + 4], r[8 * hh + 5], r[8 * hh + 6], r[8 * hh + 7]);
+          } else {
+#pragma unroll
+            for (int j = 0; j < 8; j++) dx[j] = __uint_as_float(r[8 * hh + j]);
+          }
+        }
+      }
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == ROW_LOADERS / 32) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols) : "memory");
+  }
+}
+
 // dw[co][t][ci] = sum over splits of ws[split][(t, ci)][co].
 __global__ void wgrad_reduce_kernel(const float* __restrict__ ws, float* __restrict__ dw, uint32_t splits,
                                     uint32_t rows, uint32_t cout, uint32_t taps, uint32_t cin) {
@@ -385,6 +719,102 @@ int launch_gemm(const GemmArgs& p, uint32_t splits, cudaStream_t st) {
   return WT_OK;
 }
 
+// Tiling of conv_rows_kernel.  Wide tiles (xg groups of 8 voxels along x) share
+// their halo and their weights; narrow ones and a split of N give a small grid
+// enough blocks.  Shared memory of a block stays below a third of an SM's where it
+// can, so that several blocks overlap their loads, MMAs and epilogues.
+constexpr uint32_t SMS = 152, SMEM_MAX = 227 * 1024, SMEM_THIRD = 74 * 1024;
+
+template <int MODE, int XG>
+int launch_rows_xg(const RowArgs& p, uint32_t smem, dim3 grid, cudaStream_t st) {
+  cudaError_t e = cudaFuncSetAttribute(conv_rows_kernel<MODE, XG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX);
+  if (e != cudaSuccess) return nfail(WT_ERR_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
+  conv_rows_kernel<MODE, XG><<<grid, ROW_THREADS, smem, st>>>(p);
+  e = cudaGetLastError();
+  if (e != cudaSuccess) return nfail(WT_ERR_CUDA, std::string("conv kernel launch: ") + cudaGetErrorString(e));
+  return WT_OK;
+}
+
+template <int MODE>
+int launch_rows(const wt_conv_shape* s, const void* a, const void* b, const float* bias, void* out, int relu, void* stream) {
+  RowArgs p = {};
+  p.a = static_cast<const __nv_bfloat16*>(a);
+  p.b = static_cast<const __nv_bfloat16*>(b);
+  p.bias = bias;
+  p.out = out;
+  p.relu = relu;
+  p.C = MODE == FWD ? s->cin : s->cout;
+  p.N = MODE == FWD ? s->cout : s->cin;
+  p.taps = s->taps;
+  p.K = p.taps * p.C;
+  p.M = s->batch * s->d * s->h * s->w;
+  p.stage_wait = g_stage_wait.load();
+  p.vec = (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
+  p.halo = s->taps == 27 ? 1u : 0u;
+  uint32_t batch = s->batch;
+  if (p.halo) {
+    p.d = s->d, p.h = s->h, p.w = s->w;
+    p.hp = p.h + 1, p.dp = p.d + 1;
+  } else {  // pointwise: the voxels in rows of 32
+    batch = 1, p.d = 1, p.w = 32, p.h = (p.M + 31) / 32;
+    p.hp = p.h, p.dp = 1;
+  }
+  const uint64_t rows = (uint64_t)batch * p.dp * p.hp;
+  if (rows >= (1ull << 31)) return nfail(WT_ERR_ARG, "convolution: grid too large");
+  p.rows = (uint32_t)rows;
+  p.cg = p.C / 8;
+  p.planes = p.cg + (p.cg & 1u);
+  p.cg_magic = (65536u + p.cg - 1) / p.cg;
+  const uint32_t halo_rows = p.halo * (p.hp + 1);
+  p.run = !p.halo || ROW_TILE + 2 * halo_rows <= ROW_ROWS;
+  p.nrows = p.run ? ROW_TILE + 2 * halo_rows : ROW_ROWS;
+  p.band0 = p.halo;  // row -1 of the first band is shared-memory row 0
+  p.zstep = !p.halo ? 0 : p.run ? p.hp : ROW_TILE + 2;
+  if (p.cg & 1u) {
+    p.upt = (p.cg + 1) / 2;
+    if (p.cg == 1 && MODE == FWD && p.h > 1) p.upt = 0;  // (planes of one row: the distance of two taps may be negative)
+  }
+  p.units = p.upt ? p.taps * p.upt : (p.K + 15) / 16;
+  const uint32_t rt = (p.rows + ROW_TILE - 1) / ROW_TILE, groups = (p.w + 7) / 8, n16 = (p.N + 15) / 16 * 16;
+  auto tile = [&](uint32_t xg) {
+    p.W = 8 * xg + 2 * p.halo;
+    p.pitch = p.nrows * p.W * 16;
+    p.pitch += (144u - p.pitch % 128u) % 128u;  // 16 mod 128: the planes of a voxel fall in different banks
+    p.ctiles = (groups + xg - 1) / xg;
+  };
+  // Longer stages where K is long: an MMA takes 40-70 cycles to issue, a stage's
+  // waits about 400.  (Fewer than 32 MMAs: 4 to a stage, K slices of 64.)
+  auto stage = [&](uint32_t nt) { return p.units < 32 ? 4u : p.units < 64 || nt > 32 ? 8u : 16u; };
+  auto ring = [&](uint32_t nt) { return 2 * stage(nt) * (nt * 16 + 16); };
+  uint32_t xg = 4;
+  for (; xg > 1; xg >>= 1) {
+    tile(xg);
+    if (xg < 2 * groups && p.planes * p.pitch + 4 * ring(n16) <= (xg == 2 ? SMEM_MAX / 2 : SMEM_THIRD) - 4096 && xg * n16 <= 128 &&
+        (uint64_t)rt * p.ctiles >= 2 * SMS)
+      break;
+  }
+  tile(xg);
+  p.nt = n16;
+  while (p.nt > 16 && ((uint64_t)rt * p.ctiles * ((p.N + p.nt - 1) / p.nt) < SMS ||
+                       row_tables(p.units) + p.planes * p.pitch + 4 * ring(p.nt) > SMEM_MAX))
+    p.nt = (p.nt / 2 + 15) / 16 * 16;
+  p.ups = stage(p.nt);
+  const uint32_t nst = (p.units + p.ups - 1) / p.ups, a_bytes = row_tables(p.units) + p.planes * p.pitch;
+  const dim3 grid(rt * p.ctiles, (p.N + p.nt - 1) / p.nt);
+  // A deep ring hides the weights' latency; it must not cost resident blocks.
+  auto per_sm = [&](uint32_t depth) {
+    const uint32_t fit = SMEM_MAX / (a_bytes + depth * ring(p.nt)), have = (grid.x * grid.y + SMS - 1) / SMS;
+    return fit < have ? fit : have;
+  };
+  p.depth = ROW_DEPTH_MAX;
+  while (p.depth > 4 && (p.depth >= 2 * nst || !per_sm(p.depth) || per_sm(p.depth) < per_sm(4))) p.depth /= 2;
+  const uint32_t smem = a_bytes + p.depth * ring(p.nt);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (xg == 4) return launch_rows_xg<MODE, 4>(p, smem, grid, st);
+  if (xg == 2) return launch_rows_xg<MODE, 2>(p, smem, grid, st);
+  return launch_rows_xg<MODE, 1>(p, smem, grid, st);
+}
+
 GemmArgs base_args(const wt_conv_shape* s) {
   GemmArgs p = {};
   p.batch = s->batch; p.d = s->d; p.h = s->h; p.w = s->w;
@@ -405,32 +835,14 @@ int wt_conv3d_forward(const wt_conv_shape* s, const void* x, const void* w, cons
   int rc = check_shape(s, "wt_conv3d_forward");
   if (rc) return rc;
   if (!x || !w || !y) return nfail(WT_ERR_ARG, "wt_conv3d_forward: null tensor");
-  GemmArgs p = base_args(s);
-  p.M = s->batch * s->d * s->h * s->w;
-  p.N = s->cout;
-  p.K = s->taps * s->cin;
-  p.k_chunk = p.K;
-  p.a = static_cast<const __nv_bfloat16*>(x);
-  p.b = static_cast<const __nv_bfloat16*>(w);
-  p.bias = bias;
-  p.out = y;
-  p.relu = relu;
-  return launch_gemm<FWD>(p, 1, static_cast<cudaStream_t>(stream));
+  return launch_rows<FWD>(s, x, w, bias, y, relu, stream);
 }
 
 int wt_conv3d_backward_data(const wt_conv_shape* s, const void* dy, const void* wt, float* dx, void* stream) {
   int rc = check_shape(s, "wt_conv3d_backward_data");
   if (rc) return rc;
   if (!dy || !wt || !dx) return nfail(WT_ERR_ARG, "wt_conv3d_backward_data: null tensor");
-  GemmArgs p = base_args(s);
-  p.M = s->batch * s->d * s->h * s->w;
-  p.N = s->cin;
-  p.K = s->taps * s->cout;
-  p.k_chunk = p.K;
-  p.a = static_cast<const __nv_bfloat16*>(dy);
-  p.b = static_cast<const __nv_bfloat16*>(wt);
-  p.out = dx;
-  return launch_gemm<DGRAD>(p, 1, static_cast<cudaStream_t>(stream));
+  return launch_rows<DGRAD>(s, dy, wt, nullptr, dx, 0, stream);
 }
 
 size_t wt_conv3d_workspace_bytes(const wt_conv_shape* s) {
