@@ -10,7 +10,7 @@
 // FWD and DGRAD (conv_rows_kernel): a block holds one input tile with its halo in
 // shared memory and runs all 27 taps on it; a tap is a shift of the matrix
 // descriptor's start address, so every input value is fetched once per tile
-// instead of once per tap.  WGRAD (conv_gemm_kernel) gathers K slices.
+// instead of once per tap.  WGRAD (conv_wgrad_kernel) does the same with voxels as K.
 // The accumulators live in tensor memory; the epilogues read them with
 // tcgen05.ld (warp w owns lanes 32w..32w+31).  Every mbarrier wait is bounded:
 // on expiry the kernel raises g_conv_error, still waits (bounded) for its own
@@ -35,26 +35,10 @@ std::string& net_error() {
 
 namespace {
 
-constexpr int BM = 128, BK = 64, NTHREADS = 128;
-constexpr uint32_t STAGE_BYTES = BM * BK * 2;       // one operand slice, 16 KB
-constexpr uint32_t SMEM_BYTES = 4 * STAGE_BYTES + 64;  // A0 A1 B0 B1 + barriers + TMEM slot
-constexpr uint32_t TMEM_COLS = 128;
+constexpr uint32_t BM = 128;
 constexpr uint32_t WAIT_LIMIT = 1u << 21;
 
-enum Mode { FWD = 0, DGRAD = 1, WGRAD = 2 };
-
-struct GemmArgs {
-  uint32_t batch, d, h, w;
-  uint32_t cin, cout, taps;
-  uint32_t M, N, K;        // GEMM extents
-  uint32_t k_chunk;        // K per split (WGRAD; multiple of BK), K otherwise
-  const __nv_bfloat16* a;  // FWD x, DGRAD dy, WGRAD x
-  const __nv_bfloat16* b;  // FWD w, DGRAD wt, WGRAD dy
-  const float* bias;
-  void* out;               // FWD bf16 y[M][cout], DGRAD f32 dx[M][cin], WGRAD f32 ws[split][M][N]
-  int relu;
-  uint32_t stage_wait;     // polls of a K-slice stage wait (WAIT_LIMIT unless a test lowers it)
-};
+enum Mode { FWD = 0, DGRAD = 1 };
 
 // Poll budget of the pipeline's stage waits for the next launches (see
 // wt_net_set_stage_wait_limit); the drain before tensor memory is freed always
@@ -75,9 +59,10 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint3
 }
 
 // Instruction descriptor of kind::f16: D FP32 (bits 4-5 = 1), A and B BF16
-// (bits 7-9 = 1, 10-12 = 1), both K-major, N >> 3 at bit 17, M >> 4 at bit 24.
-__host__ __device__ constexpr uint32_t idesc_bf16(uint32_t m, uint32_t n) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((n >> 3) << 17) | ((m >> 4) << 24);
+// (bits 7-9 = 1, 10-12 = 1), both K-major (bits 15, 16 = 0) or both M/N-major (1),
+// N >> 3 at bit 17, M >> 4 at bit 24.
+__host__ __device__ constexpr uint32_t idesc_bf16(uint32_t m, uint32_t n, uint32_t mn_major = 0) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | (mn_major * 3u << 15) | ((n >> 3) << 17) | ((m >> 4) << 24);
 }
 
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
@@ -100,238 +85,6 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_
 __device__ __forceinline__ int tap_dz(uint32_t t, uint32_t taps) { return taps == 27 ? (int)(t / 9) - 1 : 0; }
 __device__ __forceinline__ int tap_dy(uint32_t t, uint32_t taps) { return taps == 27 ? (int)((t / 3) % 3) - 1 : 0; }
 __device__ __forceinline__ int tap_dx(uint32_t t, uint32_t taps) { return taps == 27 ? (int)(t % 3) - 1 : 0; }
-
-// Byte offset of 16-byte chunk (row r, k-group g) in the core-matrix layout.
-__device__ __forceinline__ uint32_t chunk_off(uint32_t r, uint32_t g) { return ((r >> 3) * 8u + g) * 128u + (r & 7u) * 16u; }
-
-__device__ __forceinline__ uint4 ld16(const __nv_bfloat16* p) { return __ldg(reinterpret_cast<const uint4*>(p)); }
-
-
-// Grid position of a voxel (x fastest, then y, z, batch item).
-struct VoxPos {
-  int x, y, z;
-  int64_t vox;
-  bool ok;
-};
-
-__device__ __forceinline__ VoxPos vox_pos(const GemmArgs& p, uint32_t m, uint32_t end) {
-  VoxPos r;
-  r.ok = m < end;
-  const uint32_t mm = r.ok ? m : 0u;
-  r.x = (int)(mm % p.w);
-  r.y = (int)((mm / p.w) % p.h);
-  r.z = (int)((mm / (p.w * p.h)) % p.d);
-  r.vox = mm;
-  return r;
-}
-
-// Index of the voxel r + (dz, dy, dx) in the same batch item, or -1 outside the grid.
-__device__ __forceinline__ int64_t nbr(const GemmArgs& p, const VoxPos& r, int dz, int dy, int dx) {
-  const int xx = r.x + dx, yy = r.y + dy, zz = r.z + dz;
-  if ((unsigned)xx >= p.w || (unsigned)yy >= p.h || (unsigned)zz >= p.d) return -1;
-  return r.vox + ((int64_t)dz * p.h + dy) * p.w + dx;
-}
-
-// Gather K slice [k0, k0 + 64) of both operands into the stage buffers sa, sb.
-//   FWD / DGRAD: thread t owns A row t (a voxel, position precomputed in `row`)
-//   and B row t (a weight row); each 16-byte chunk is 8 consecutive channels of
-//   one tap, one vector load.
-//   WGRAD: K runs over voxels; thread t owns voxel k0 + (t & 63) and half
-//   (t >> 6) of the A rows (taps x channels) and B rows (output channels); it
-//   loads 8 channels of its voxel with one vector load and stores them into 8
-//   rows of the K-major tile (2-byte stores).
-// Rows past the MMA's N (B) are never read and not written; K past the range
-// is zero in both operands.
-template <int MODE>
-__device__ __forceinline__ void gather(const GemmArgs& p, const VoxPos& row, uint32_t tile_m, uint32_t n_mma,
-                                       uint32_t k0, uint32_t k_end, uint8_t* sa, uint8_t* sb) {
-  const uint32_t t = threadIdx.x;
-  if constexpr (MODE == FWD || MODE == DGRAD) {
-    const uint32_t C = (MODE == FWD) ? p.cin : p.cout;
-    const int sg = (MODE == FWD) ? 1 : -1;
-    uint32_t tap = k0 / C, c = k0 % C;
-#pragma unroll
-    for (uint32_t g = 0; g < 8; g++) {
-      const uint32_t k = k0 + 8 * g;
-      uint4 v = make_uint4(0u, 0u, 0u, 0u);
-      if (row.ok && k < k_end) {
-        const int64_t sv = nbr(p, row, sg * tap_dz(tap, p.taps), sg * tap_dy(tap, p.taps), sg * tap_dx(tap, p.taps));
-        if (sv >= 0) v = ld16(p.a + (size_t)sv * C + c);
-      }
-      *reinterpret_cast<uint4*>(sa + chunk_off(t, g)) = v;
-      c += 8;
-      if (c >= C) {
-        c = 0;
-        tap++;
-      }
-    }
-    if (t < n_mma) {
-#pragma unroll
-      for (uint32_t g = 0; g < 8; g++) {
-        const uint32_t k = k0 + 8 * g;
-        uint4 v = make_uint4(0u, 0u, 0u, 0u);
-        if (t < p.N && k < k_end) v = ld16(p.b + (size_t)t * p.K + k);
-        *reinterpret_cast<uint4*>(sb + chunk_off(t, g)) = v;
-      }
-    }
-  } else {
-    const uint32_t j = t & 63u, half = t >> 6;
-    const VoxPos m = vox_pos(p, k0 + j, k_end);
-    const uint32_t jo = (j & 7u) * 2u, jg = j >> 3;
-    // A rows half*64 .. +63 = (tap, ci) rows tile_m + ...
-#pragma unroll
-    for (uint32_t q = 0; q < 8; q++) {
-      const uint32_t r0 = half * 64u + 8u * q, R0 = tile_m + r0;
-      uint4 v = make_uint4(0u, 0u, 0u, 0u);
-      if (m.ok && R0 < p.M) {
-        const uint32_t tap = R0 / p.cin, ci = R0 % p.cin;
-        const int64_t sv = nbr(p, m, tap_dz(tap, p.taps), tap_dy(tap, p.taps), tap_dx(tap, p.taps));
-        if (sv >= 0) v = ld16(p.a + (size_t)sv * p.cin + ci);
-      }
-      const uint32_t w4[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-      for (int e = 0; e < 8; e++)
-        *reinterpret_cast<uint16_t*>(sa + chunk_off(r0 + e, jg) + jo) = (uint16_t)(w4[e >> 1] >> ((e & 1) * 16));
-    }
-    // B rows (output channels) half*64 .. +63, only those the MMA reads
-#pragma unroll
-    for (uint32_t q = 0; q < 8; q++) {
-      const uint32_t r0 = half * 64u + 8u * q;
-      if (r0 >= n_mma) break;
-      uint4 v = make_uint4(0u, 0u, 0u, 0u);
-      if (m.ok && r0 < p.N) v = ld16(p.b + (size_t)m.vox * p.cout + r0);
-      const uint32_t w4[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-      for (int e = 0; e < 8; e++)
-        *reinterpret_cast<uint16_t*>(sb + chunk_off(r0 + e, jg) + jo) = (uint16_t)(w4[e >> 1] >> ((e & 1) * 16));
-    }
-  }
-}
-
-template <int MODE>
-__global__ void __launch_bounds__(NTHREADS, 1) conv_gemm_kernel(GemmArgs p) {
-  extern __shared__ __align__(1024) uint8_t smem[];
-  // stage s: A at smem + s * STAGE_BYTES, B at smem + (2 + s) * STAGE_BYTES
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 4 * STAGE_BYTES);  // [2]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + 4 * STAGE_BYTES + 16);
-  const uint32_t t = threadIdx.x, warp = t >> 5;
-  const uint32_t tile_m = blockIdx.x * BM;
-  const uint32_t k_begin = blockIdx.y * p.k_chunk;
-  const uint32_t k_end = min(p.K, k_begin + p.k_chunk);
-  const uint32_t nk = (k_end > k_begin) ? (k_end - k_begin + BK - 1) / BK : 0;
-  const uint32_t n_mma = ((p.N + 15) / 16) * 16;
-  const uint32_t idesc = idesc_bf16(BM, n_mma);
-
-  if (t == 0) {
-    mbar_init(smem_u32(&bars[0]), 1);
-    mbar_init(smem_u32(&bars[1]), 1);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                 "r"(TMEM_COLS)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  }
-  __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = *tmem_slot;
-
-  const VoxPos row_pos = vox_pos(p, tile_m + t, p.M);  // FWD / DGRAD: this thread's A row (a voxel)
-  bool ok = true;
-  uint32_t issued = 0;  // K slices whose MMAs were issued (uniform across the block)
-  for (uint32_t kt = 0; kt < nk; kt++) {
-    const uint32_t s = kt & 1u;
-    bool w = true;
-    if (kt >= 2) w = mbar_wait(smem_u32(&bars[s]), ((kt >> 1) - 1) & 1u, p.stage_wait);  // MMAs of slice kt-2 done
-    if (!__syncthreads_and(w)) {  // the block stops together
-      ok = false;
-      break;
-    }
-    uint8_t* const sa = smem + s * STAGE_BYTES;
-    uint8_t* const sb = smem + (2u + s) * STAGE_BYTES;
-    gather<MODE>(p, row_pos, tile_m, n_mma, k_begin + kt * BK, k_end, sa, sb);
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    __syncthreads();
-    if (t == 0) {
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t a0 = smem_u32(sa), b0 = smem_u32(sb);
-#pragma unroll
-      for (uint32_t kk = 0; kk < BK / 16; kk++) {
-        const uint64_t ad = smem_desc(a0 + kk * 256u, 128u, 1024u);
-        const uint64_t bd = smem_desc(b0 + kk * 256u, 128u, 1024u);
-        const uint32_t acc = (kt > 0 || kk > 0) ? 1u : 0u;
-        asm volatile(
-            "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-            " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
-            "l"(ad), "l"(bd), "r"(idesc), "r"(acc)
-            : "memory");
-      }
-      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                       smem_u32(&bars[s]))
-                   : "memory");
-    }
-    issued++;
-  }
-  // All MMAs done: the last commit covers every earlier one of the issuing thread.
-  if (issued > 0) {
-    const uint32_t last = issued - 1;
-    const bool done = mbar_wait(smem_u32(&bars[last & 1u]), (last >> 1) & 1u, WAIT_LIMIT);
-    ok = ok && done;
-  }
-  if (!ok && t == 0) atomicExch(&g_conv_error, 1);
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-
-  // ---- epilogue: lane = row t of the tile, 16 columns per tcgen05.ld
-  const uint32_t row = tile_m + t;
-  const uint32_t taddr = tmem + ((warp * 32u) << 16);
-  for (uint32_t c0 = 0; c0 < n_mma; c0 += 16) {
-    uint32_t r[16];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr + c0)
-        : "memory");
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-    if (!ok || row >= p.M || nk == 0) continue;
-#pragma unroll
-    for (int j = 0; j < 16; j++) {
-      const uint32_t col = c0 + j;
-      if (col >= p.N) break;
-      float v = __uint_as_float(r[j]);
-      if constexpr (MODE == FWD) {
-        if (p.bias) v += p.bias[col];
-        if (p.relu) v = fmaxf(v, 0.0f);
-        reinterpret_cast<__nv_bfloat16*>(p.out)[(size_t)row * p.N + col] = __float2bfloat16_rn(v);
-      } else if constexpr (MODE == DGRAD) {
-        reinterpret_cast<float*>(p.out)[(size_t)row * p.N + col] = v;
-      } else {
-        reinterpret_cast<float*>(p.out)[((size_t)blockIdx.y * p.M + row) * p.N + col] = v;
-      }
-    }
-  }
-  if (nk == 0 && row < p.M) {  // empty K range: the product is zero
-    for (uint32_t col = 0; col < p.N; col++) {
-      if constexpr (MODE == FWD) {
-        float v = p.bias ? p.bias[col] : 0.0f;
-        if (p.relu) v = fmaxf(v, 0.0f);
-        reinterpret_cast<__nv_bfloat16*>(p.out)[(size_t)row * p.N + col] = __float2bfloat16_rn(v);
-      } else if constexpr (MODE == DGRAD) {
-        reinterpret_cast<float*>(p.out)[(size_t)row * p.N + col] = 0.0f;
-      } else {
-        reinterpret_cast<float*>(p.out)[((size_t)blockIdx.y * p.M + row) * p.N + col] = 0.0f;
-      }
-    }
-  }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  if (warp == 0) {
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
-  }
-}
 
 // ---------------------------------------------------------------------------
 // FWD / DGRAD: the input tile with its halo stays in shared memory for all taps.
@@ -671,6 +424,318 @@ __global__ void __launch_bounds__(ROW_THREADS) conv_rows_kernel(RowArgs p) {
   }
 }
 
+// ---------------------------------------------------------------------------
+// WGRAD: D[co][(dy, ci)] += sum over a tile's voxels of dy[m][co] x[m + off][ci].
+//
+// A block owns one dz and one or all three dx (its accumulators in tensor memory)
+// and a range of tiles (16 numbered rows x 8 XG voxels, as above) for which it
+// loads the output gradient and, with its halo, the input, into two buffers in
+// turn.  Both operands are M/N-major: 8 channels of a voxel are 16 contiguous
+// bytes, 8 voxels along x one core matrix, and the channel groups of a row are laid
+// out one after the other (group pitch), rows following at channel groups x group
+// pitch.  So the N groups of one MMA run through the channels of three successive
+// rows: the taps dy = -1, 0, 1 come in one MMA of N = 3 cin (up to 256), with K =
+// two groups of 8 voxels.  Only rows of the grid are walked: the K steps of a tile
+// are tabulated by the loaders from the rows' validity, an odd group paired with
+// zeros.  Measured, the network's 12 distinct layers at batch 16 / 1 (us in all, with
+// the reduction): 3620 -> 792 / 1390 -> 252 against a gather of every tap's K slices
+// through registers with 2-byte stores.  What bounds it now: on the wide layers the
+// MMAs (cout of 8-16 uses an eighth to a quarter of M), on the others the copies'
+// latency per tile.  M is 64 or 128: rows above cout are computed from whatever follows in
+// shared memory and not read.
+struct WgradArgs {
+  const __nv_bfloat16 *x, *dy;
+  float* ws;               // [split][taps * cin][cout]
+  uint32_t cin, cout, taps;
+  uint32_t d, h, w, M, hp, dp, rows;  // as RowArgs
+  uint32_t cgx, cgy;       // channel groups of x in a block, and of dy
+  uint32_t chunks;         // blocks along cin
+  uint32_t nbuf;           // tile buffers
+  uint32_t magx, magy;     // ceil(2^16 / cgx), ceil(2^16 / cgy)
+  uint32_t halo, W;        // voxels per row of the x tile
+  uint32_t gpx, gpy;       // bytes per channel group of a row
+  uint32_t xrows;          // rows of the x tile
+  uint32_t xofs, buf;      // offset of the x tile in a buffer, bytes per buffer
+  uint32_t xg, ctiles, tiles, splits;
+  uint32_t groups;         // x groups of a row of the grid
+  uint32_t dxs;            // dx per block: 3, or 1 (one also splits cin into chunks)
+  uint32_t m, n, bstep;    // M and N of one MMA; bytes between the x operands of an MMA and the next of its K step
+  uint32_t cols;           // tensor-memory columns
+  uint32_t stage_wait, throttle;  // throttle: more than two K slices of 64 voxels
+};
+
+constexpr uint32_t WG_STEPS = 32, WG_BUFS = 4, WG_TABLES = WG_BUFS + 2;  // K steps of a tile
+constexpr uint32_t WG_HEAD = 256 + WG_TABLES * 400 + 32;               // barriers, tables
+constexpr uint32_t WG_THREADS = ROW_THREADS + 32;                        // loaders, issuer, table warp
+
+// Voxels of the tile's gradient rows and x rows (-1: zeros) and its K steps.
+struct WgTile {
+  int32_t yv[ROW_TILE], xv[ROW_TILE + 2];
+  uint32_t steps, pad;
+  uint2 step[WG_STEPS];    // descriptor low words of dy and x
+};
+static_assert(sizeof(WgTile) == 400 && WG_HEAD % 128 == 0, "tables fit the head");
+
+template <int NM>
+__global__ void __launch_bounds__(WG_THREADS) conv_wgrad_kernel(WgradArgs p) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  uint64_t* const full = reinterpret_cast<uint64_t*>(smem);  // [WG_BUFS]
+  uint64_t* const done = full + WG_BUFS;
+  uint64_t* const tfull = done + WG_BUFS;     // [WG_TABLES]: a table is there
+  uint64_t* const tfree = tfull + WG_TABLES;  // its readers are through with it
+  uint32_t* const tmem_slot = reinterpret_cast<uint32_t*>(smem + 192);
+  uint32_t* const stop = tmem_slot + 1;
+  uint32_t* const nonzero = tmem_slot + 2;  // 0: no row of the grid in this block's tiles, the accumulators are unset
+  WgTile* const tile = reinterpret_cast<WgTile*>(smem + 256);  // [WG_TABLES]
+  const uint32_t s0 = smem_u32(smem) + WG_HEAD;
+  const uint32_t zero = s0 + p.nbuf * p.buf;  // a zero row of the gradient tile
+  const uint32_t t = threadIdx.x, warp = __shfl_sync(0xffffffffu, t >> 5, 0), lane = t & 31u;
+  const uint32_t split = blockIdx.x, tg = blockIdx.y / p.chunks, g0 = (blockIdx.y - tg * p.chunks) * p.cgx;
+  const int dz = p.halo ? (int)(p.dxs == 3 ? tg : tg / 3u) - 1 : 0;
+  const uint32_t dx0 = p.halo && p.dxs == 1 ? tg % 3u : 0u;  // first dx + 1 of this block
+  const uint32_t tb = (uint32_t)((uint64_t)split * p.tiles / p.splits), te = (uint32_t)((uint64_t)(split + 1) * p.tiles / p.splits);
+  // dx = -1 never reads the last column; where a row's last group reaches past the
+  // grid, its gradient there is zero and so has to be x (0 times infinity)
+  const uint32_t xlim = p.halo && p.dxs == 1 && dx0 == 0 ? p.w - 1 : p.w;
+  const uint32_t rpx = p.cgx * p.gpx, rpy = p.cgy * p.gpy;
+
+  if (warp == ROW_LOADERS / 32) {
+    if (lane == 0) {
+      for (uint32_t i = 0; i < WG_BUFS; i++) {
+        mbar_init(smem_u32(&full[i]), ROW_LOADERS);
+        mbar_init(smem_u32(&done[i]), 1);
+      }
+      for (uint32_t i = 0; i < WG_TABLES; i++) {
+        mbar_init(smem_u32(&tfull[i]), 1);
+        mbar_init(smem_u32(&tfree[i]), ROW_LOADERS / 32 + 1);
+      }
+      *stop = 0u;
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncwarp();
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(p.cols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  } else if (warp < ROW_LOADERS / 32) {
+    for (uint32_t i = t * 16u; i < rpy; i += ROW_LOADERS * 16u)
+      *reinterpret_cast<uint4*>(smem + WG_HEAD + p.nbuf * p.buf + i) = make_uint4(0u, 0u, 0u, 0u);
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *tmem_slot;
+
+  bool ok = true;
+  if (warp == ROW_LOADERS / 32) {
+    const uint32_t idesc = idesc_bf16(p.m, p.n, 1);
+    const uint64_t ahi = (uint64_t)((p.gpy >> 4) | (1u << 14)) << 32, bhi = (uint64_t)((p.gpx >> 4) | (1u << 14)) << 32;
+    uint32_t elected;
+    asm volatile("{\n .reg .pred q;\n elect.sync _|q, 0xffffffff;\n selp.u32 %0, 1, 0, q;\n}\n" : "=r"(elected));
+    uint32_t acc = 0, kt = 0, b = 0, phase = 0, tab = 0, tphase = 0;
+    for (uint32_t i = tb; i < te; i++, kt++) {
+      ok = mbar_wait_or(smem_u32(&tfull[tab]), tphase, stop) && mbar_wait_or(smem_u32(&full[b]), phase, stop);
+      if (!__all_sync(0xffffffffu, ok)) {
+        ok = false;
+        if (elected) *reinterpret_cast<volatile uint32_t*>(stop) = 1u;
+        break;
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      if (elected) {
+        const WgTile& T = tile[tab];
+        const uint32_t steps = T.steps, bs = p.bstep >> 4;
+#pragma unroll 4
+        for (uint32_t s = 0; s < steps; s++) {
+          const uint2 v = T.step[s];
+#pragma unroll
+          for (uint32_t j = 0; j < NM; j++) mma_bf16(tmem + j * p.n, ahi | v.x, bhi | (v.y + j * bs), idesc, acc);
+          acc = 1u;
+        }
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(&done[b]))
+                     : "memory");
+      }
+      __syncwarp();
+      if (elected) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&tfree[tab])) : "memory");
+      if (++tab == WG_TABLES) {
+        tab = 0;
+        tphase ^= 1u;
+      }
+      if (++b == p.nbuf) {
+        b = 0;
+        phase ^= 1u;
+      }
+    }
+    if (elected) *nonzero = acc;
+    if (kt > 0) {
+      const uint32_t last = smem_u32(&done[b ? b - 1 : p.nbuf - 1]), ph = b ? phase : phase ^ 1u;
+      if (p.throttle) ok = mbar_wait(last, ph, p.stage_wait) && ok;
+      ok = mbar_wait(last, ph, WAIT_LIMIT) && ok;  // before the tensor memory is freed, whatever came before
+    }
+  } else if (warp == ROW_LOADERS / 32 + 1) {
+    // Rows and K steps of tile i (buffer b), by one warp.
+    auto make_table = [&](uint32_t i, uint32_t b, WgTile& T) {
+      const uint32_t base = s0 + b * p.buf, x0 = (i % p.ctiles) * p.xg * 8u, r0 = (i / p.ctiles) * ROW_TILE;
+      const uint32_t ng = min(p.xg, p.groups - (x0 >> 3));
+      auto voxel = [&](int64_t R) -> int32_t {
+        if (R < 0 || R >= (int64_t)p.rows) return -1;
+        const uint32_t r = (uint32_t)R, q = r / p.hp, y = r - q * p.hp, bb = q / p.dp, z = q - bb * p.dp;
+        return y < p.h && z < p.d ? (int32_t)(((bb * p.d + z) * p.h + y) * p.w) : -1;
+      };
+      if (lane < p.xrows) T.xv[lane] = voxel((int64_t)r0 + dz * (int)p.hp + lane - p.halo);
+      const int32_t yv = lane < ROW_TILE ? voxel((int64_t)r0 + lane) : -1;
+      if (lane < ROW_TILE) T.yv[lane] = yv;
+      const uint32_t valid = __ballot_sync(0xffffffffu, yv >= 0), units = __popc(valid) * ng;
+      if (lane == 0) T.steps = (units + 1) / 2;
+      const uint32_t u = 2u * lane;
+      if (u < units) {
+        auto place = [&](uint32_t v, uint32_t& row, uint32_t& g) {
+          uint32_t rank = v / ng;
+          g = v - rank * ng;
+          uint32_t m = valid;
+          for (; rank > 0; rank--) m &= m - 1;
+          row = __ffs(m) - 1;
+        };
+        uint32_t ra, ga, rb, gb;
+        place(u, ra, ga);
+        const uint32_t aa = base + ra * rpy + ga * 128u, xa = base + p.xofs + ra * rpx + ga * 128u + (p.halo ? dx0 * 16u : 0u);
+        uint32_t la = zero - aa, lx = 0u;  // zeros against the same x (whose own products are in the first half)
+        if (u + 1 < units) {
+          place(u + 1, rb, gb);
+          la = (rb - ra) * rpy + gb * 128u - ga * 128u;
+          lx = (rb - ra) * rpx + gb * 128u - ga * 128u;
+        }
+        T.step[lane] = make_uint2((aa >> 4) | ((la >> 4) << 16), (xa >> 4) | ((lx >> 4) << 16));
+      }
+    };
+    // (Formed by a loading warp between its copies a table kept the others waiting for
+    // 2300 cycles a tile.)
+    uint32_t kt = 0, b = 0, tab = 0, phase = 1;
+    for (uint32_t i = tb; i < te; i++, kt++) {
+      if (kt >= WG_TABLES) ok = mbar_wait_or(smem_u32(&tfree[tab]), phase, stop);
+      if (!__all_sync(0xffffffffu, ok)) {
+        ok = false;
+        *reinterpret_cast<volatile uint32_t*>(stop) = 1u;
+        break;
+      }
+      make_table(i, b, tile[tab]);
+      __syncwarp();
+      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&tfull[tab])) : "memory");
+      if (++tab == WG_TABLES) {
+        tab = 0;
+        phase ^= 1u;
+      }
+      if (++b == p.nbuf) b = 0;
+    }
+  } else {
+    uint32_t kt = 0, b = 0, phase = 1, tab = 0, tphase = 0;
+    for (uint32_t i = tb; i < te; i++, kt++) {
+      const uint32_t base = s0 + b * p.buf;
+      ok = mbar_wait_or(smem_u32(&tfull[tab]), tphase, stop) && (kt < p.nbuf || mbar_wait_or(smem_u32(&done[b]), phase, stop));
+      if (!ok) {
+        *reinterpret_cast<volatile uint32_t*>(stop) = 1u;
+        break;
+      }
+      const WgTile& T = tile[tab];
+      const uint32_t x0 = (i % p.ctiles) * p.xg * 8u;
+      {
+        const uint32_t per = 8u * p.xg * p.cgy, q = ROW_LOADERS / per, rem = ROW_LOADERS - q * per;
+        uint32_t r = t / per, e = t - r * per;
+#pragma unroll 4
+        for (uint32_t k = t; k < ROW_TILE * per; k += ROW_LOADERS) {
+          const int32_t v0 = T.yv[r];
+          const uint32_t xx = (e * p.magy) >> 16, g = e - xx * p.cgy, x = x0 + xx;
+          const bool in = v0 >= 0 && x < p.w && (uint32_t)v0 + x < p.M;
+          cp16(base + r * rpy + g * p.gpy + xx * 16u, in ? p.dy + (size_t)((uint32_t)v0 + x) * p.cout + g * 8u : p.dy, in);
+          r += q;
+          e += rem;
+          if (e >= per) {
+            e -= per;
+            r++;
+          }
+        }
+      }
+      {
+        const uint32_t per = p.W * p.cgx, q = ROW_LOADERS / per, rem = ROW_LOADERS - q * per;
+        uint32_t r = t / per, e = t - r * per;
+#pragma unroll 4
+        for (uint32_t k = t; k < p.xrows * per; k += ROW_LOADERS) {
+          const int32_t v0 = T.xv[r];
+          const uint32_t xx = (e * p.magx) >> 16, g = e - xx * p.cgx, x = x0 + xx - p.halo;
+          const bool in = v0 >= 0 && x < xlim && (uint32_t)v0 + x < p.M && (g0 + g) * 8u < p.cin;
+          cp16(base + p.xofs + r * rpx + g * p.gpx + xx * 16u, in ? p.x + (size_t)((uint32_t)v0 + x) * p.cin + (g0 + g) * 8u : p.x, in);
+          r += q;
+          e += rem;
+          if (e >= per) {
+            e -= per;
+            r++;
+          }
+        }
+      }
+      asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&full[b])) : "memory");
+      __syncwarp();
+      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&tfree[tab])) : "memory");
+      if (++tab == WG_TABLES) {
+        tab = 0;
+        tphase ^= 1u;
+      }
+      if (++b == p.nbuf) {
+        b = 0;
+        phase ^= 1u;
+      }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+  }
+  __syncwarp();
+  ok = __syncthreads_and(ok);
+  if (!ok && t == 0) atomicExch(&g_conv_error, 1);
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+
+  // ---- epilogue: lane = output channel, columns = (dy, ci) of each dx (or ci of each dy)
+  if (ok && warp < ROW_LOADERS / 32) {
+    // M 128: lane = row; M 64: rows 16 w .. 16 w + 15 in the first lanes of quarter w
+    const uint32_t co = p.m == 64 ? ((warp & 3u) * 16u + lane) | (lane & 16u ? 128u : 0u) : t & 127u, taddr = tmem + (((warp & 3u) * 32u) << 16), per = p.n / 16u;
+    const uint32_t cb = 8u * p.cgx;  // channels of this block
+    const uint32_t used = NM == 3 && p.dxs == 1 ? cb : (p.halo ? 3u : 1u) * cb;  // columns of an accumulator
+    float* const out = p.ws + (size_t)split * p.taps * p.cin * p.cout + co;
+    const bool zeros = *nonzero == 0u;
+    for (uint32_t c = warp >> 2; c < NM * per; c += 2) {
+      __syncwarp();
+      const uint32_t j = c / per, c0 = 16u * (c - j * per);
+      uint32_t r[16];
+      asm volatile(
+          "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+          : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+            "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+          : "r"(taddr + j * p.n + c0)
+          : "memory");
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      if (co >= p.cout) continue;
+#pragma unroll
+      for (uint32_t k = 0; k < 16; k++) {
+        const uint32_t col = c0 + k;
+        if (col >= used) break;
+        uint32_t ci = col, tap = 0;
+        if (p.halo) {
+          const uint32_t dyi = NM == 3 && p.dxs == 1 ? j : col / cb;
+          if (!(NM == 3 && p.dxs == 1)) ci = col - dyi * cb;
+          tap = (uint32_t)(dz + 1) * 9u + dyi * 3u + (p.dxs == 3 ? j : dx0);
+        }
+        ci += 8u * g0;
+        if (ci >= p.cin) continue;
+        const uint32_t row = tap * p.cin + ci;
+        out[(size_t)row * p.cout] = zeros ? 0.0f : __uint_as_float(r[k]);
+      }
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == ROW_LOADERS / 32) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(p.cols) : "memory");
+  }
+}
+
 // dw[co][t][ci] = sum over splits of ws[split][(t, ci)][co].
 __global__ void wgrad_reduce_kernel(const float* __restrict__ ws, float* __restrict__ dw, uint32_t splits,
                                     uint32_t rows, uint32_t cout, uint32_t taps, uint32_t cin) {
@@ -708,22 +773,18 @@ uint32_t wgrad_splits(uint64_t voxels) {
   return (uint32_t)s;
 }
 
-template <int MODE>
-int launch_gemm(const GemmArgs& p, uint32_t splits, cudaStream_t st) {
-  cudaError_t ea = cudaFuncSetAttribute(conv_gemm_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-  if (ea != cudaSuccess) return nfail(WT_ERR_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(ea));
-  const dim3 grid((p.M + BM - 1) / BM, splits);
-  conv_gemm_kernel<MODE><<<grid, NTHREADS, SMEM_BYTES, st>>>(p);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return nfail(WT_ERR_CUDA, std::string("conv kernel launch: ") + cudaGetErrorString(e));
-  return WT_OK;
-}
-
 // Tiling of conv_rows_kernel.  Wide tiles (xg groups of 8 voxels along x) share
 // their halo and their weights; narrow ones and a split of N give a small grid
 // enough blocks.  Shared memory of a block stays below a third of an SM's where it
 // can, so that several blocks overlap their loads, MMAs and epilogues.
 constexpr uint32_t SMS = 152, SMEM_MAX = 227 * 1024, SMEM_THIRD = 74 * 1024;
+
+// A channel group's pitch such that eight successive 16-byte copies (channel groups
+// fastest, then voxels) fall in different banks: 64, 32 or 16 mod 128 bytes.
+uint32_t pad_pitch(uint32_t bytes, uint32_t cg) {
+  const uint32_t want = cg >= 8 ? 16u : cg >= 4 ? 32u : cg >= 2 ? 64u : 0u;
+  return bytes + (want + 128u - bytes % 128u) % 128u;
+}
 
 template <int MODE, int XG>
 int launch_rows_xg(const RowArgs& p, uint32_t smem, dim3 grid, cudaStream_t st) {
@@ -759,7 +820,7 @@ int launch_rows(const wt_conv_shape* s, const void* a, const void* b, const floa
     batch = 1, p.d = 1, p.w = 32, p.h = (p.M + 31) / 32;
     p.hp = p.h, p.dp = 1;
   }
-  const uint64_t rows = (uint64_t)batch * p.dp * p.hp;
+  const uint64_t rows = ((uint64_t)batch * p.dp - p.halo) * p.hp - p.halo;  // up to the last row of the grid
   if (rows >= (1ull << 31)) return nfail(WT_ERR_ARG, "convolution: grid too large");
   p.rows = (uint32_t)rows;
   p.cg = p.C / 8;
@@ -779,7 +840,7 @@ int launch_rows(const wt_conv_shape* s, const void* a, const void* b, const floa
   auto tile = [&](uint32_t xg) {
     p.W = 8 * xg + 2 * p.halo;
     p.pitch = p.nrows * p.W * 16;
-    p.pitch += (144u - p.pitch % 128u) % 128u;  // 16 mod 128: the planes of a voxel fall in different banks
+    p.pitch = pad_pitch(p.pitch, p.cg);
     p.ctiles = (groups + xg - 1) / xg;
   };
   // Longer stages where K is long: an MMA takes 40-70 cycles to issue, a stage's
@@ -815,12 +876,79 @@ int launch_rows(const wt_conv_shape* s, const void* a, const void* b, const floa
   return launch_rows_xg<MODE, 1>(p, smem, grid, st);
 }
 
-GemmArgs base_args(const wt_conv_shape* s) {
-  GemmArgs p = {};
-  p.batch = s->batch; p.d = s->d; p.h = s->h; p.w = s->w;
-  p.cin = s->cin; p.cout = s->cout; p.taps = s->taps;
+// Tiling of conv_wgrad_kernel.  A block takes all three dx where their accumulators
+// fit the tensor memory (9 cin columns), the splits alone give every SM a block and
+// rows end with a group of 8; otherwise one dx, for a finer grid, and where that
+// still leaves SMs idle, cin in chunks (16 channels at least).  The workspace bounds
+// the splits.
+int launch_wgrad(const wt_conv_shape* s, const void* x, const void* dy, float* ws, uint32_t splits, cudaStream_t st) {
+  WgradArgs p = {};
+  p.x = static_cast<const __nv_bfloat16*>(x);
+  p.dy = static_cast<const __nv_bfloat16*>(dy);
+  p.ws = ws;
+  p.cin = s->cin, p.cout = s->cout, p.taps = s->taps;
+  p.M = s->batch * s->d * s->h * s->w;
+  p.halo = s->taps == 27 ? 1u : 0u;
+  uint32_t batch = s->batch;
+  if (p.halo) {
+    p.d = s->d, p.h = s->h, p.w = s->w;
+    p.hp = p.h + 1, p.dp = p.d + 1;
+  } else {
+    batch = 1, p.d = 1, p.w = 32, p.h = (p.M + 31) / 32;
+    p.hp = p.h, p.dp = 1;
+  }
+  const uint64_t rows = ((uint64_t)batch * p.dp - p.halo) * p.hp - p.halo;  // up to the last row of the grid
+  if (rows >= (1ull << 31)) return nfail(WT_ERR_ARG, "convolution: grid too large");
+  p.rows = (uint32_t)rows;
+  p.cgy = p.cout / 8;
+  p.magy = (65536u + p.cgy - 1) / p.cgy;
+  p.groups = (p.w + 7) / 8;
+  p.splits = splits;
+  p.xrows = ROW_TILE + 2 * p.halo;
   p.stage_wait = g_stage_wait.load();
-  return p;
+  p.throttle = p.M / splits > 128 ? 1u : 0u;
+  auto r16 = [](uint32_t v) { return (v + 15) / 16 * 16; };
+  const uint32_t cg = p.cin / 8, n3 = r16(3 * p.cin);
+  uint32_t nm = 1, blocks = splits * (p.halo ? 9 : 1);
+  p.cgx = cg;
+  p.dxs = 1;
+  if (p.halo && 3 * n3 <= 512 && 3 * splits >= SMS && p.w % 8 == 0) {
+    p.dxs = nm = 3;
+    blocks = 3 * splits;
+  } else {
+    while (p.cgx > 2 && blocks * ((cg + p.cgx - 1) / p.cgx) < SMS) p.cgx = (p.cgx + 1) / 2;
+    if (p.halo && 3 * p.cgx * 8 > 256) nm = 3;  // one MMA per dy
+  }
+  p.chunks = (cg + p.cgx - 1) / p.cgx;
+  blocks *= p.chunks;
+  p.m = p.cout <= 64 ? 64 : 128;  // (N 48: 29 and 44 cycles an MMA)
+  p.n = r16((p.halo && !(nm == 3 && p.dxs == 1) ? 3 : 1) * p.cgx * 8);
+  p.magx = (65536u + p.cgx - 1) / p.cgx;
+  uint32_t smem = 0;
+  for (p.xg = p.groups >= 3 ? 4 : p.groups; ; p.xg /= 2) {
+    p.W = 8 * p.xg + 2 * p.halo;
+    p.gpx = pad_pitch(p.W * 16, p.cgx);
+    p.gpy = pad_pitch(8 * p.xg * 16, p.cgy);
+    p.xofs = ROW_TILE * p.cgy * p.gpy;
+    p.buf = (p.xofs + p.xrows * p.cgx * p.gpx + 127) / 128 * 128;
+    // after the buffers: the zero row, and what the junk M rows and N columns of the last rows read
+    const uint32_t rest = WG_HEAD + 16 * p.gpy + 16 * p.gpx + 2048, most = blocks > SMS ? SMEM_MAX / 2 : SMEM_MAX;
+    for (p.nbuf = WG_BUFS; p.nbuf > 2 && rest + p.nbuf * p.buf > most; p.nbuf--) {}
+    smem = rest + p.nbuf * p.buf;
+    if (p.xg == 1 || smem <= most) break;
+  }
+  p.bstep = p.dxs == 3 ? 16u : p.cgx * p.gpx;
+  p.ctiles = (p.groups + p.xg - 1) / p.xg;
+  p.tiles = (p.rows + ROW_TILE - 1) / ROW_TILE * p.ctiles;
+  for (p.cols = 32; p.cols < nm * p.n; p.cols *= 2) {}
+  const dim3 grid(splits, (p.halo ? (p.dxs == 3 ? 3 : 9) : 1) * p.chunks);
+  const auto kernel = nm == 3 ? conv_wgrad_kernel<3> : conv_wgrad_kernel<1>;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX);
+  if (e != cudaSuccess) return nfail(WT_ERR_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
+  kernel<<<grid, WG_THREADS, smem, st>>>(p);
+  e = cudaGetLastError();
+  if (e != cudaSuccess) return nfail(WT_ERR_CUDA, std::string("conv kernel launch: ") + cudaGetErrorString(e));
+  return WT_OK;
 }
 
 }  // namespace
@@ -856,22 +984,13 @@ int wt_conv3d_backward_weight(const wt_conv_shape* s, const void* x, const void*
   int rc = check_shape(s, "wt_conv3d_backward_weight");
   if (rc) return rc;
   if (!x || !dy || !dw || !workspace) return nfail(WT_ERR_ARG, "wt_conv3d_backward_weight: null tensor");
-  GemmArgs p = base_args(s);
   const uint64_t vox = (uint64_t)s->batch * s->d * s->h * s->w;
-  const uint32_t splits = wgrad_splits(vox);
-  p.M = s->taps * s->cin;
-  p.N = s->cout;
-  p.K = (uint32_t)vox;
-  p.k_chunk = (uint32_t)(((vox + splits - 1) / splits + BK - 1) / BK * BK);
-  p.a = static_cast<const __nv_bfloat16*>(x);
-  p.b = static_cast<const __nv_bfloat16*>(dy);
-  p.out = workspace;
+  const uint32_t splits = wgrad_splits(vox), rows = s->taps * s->cin, total = rows * s->cout;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  rc = launch_gemm<WGRAD>(p, splits, st);
+  rc = launch_wgrad(s, x, dy, static_cast<float*>(workspace), splits, st);
   if (rc) return rc;
-  const uint32_t total = p.M * p.N;
-  wgrad_reduce_kernel<<<(total + 255) / 256, 256, 0, st>>>(static_cast<const float*>(workspace), dw, splits, p.M,
-                                                           s->cout, s->taps, s->cin);
+  wgrad_reduce_kernel<<<(total + 255) / 256, 256, 0, st>>>(static_cast<const float*>(workspace), dw, splits, rows, s->cout,
+                                                           s->taps, s->cin);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return nfail(WT_ERR_CUDA, std::string("wgrad reduce: ") + cudaGetErrorString(e));
   return WT_OK;

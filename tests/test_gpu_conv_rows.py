@@ -64,3 +64,47 @@ def test_forward_and_data_gradient(ops, case, aligned):
     assert np.abs(dx.cpu().numpy() - want).max() <= 1e-4 * np.abs(want).max()
     if not aligned:
         assert float(yf[0]) == 7.0 and float(dxf[0]) == 7.0
+
+
+WEIGHT_SHAPES = SHAPES + [
+    (1, 17, 65, 66, 88, 8, 27),    # enough splits for all channels in a block: one MMA per dy (N = 96)
+    (1, 8, 160, 161, 8, 16, 27),   # enough splits for the three dx in a block; ragged last x group
+    (1, 8, 160, 160, 48, 72, 27),  # the same at the most accumulator columns (432), M = 128
+    (2, 9, 31, 30, 40, 64, 27),    # channels in chunks, the last one short; M = 64
+]
+
+
+@pytest.mark.parametrize("case", WEIGHT_SHAPES)
+def test_weight_gradient(ops, case):
+    """FP32 sums of at most 9216 products per split: 1e-4 of the output's scale."""
+    from oracle import conv_ref as ref
+    b, d, h, w, cin, cout, taps = case
+    rng = np.random.default_rng(sum(case))
+    x = ref.bf16_round(rng.standard_normal((b, d, h, w, cin)))
+    dy = ref.bf16_round(rng.standard_normal((b, d, h, w, cout)))
+    xs, ds = (torch.tensor(np.ascontiguousarray(a, np.float32), device="cuda").to(torch.bfloat16) for a in (x, dy))
+    ws = torch.empty(max(1, ops.workspace_bytes(xs.shape, cin, cout, taps) // 4), device="cuda")
+    dw = torch.full((cout, taps, cin), 7.0, device="cuda")
+    ops.conv_backward_weight(xs, ds, dw, ws, taps)
+    ops.check()
+    want = ref.conv3d_backward_weight(x, dy, taps)
+    assert np.abs(dw.cpu().numpy() - want).max() <= 1e-4 * np.abs(want).max()
+
+
+def test_weight_gradient_keeps_infinities_in_their_taps(ops):
+    """An infinite input in the last column of a ragged row reaches the taps whose
+    products contain it and no others (dx = -1 never reads that column)."""
+    b, d, h, w, c = 1, 3, 5, 13, 16
+    g = torch.Generator(device="cuda").manual_seed(3)
+    x = torch.randn((b, d, h, w, c), generator=g, device="cuda").to(torch.bfloat16)
+    dy = torch.randn((b, d, h, w, c), generator=g, device="cuda").to(torch.bfloat16)
+    x[0, 1, 4, 12, 5] = float("inf")
+    ws = torch.empty(max(1, ops.workspace_bytes(x.shape, c, c, 27) // 4), device="cuda")
+    dw = torch.empty((c, 27, c), device="cuda")
+    ops.conv_backward_weight(x, dy, dw, ws, 27)
+    ops.check()
+    finite = torch.isfinite(dw).all(dim=0).cpu().numpy()  # [tap, ci]
+    for t in range(27):
+        dyi, dxi = t // 3 % 3 - 1, t % 3 - 1
+        hit = dxi >= 0 and dyi >= 0  # the voxel minus the tap's offset lies in the grid (it is in the last row and column)
+        assert finite[t, 5] == (not hit) and finite[t, np.arange(c) != 5].all(), t
