@@ -736,14 +736,22 @@ __global__ void __launch_bounds__(WG_THREADS) conv_wgrad_kernel(WgradArgs p) {
   }
 }
 
-// dw[co][t][ci] = sum over splits of ws[split][(t, ci)][co].
+// dw[co][t][ci] = sum over splits of ws[split][(t, ci)][co]: a block takes 32
+// outputs, its eight warps every eighth split each (in FP64, folded in order).
 __global__ void wgrad_reduce_kernel(const float* __restrict__ ws, float* __restrict__ dw, uint32_t splits,
                                     uint32_t rows, uint32_t cout, uint32_t taps, uint32_t cin) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= rows * cout) return;
-  const uint32_t row = i / cout, co = i % cout;  // row = t * cin + ci
+  __shared__ double red[8][32];
+  const uint32_t lane = threadIdx.x & 31u, ph = threadIdx.x >> 5;
+  const uint32_t i = blockIdx.x * 32 + lane;
   double s = 0.0;
-  for (uint32_t k = 0; k < splits; k++) s += ws[((size_t)k * rows + row) * cout + co];
+  if (i < rows * cout)
+#pragma unroll 4
+    for (uint32_t k = ph; k < splits; k += 8) s += ws[(size_t)k * rows * cout + i];
+  red[ph][lane] = s;
+  __syncthreads();
+  if (ph != 0 || i >= rows * cout) return;
+  for (uint32_t q = 1; q < 8; q++) s += red[q][lane];
+  const uint32_t row = i / cout, co = i % cout;  // row = t * cin + ci
   const uint32_t tap = row / cin, ci = row % cin;
   dw[((size_t)co * taps + tap) * cin + ci] = (float)s;
 }
@@ -989,7 +997,7 @@ int wt_conv3d_backward_weight(const wt_conv_shape* s, const void* x, const void*
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   rc = launch_wgrad(s, x, dy, static_cast<float*>(workspace), splits, st);
   if (rc) return rc;
-  wgrad_reduce_kernel<<<(total + 255) / 256, 256, 0, st>>>(static_cast<const float*>(workspace), dw, splits, rows, s->cout,
+  wgrad_reduce_kernel<<<(total + 31) / 32, 256, 0, st>>>(static_cast<const float*>(workspace), dw, splits, rows, s->cout,
                                                            s->taps, s->cin);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return nfail(WT_ERR_CUDA, std::string("wgrad reduce: ") + cudaGetErrorString(e));
