@@ -106,39 +106,127 @@ __device__ V3 seed_of(const StreamArgs& st, uint32_t line) {
   return v3(st.smin[0], wmix(st.smin[1], st.smax[1], fy), wmix(st.smin[2], st.smax[2], fz));
 }
 
+// a / b, correctly rounded, from r = RN(1 / b) by Markstein's correction (see
+// div_rcp in wt_lattice.cuh) for b in [2^-20, 2^20] and a = 0 or |a| in [2^-60, 2^60);
+// other operands (`fast` false, or a outside) take the division itself.  The built-in
+// division leaves its short path for a zero numerator too, and the temperatures and
+// the cross velocities of undisturbed air are zeros: 400 cycles instead of 20.
+__device__ __noinline__ float div_slow(float a, float b) { return __fdiv_rn(a, b); }
+__device__ __forceinline__ float div_known(float a, float b, float r, bool fast) {
+  const uint32_t m = __float_as_uint(a) & 0x7fffffffu;
+  float q = __fmul_rn(a, r);
+  const float c = __fmaf_rn(__fmaf_rn(-q, b, a), r, q);
+  q = m ? c : q;
+  if (!fast || (m - 0x21800000u >= 0x5d800000u - 0x21800000u && m != 0u)) q = div_slow(a, b);
+  return q;
+}
+__device__ __forceinline__ bool div_range(float b) { return b >= 0x1p-20f && b <= 0x1p20f; }
+
+// The velocity and fluid weight of sampleFlow (wgsl.ts:332-357) by one warp at one
+// point.  Lane 4 k + c stands for corner k and, with c < 3, axis and component c: it
+// holds coordinate c of the point (pa), reads component c of the corner's cell (c =
+// 3: its density, which says whether the cell is fluid), and gets u_c.  The
+// operations and their order per value are sample_flow's; the corners' products are
+// formed side by side and summed in order.
+__device__ __forceinline__ float sample_u_warp(const FieldGrid& g, float rh, bool fast_h, float pa, float& fluid) {
+  const uint32_t lane = threadIdx.x, c = lane & 3u, quad = lane & 28u, k = lane >> 2;
+  const bool one = c == 0 ? k & 1u : c == 1 ? k >> 1 & 1u : k >> 2 & 1u;  // the upper corner along axis c
+  const float o = c == 0 ? g.ox : c == 1 ? g.oy : g.oz;
+  const int n = (int)(c == 0 ? g.nx : c == 1 ? g.ny : g.nz);
+  const uint32_t stride = c == 0 ? 1u : c == 1 ? g.nx : g.nx * g.ny;
+  const float gg = div_known((c < 2 ? pa : fabsf(pa)) - o, g.h, rh, fast_h) - 0.5f;
+  const int i0 = __float2int_rd(gg);  // saturating, NaN to 0
+  const float f = gg - (float)i0;
+  int q = i0 + (one ? 1 : 0);
+  if (c >= 2) q ^= q >> 31;  // z: -q - 1 below the symmetry plane
+  const uint32_t part = (uint32_t)min(max(q, 0), n - 1) * stride;
+  const float wa = one ? f : 1.0f - f;
+  const uint32_t id = __shfl_sync(0xffffffffu, part, quad) + __shfl_sync(0xffffffffu, part, quad + 1) +
+                      __shfl_sync(0xffffffffu, part, quad + 2);
+  const float val = __ldg(reinterpret_cast<const float*>(g.fields + id) + c);
+  const float w = __shfl_sync(0xffffffffu, wa, quad) * __shfl_sync(0xffffffffu, wa, quad + 1) *
+                  __shfl_sync(0xffffffffu, wa, quad + 2);
+  const uint32_t wet = __ballot_sync(0xffffffffu, val > 0.0f);  // bits 4 k + 3
+  const float term = c == 3 ? w : val * w;
+  float acc = 0.0f;
+#pragma unroll
+  for (uint32_t j = 0; j < 8; j++) {
+    const float t = __shfl_sync(0xffffffffu, term, 4 * j + c);
+    if (wet >> (4 * j + 3) & 1u) acc = acc + t;
+  }
+  const float wsum = __shfl_sync(0xffffffffu, acc, 3);
+  const bool dry = wsum < 1e-5f;
+  const float ws = dry ? 1.0f : wsum;
+  fluid = dry ? 0.0f : wsum;
+  const float r = div_known(acc, ws, __frcp_rn(ws), div_range(ws));
+  return dry ? 0.0f : c == 2 && pa < 0.0f ? -r : r;
+}
+
+// length(u) of a vector held in lanes 0-2, in every lane.
+__device__ __forceinline__ float len3_warp(float ua) {
+  const float q = ua * ua;
+  return __fsqrt_rn(__shfl_sync(0xffffffffu, q, 0) + __shfl_sync(0xffffffffu, q, 1) + __shfl_sync(0xffffffffu, q, 2));
+}
+// A component of u / len (lanes c < 3; the others' quotients are not used).
+__device__ __forceinline__ float unit_warp(float ua, float len) {
+  const bool fast = div_range(len);
+  return div_known(ua, len, __frcp_rn(fast ? len : 1.0f), fast);
+}
+
 // Streamline pass cs_main (render-wgsl.ts:551-575): one line per block of one
-// warp, lane 0 only.  A line is a chain of dependent RK2 steps, two field samples
-// each; lines packed 32 to a warp would gather from 32 places per load (32 L1
-// lookups per instruction) and sit on a couple of SMs.  One line per warp spreads
-// the (at most a few hundred) lines over the SMs and leaves each gather a single
-// lookup, so each step costs about one L1 round trip per sample.
+// warp.  A line is a chain of dependent RK2 steps, two field samples each, so its
+// time is the chain's latency: the lanes share out each sample's corners and
+// components, and the colours, which no step depends on, are left to the whole warp
+// (a point per lane) once STREAM_CHUNK steps are done.  One lane doing all of it took
+// 1.37 us a step; lines packed 32 to a warp gather from 32 places per load.
+constexpr uint32_t STREAM_CHUNK = 128;
+
 __global__ void __launch_bounds__(32) streamlines_kernel(FieldGrid g, StreamArgs st, ViewArgs view,
                                                         float4* __restrict__ pts) {
-  const uint32_t line = blockIdx.x;
-  if (line >= st.lines || threadIdx.x != 0) return;
+  __shared__ float rec[STREAM_CHUNK][3];  // the points of a chunk
+  const uint32_t line = blockIdx.x, lane = threadIdx.x, c = lane & 3u;
   const uint32_t base = line * st.steps;
-  V3 p = seed_of(st, line);
-  bool alive = true;
+  const V3 seed = seed_of(st, line);
+  float pa = c == 0 ? seed.x : c == 1 ? seed.y : seed.z;
   const V3 hi = v3(g.ox + (float)g.nx * g.h, g.oy + (float)g.ny * g.h, g.oz + (float)g.nz * g.h);
-  for (uint32_t k = 0; k < st.steps; k++) {
-    if (!alive) {
-      pts[base + k] = make_float4(p.x, p.y, p.z, -1.0f);
-      continue;
+  const bool fast_h = div_range(g.h);
+  const float rh = __frcp_rn(fast_h ? g.h : 1.0f);
+  bool alive = true;
+  uint32_t k = 0;
+  while (alive && k < st.steps) {
+    const uint32_t k0 = k, k1 = min(st.steps, k + STREAM_CHUNK);
+    for (; k < k1; k++) {
+      float fluid, fluid2;
+      const float s1 = sample_u_warp(g, rh, fast_h, pa, fluid);
+      const float len1 = len3_warp(s1);
+      if (fluid < 0.3f || len1 < view.uIn * 0.03f) {
+        alive = false;
+        break;
+      }
+      if (lane < 3) rec[k - k0][lane] = pa;
+      const float mid = pa + (unit_warp(s1, len1) * st.stepLen) * 0.5f;
+      const float s2 = sample_u_warp(g, rh, fast_h, c == 3 ? pa : mid, fluid2);
+      const float dir = fluid2 > 0.3f ? s2 : s1;
+      const float step = unit_warp(dir, len3_warp(dir)) * st.stepLen;
+      if (c < 3) pa = pa + step;
+      // past the domain (lane c tests its coordinate)
+      const bool out = c == 0 ? pa > hi.x - g.h * 3.0f : c == 1 ? pa < 0.01f || pa > hi.y : c == 2 && wabs(pa) > hi.z;
+      if (__any_sync(0xffffffffu, out)) {
+        alive = false;
+        k++;
+        break;
+      }
     }
-    const Sample s1 = sample_flow(g, p);
-    if (s1.fluid < 0.3f || len3(s1.u) < view.uIn * 0.03f) {
-      alive = false;
-      pts[base + k] = make_float4(p.x, p.y, p.z, -1.0f);
-      continue;
+    __syncwarp();
+    for (uint32_t i = k0 + lane; i < k; i += 32) {
+      const V3 p = v3(rec[i - k0][0], rec[i - k0][1], rec[i - k0][2]);
+      const Sample s = sample_flow(g, p);
+      pts[base + i] = make_float4(p.x, p.y, p.z, wclamp(field_value(g, view, st.colorMode, s, p), 0.0f, 1.0f));
     }
-    pts[base + k] = make_float4(p.x, p.y, p.z, wclamp(field_value(g, view, st.colorMode, s1, p), 0.0f, 1.0f));
-    const V3 mid = add(p, mul(mul(normalize3(s1.u), st.stepLen), 0.5f));
-    const Sample s2 = sample_flow(g, mid);
-    V3 dir = s1.u;
-    if (s2.fluid > 0.3f) dir = s2.u;
-    p = add(p, mul(normalize3(dir), st.stepLen));
-    if (p.x > hi.x - g.h * 3.0f || p.y < 0.01f || p.y > hi.y || wabs(p.z) > hi.z) alive = false;
+    __syncwarp();
   }
+  const float px = __shfl_sync(0xffffffffu, pa, 0), py = __shfl_sync(0xffffffffu, pa, 1), pz = __shfl_sync(0xffffffffu, pa, 2);
+  for (uint32_t i = k + lane; i < st.steps; i += 32) pts[base + i] = make_float4(px, py, pz, -1.0f);
 }
 
 __global__ void sample_points_kernel(FieldGrid g, const float* __restrict__ pts, uint32_t n, float* __restrict__ out,
