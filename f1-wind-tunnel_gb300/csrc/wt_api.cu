@@ -123,30 +123,22 @@ ReduceArgs reduce_args(const wt_ctx* c) {
 
 int flush_forces(wt_ctx* c);
 
-// After new flags: cell words, force-carrying blocks and their partial slots.
+// After new flags: cell words, force-carrying blocks and their partial slots.  The
+// slots and the cell counts are formed on the device; four words come back (copying
+// the flags and counting on the host took most of a re-voxelization).
 int rebuild_links(wt_ctx* c) {
   if (int rc = flush_forces(c)) return rc;  // pending records use the current slot layout
   WT_CUDA(c, launch_cell_words(c->solid, c->emit, c->cellw, c->nx, c->ny, c->nz, c->stream));
   WT_CUDA(c, launch_heat_sources(c->emit, c->heat_src, c->nx, c->ny, c->nz, c->stream));
-  uint8_t* dflags = nullptr;
-  WT_CUDA(c, cudaMallocAsync((void**)&dflags, c->geom.nblocks, c->stream));
-  WT_CUDA(c, launch_block_flags(c->cellw, c->geom, c->nx, c->ny, c->nz, dflags, c->stream));
-  std::vector<uint8_t> flags(c->geom.nblocks);
-  std::vector<uint8_t> sol(c->n);
-  WT_CUDA(c, cudaMemcpyAsync(flags.data(), dflags, c->geom.nblocks, cudaMemcpyDeviceToHost, c->stream));
-  WT_CUDA(c, cudaMemcpyAsync(sol.data(), c->solid, c->n, cudaMemcpyDeviceToHost, c->stream));
-  WT_CUDA(c, cudaFreeAsync(dflags, c->stream));
+  uint32_t* const dcounts = c->counters + 4;
+  WT_CUDA(c, launch_block_slots(c->cellw, c->solid, c->geom, c->nx, c->ny, c->block_slot, dcounts, c->stream));
+  uint32_t counts[4];
+  WT_CUDA(c, cudaMemcpyAsync(counts, dcounts, sizeof(counts), cudaMemcpyDeviceToHost, c->stream));
   WT_CUDA(c, cudaStreamSynchronize(c->stream));
-  std::vector<int32_t> map(c->geom.nblocks);
-  uint32_t ns = 0;
-  for (uint32_t b = 0; b < c->geom.nblocks; b++) map[b] = flags[b] ? (int32_t)ns++ : -1;
+  const uint32_t ns = counts[0];
   c->nslots = ns;
-  c->fluid_cells = 0;
-  c->solid_cells[0] = c->solid_cells[1] = c->solid_cells[2] = 0;
-  for (uint64_t i = 0; i < c->n; i++) {
-    if (sol[i] == 0) c->fluid_cells++;
-    else c->solid_cells[(sol[i] - 1) % 3]++;
-  }
+  for (int k = 0; k < 3; k++) c->solid_cells[k] = counts[1 + k];
+  c->fluid_cells = (uint32_t)(c->n - counts[1] - counts[2] - counts[3]);
   // Partial records for up to WT_PENDING_MAX steps, capped at 64 MiB.
   uint64_t per_step = (uint64_t)(ns ? ns : 1) * sizeof(ForceSlot);
   uint64_t cap_steps = (64ull << 20) / per_step;
@@ -164,10 +156,7 @@ int rebuild_links(wt_ctx* c) {
     c->slot_cap = (uint32_t)need;
   }
   c->pending_cap = (uint32_t)cap_steps;
-  WT_CUDA(c, cudaMemcpyAsync(c->block_slot, map.data(), map.size() * 4, cudaMemcpyHostToDevice, c->stream));
-  ReduceArgs ra = reduce_args(c);
-  WT_CUDA(c, cudaMemcpyAsync(c->d_reduce, &ra, sizeof(ra), cudaMemcpyHostToDevice, c->stream));
-  WT_CUDA(c, cudaStreamSynchronize(c->stream));
+  WT_CUDA(c, launch_put_reduce_args(c->d_reduce, reduce_args(c), c->stream));
   c->version++;
   return WT_OK;
 }
@@ -328,7 +317,7 @@ int create_ctx(const wt_grid* grid, const wt_sim* sim, cudaStream_t ext, wt_ctx*
       (rc = dalloc(c, &c->block_slot, (uint64_t)c->geom.nblocks * 4)) ||
       (rc = dalloc(c, &c->mass_partial, (uint64_t)c->geom.nblocks * warps_per_block(c->geom) * 8)) ||
       (rc = dalloc(c, &c->hist, (uint64_t)WT_HIST_CAP * 16 * 8)) || (rc = dalloc(c, &c->totals, 18 * 8)) ||
-      (rc = dalloc(c, &c->raw_totals, 12 * 4)) || (rc = dalloc(c, &c->counters, 4 * 4)) ||
+      (rc = dalloc(c, &c->raw_totals, 12 * 4)) || (rc = dalloc(c, &c->counters, 8 * 4)) ||
       (rc = dalloc(c, &c->hist_pos, 8)) || (rc = dalloc(c, &c->d_reduce, sizeof(ReduceArgs))) ||
       (rc = dalloc(c, &c->red_part, WT_RED_PART * 8)) || (rc = dalloc(c, &c->heat_src, n * 4)))
     return cleanup(rc);
@@ -375,7 +364,8 @@ int wt_destroy(wt_ctx* c) {
   if (c->fpinned) cudaFreeHost(c->fpinned);
   for (cudaEvent_t& ev : c->fevent)
     if (ev) cudaEventDestroy(ev);
-  for (auto& g : c->graphs) cudaGraphExecDestroy(g.exec);
+  for (auto& g : c->graphs)
+    if (g.exec) cudaGraphExecDestroy(g.exec);
   void* bufs[] = {c->pop, c->cellw, c->solid, c->emit, c->fields, c->tA, c->tB, c->outlet_u, c->tau0_x,
                   c->block_slot, c->slots, c->mass_partial, c->hist, c->totals, c->raw_totals, c->counters,
                   c->hist_pos, c->d_reduce, c->car_body, c->car_parts, c->car_rig, c->red_part, c->heat_src};

@@ -283,7 +283,8 @@ int wt_batch_destroy(wt_batch* b) {
   if (!b) return WT_OK;
   cudaSetDevice(b->device);
   if (b->stream) cudaStreamSynchronize(b->stream);
-  for (auto& g : b->graphs) cudaGraphExecDestroy(g.exec);
+  for (auto& g : b->graphs)
+    if (g.exec) cudaGraphExecDestroy(g.exec);
   for (auto* c : b->lat) wt_destroy(c);
   if (b->d_args) cudaFree(b->d_args);
   if (b->d_tiles) cudaFree(b->d_tiles);

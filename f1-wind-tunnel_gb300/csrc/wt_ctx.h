@@ -50,7 +50,7 @@ struct wt_ctx {
   double* hist = nullptr;
   double* totals = nullptr;   // [9] FP64 force sums, [9] mass
   int32_t* raw_totals = nullptr;  // [12]
-  unsigned int* counters = nullptr;  // [0] guard count, [1] reduce counter
+  unsigned int* counters = nullptr;  // [0] guard count, [1] reduce counter, [4..7] force blocks and solid cells per group
   // host state
   uint64_t steps_total = 0, steps_since_read = 0, steps_recorded = 0;
   uint64_t device_bytes = 0;
@@ -76,7 +76,7 @@ struct wt_ctx {
     float dt;
     uint64_t version;
     uint32_t pend0;                        // pending records when the sequence starts
-    cudaGraphExec_t exec;
+    cudaGraphExec_t exec;                  // null until the sequence is asked for again
   };
   std::vector<Graph> graphs;               // captured wt_step sequences
   wt_shape shape{WT_KIND_EMPTY};           // last voxelized shape (the renderer's scene)
@@ -167,7 +167,10 @@ void release_renderer_buffers(wt_renderer* r);
 void release_mesh_buffers(wt_mesh* m);
 
 // Launch a step sequence through a CUDA graph captured once per (n, heat, dt)
-// and argument version; WT_NO_GRAPH=1 launches the kernels directly.
+// and argument version; WT_NO_GRAPH=1 launches the kernels directly.  A sequence is
+// captured when it is asked for the second time (its entry has no graph until
+// then): a re-voxelized lattice that runs one frame would pay for a capture and an
+// instantiation, several times its ten direct launches, and use them once.
 template <class Owner, class F>
 int run_graphed(Owner* o, std::vector<wt_ctx::Graph>& cache, uint64_t version, int n, int heat, float dt,
                 uint32_t pend0, F&& enqueue) {
@@ -180,15 +183,27 @@ int run_graphed(Owner* o, std::vector<wt_ctx::Graph>& cache, uint64_t version, i
   }
   for (size_t i = 0; i < cache.size();) {
     if (cache[i].version != version) {
-      cudaGraphExecDestroy(cache[i].exec);
+      if (cache[i].exec) cudaGraphExecDestroy(cache[i].exec);
       cache.erase(cache.begin() + i);
     } else {
       i++;
     }
   }
   cudaGraphExec_t exec = nullptr;
-  for (auto& g : cache)
-    if (g.n == n && g.heat == heat && g.dt == dt && g.pend0 == pend0) exec = g.exec;
+  size_t at = cache.size();
+  for (size_t i = 0; i < cache.size(); i++)
+    if (cache[i].n == n && cache[i].heat == heat && cache[i].dt == dt && cache[i].pend0 == pend0) at = i;
+  if (at == cache.size()) {
+    cudaError_t e = enqueue(s);
+    if (e != cudaSuccess) { o->err = std::string("kernel launch: ") + cudaGetErrorString(e); return WT_ERR_CUDA; }
+    if (cache.size() >= 16) {
+      if (cache.front().exec) cudaGraphExecDestroy(cache.front().exec);
+      cache.erase(cache.begin());
+    }
+    cache.push_back({n, heat, dt, version, pend0, nullptr});
+    return WT_OK;
+  }
+  exec = cache[at].exec;
   if (!exec) {
     cudaGraph_t graph = nullptr;
     cudaError_t e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
@@ -203,11 +218,7 @@ int run_graphed(Owner* o, std::vector<wt_ctx::Graph>& cache, uint64_t version, i
     e = cudaGraphInstantiate(&exec, graph, 0);
     cudaGraphDestroy(graph);
     if (e != cudaSuccess) { o->err = std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e); return WT_ERR_CUDA; }
-    if (cache.size() >= 16) {
-      cudaGraphExecDestroy(cache.front().exec);
-      cache.erase(cache.begin());
-    }
-    cache.push_back({n, heat, dt, version, pend0, exec});
+    cache[at].exec = exec;
   }
   cudaError_t e = cudaGraphLaunch(exec, s);
   if (e != cudaSuccess) { o->err = std::string("cudaGraphLaunch: ") + cudaGetErrorString(e); return WT_ERR_CUDA; }

@@ -163,8 +163,11 @@ cudaError_t launch_voxelize(const wt_shape& shape, const CarView& car, const wt_
 cudaError_t launch_sdf_sample(const wt_shape& shape, const wt_grid& grid, float* out, cudaStream_t s);
 cudaError_t launch_cell_words(const uint8_t* solid, const float* emit, uint32_t* cellw, uint32_t nx, uint32_t ny,
                               uint32_t nz, cudaStream_t s);
-cudaError_t launch_block_flags(const uint32_t* cellw, const StepGeom& g, uint32_t nx, uint32_t ny, uint32_t nz,
-                               uint8_t* flags, cudaStream_t s);
+// The slot of each step-kernel block's force records (-1: no force link) in block
+// order; counts[0]: slots, counts[1..3]: cells of the solid groups.
+cudaError_t launch_block_slots(const uint32_t* cellw, const uint8_t* solid, const StepGeom& g, uint32_t nx, uint32_t ny,
+                               int32_t* slots, uint32_t* counts, cudaStream_t s);
+cudaError_t launch_put_reduce_args(ReduceArgs* dst, const ReduceArgs& a, cudaStream_t s);
 cudaError_t launch_links_out(const uint32_t* cellw, uint32_t* links, uint64_t n, cudaStream_t s);
 cudaError_t launch_solid_u32(const uint8_t* solid, uint32_t* out, uint64_t n, cudaStream_t s);
 cudaError_t launch_solid_from_u32(const uint32_t* in, uint8_t* solid, uint64_t n, cudaStream_t s);

@@ -97,16 +97,64 @@ __global__ void cell_words_kernel(const uint8_t* __restrict__ solid, const float
   cellw[idx] = w;
 }
 
-__global__ void block_flags_kernel(const uint32_t* __restrict__ cellw, uint32_t nx, uint32_t ny,
-                                   uint8_t* __restrict__ flags) {
+// Per step-kernel block: whether it carries a force link, and the cells of each
+// solid group (0 fluid) added to counts[0..3].
+__global__ void block_flags_kernel(const uint32_t* __restrict__ cellw, const uint8_t* __restrict__ solid, uint32_t nx,
+                                   uint32_t ny, int32_t* __restrict__ flags, uint32_t* __restrict__ counts) {
   const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t y = blockIdx.y * blockDim.y + threadIdx.y;
   const uint32_t z = blockIdx.z;
-  bool f = false;
-  if (x < nx && y < ny) f = (cellw[x + nx * (y + ny * z)] & CW_FORCE) != 0u;
+  const bool in = x < nx && y < ny;
+  const uint32_t idx = in ? x + nx * (y + ny * z) : 0u;
+  const bool f = in && (cellw[idx] & CW_FORCE) != 0u;
+  const uint32_t v = in ? solid[idx] : 0u, g = v ? (v - 1u) % 3u + 1u : 0u;
+  const uint32_t lane = (threadIdx.x + blockDim.x * threadIdx.y) & 31u;
+#pragma unroll
+  for (uint32_t k = 1; k < 4; k++) {  // few warps hold solid cells; the fluid count follows from the others
+    const unsigned m = __ballot_sync(0xffffffffu, g == k);
+    if (m && lane == 0) atomicAdd(counts + k, (unsigned)__popc(m));
+  }
   const int any = __syncthreads_or(f);
   if (threadIdx.x == 0 && threadIdx.y == 0)
     flags[blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z)] = any ? 1 : 0;
+}
+
+// In place: flags[b] becomes the block's slot (the number of flagged blocks before
+// it), or -1; counts[0] their number.  One block, each thread a run of blocks.
+__global__ void __launch_bounds__(1024) block_slots_kernel(int32_t* __restrict__ flags, uint32_t nblocks,
+                                                           uint32_t* __restrict__ counts) {
+  __shared__ uint32_t warp_sum[32];
+  const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
+  const uint32_t per = (nblocks + 1023u) / 1024u, b0 = min(t * per, nblocks), b1 = min(b0 + per, nblocks);
+  uint32_t n = 0;
+#pragma unroll 8
+  for (uint32_t b = b0; b < b1; b++) n += (uint32_t)flags[b];
+  uint32_t inc = n;  // inclusive sums over the warp, then the warps
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t v = __shfl_up_sync(0xffffffffu, inc, d);
+    if (lane >= (uint32_t)d) inc += v;
+  }
+  if (lane == 31) warp_sum[warp] = inc;
+  __syncthreads();
+  if (warp == 0) {
+    uint32_t v = warp_sum[lane];
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t u = __shfl_up_sync(0xffffffffu, v, d);
+      if (lane >= (uint32_t)d) v += u;
+    }
+    warp_sum[lane] = v;
+  }
+  __syncthreads();
+  uint32_t slot = inc - n + (warp ? warp_sum[warp - 1] : 0u);
+#pragma unroll 8
+  for (uint32_t b = b0; b < b1; b++) {
+    const int32_t f = flags[b];
+    flags[b] = f ? (int32_t)slot : -1;
+    slot += (uint32_t)f;
+  }
+  if (t == 1023) counts[0] = slot;
 }
 
 __global__ void links_out_kernel(const uint32_t* __restrict__ cellw, uint32_t* __restrict__ links, uint64_t n) {
@@ -166,10 +214,18 @@ cudaError_t launch_cell_words(const uint8_t* solid, const float* emit, uint32_t*
   return cudaGetLastError();
 }
 
-cudaError_t launch_block_flags(const uint32_t* cellw, const StepGeom& g, uint32_t nx, uint32_t ny, uint32_t nz,
-                               uint8_t* flags, cudaStream_t s) {
-  (void)nz;
-  block_flags_kernel<<<g.grid, g.block, 0, s>>>(cellw, nx, ny, flags);
+cudaError_t launch_block_slots(const uint32_t* cellw, const uint8_t* solid, const StepGeom& g, uint32_t nx, uint32_t ny,
+                               int32_t* slots, uint32_t* counts, cudaStream_t s) {
+  cudaError_t e = cudaMemsetAsync(counts, 0, 4 * sizeof(uint32_t), s);
+  if (e != cudaSuccess) return e;
+  block_flags_kernel<<<g.grid, g.block, 0, s>>>(cellw, solid, nx, ny, slots, counts);
+  block_slots_kernel<<<1, 1024, 0, s>>>(slots, g.nblocks, counts);
+  return cudaGetLastError();
+}
+
+__global__ void put_reduce_args_kernel(ReduceArgs* dst, ReduceArgs a) { *dst = a; }
+cudaError_t launch_put_reduce_args(ReduceArgs* dst, const ReduceArgs& a, cudaStream_t s) {
+  put_reduce_args_kernel<<<1, 1, 0, s>>>(dst, a);
   return cudaGetLastError();
 }
 
