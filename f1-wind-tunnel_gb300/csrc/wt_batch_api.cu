@@ -1,5 +1,5 @@
 // The C ABI of the block-shape autotuner and of batches (many lattices advanced
-// by one kernel launch per step: the aero-map sweep, src/ui/aeromap.ts:73-114).
+// together: the aero-map sweep, src/ui/aeromap.ts:73-114).
 #include <cuda_runtime.h>
 #include <stdio.h>
 #include <stdlib.h>
@@ -129,7 +129,7 @@ int wt_tune(wt_ctx* c, uint32_t* bx_out, uint32_t* by_out, float* ms_out) {
 }  // extern "C"
 
 // ---------------------------------------------------------------------------
-// Batches: many lattices advanced by one kernel launch per step.
+// Batches: many lattices advanced together.
 // ---------------------------------------------------------------------------
 namespace {
 
@@ -192,6 +192,83 @@ int refresh_batch(wt_batch* b) {
   return WT_OK;
 }
 
+// How a batch runs its steps.  The lattices are independent, so each can run its whole
+// call as a chain of single-lattice launches (plain-neighbour path, slot tables in the
+// parameter block, a lattice's lines staying in the L2 from step to step), several
+// chains at a time on side streams so that one's launch latency and last wave (4 us,
+// whatever the lattice's size) hide behind another's blocks.  Measured against one
+// launch per step for all lattices (us per step, f16): 25 x 256x96x80 + 8 uneven 2079
+// -> 1368 with one chain at a time; 8 of 128x48x40 .. 256x96x80 239 -> 156 with two;
+// 16 x 128x48x40 126 -> 77 with four; 64 x 96x36x30 250 -> 173 with eight.  Below about
+// 64k cells a lattice the chains' latencies no longer hide (32 x 64x24x20: 51 against
+// 62) and one launch for all is faster.  So: chains for about a million cells.
+uint32_t batch_lanes(const wt_batch* b) {
+  uint64_t cells = 0;
+  for (auto* c : b->lat) cells += c->n;
+  const uint64_t avg = cells / b->lat.size();
+  if (avg < 65536) return 0;
+  return (uint32_t)std::min({(uint64_t)b->lat.size(), (uint64_t)WT_BATCH_LANES, 1 + 1000000 / avg});
+}
+
+cudaError_t enqueue_lanes(wt_batch* b, uint32_t lanes, int n, int heat_passes, float dt, cudaStream_t s) {
+  cudaError_t e;
+  for (uint32_t j = 0; j <= lanes; j++) {  // event `lanes` marks the fork
+    if (j < lanes && !b->side[j] && (e = cudaStreamCreateWithFlags(&b->side[j], cudaStreamNonBlocking)) != cudaSuccess) return e;
+    if (!b->joined[j] && (e = cudaEventCreateWithFlags(&b->joined[j], cudaEventDisableTiming)) != cudaSuccess) return e;
+  }
+  // largest first, each to the lane with the least work
+  std::vector<wt_ctx*> order(b->lat);
+  std::stable_sort(order.begin(), order.end(), [](wt_ctx* x, wt_ctx* y) { return x->n > y->n; });
+  std::vector<std::vector<wt_ctx*>> plan(lanes);
+  std::vector<uint64_t> load(lanes, 0);
+  for (auto* c : order) {
+    const size_t j = std::min_element(load.begin(), load.end()) - load.begin();
+    plan[j].push_back(c);
+    load[j] += c->n + 100000;
+  }
+  if ((e = cudaEventRecord(b->joined[lanes], s)) != cudaSuccess) return e;
+  for (uint32_t j = 0; j < lanes; j++)
+    if ((e = cudaStreamWaitEvent(b->side[j], b->joined[lanes], 0)) != cudaSuccess) return e;
+  // the lanes' launches in turns of 16 steps, so that all are fed when they run directly
+  struct At {
+    size_t lat = 0;
+    int k = 0;
+    uint32_t pending = 0;
+  };
+  std::vector<At> at(lanes);
+  e = cudaSuccess;
+  for (bool more = true; more && e == cudaSuccess;) {
+    more = false;
+    for (uint32_t j = 0; j < lanes && e == cudaSuccess; j++) {
+      At& p = at[j];
+      if (p.lat == plan[j].size()) continue;
+      more = true;
+      wt_ctx* c = plan[j][p.lat];
+      StepArgs a = step_args(c);
+      for (int i = 0; i < 16 && p.k < n && e == cudaSuccess; i++, p.k++) {
+        const bool last = p.k == n - 1;
+        a.slots = c->slots + (size_t)p.pending * (c->nslots ? c->nslots : 1);
+        e = launch_step(b->storage, (p.k & 1) == 0, last, c->geom, a, b->side[j]);
+        if (e == cudaSuccess && (++p.pending == c->pending_cap || last)) {
+          e = launch_force_reduce(c->d_reduce, 1, p.pending, last, b->side[j]);
+          p.pending = 0;
+        }
+      }
+      if (e == cudaSuccess && p.k == n) {
+        e = enqueue_heat(c, heat_passes, dt, b->side[j]);
+        p.lat++;
+        p.k = 0;
+      }
+    }
+  }
+  for (uint32_t j = 0; j < lanes; j++) {  // also after a failure: a capture must end joined
+    cudaError_t r = cudaEventRecord(b->joined[j], b->side[j]);
+    if (r == cudaSuccess) r = cudaStreamWaitEvent(s, b->joined[j], 0);
+    if (e == cudaSuccess) e = r;
+  }
+  return e;
+}
+
 cudaError_t enqueue_batch(wt_batch* b, int n, int heat_passes, float dt, cudaStream_t s) {
   const uint32_t count = (uint32_t)b->lat.size();
   const dim3 block(b->bx, b->by, 1);
@@ -219,6 +296,8 @@ cudaError_t enqueue_batch(wt_batch* b, int n, int heat_passes, float dt, cudaStr
     // the barrier's expiry flag, read back by the next call
     cudaError_t e = cudaMemcpyAsync(b->h_flag, b->d_sync + 1, sizeof(unsigned int), cudaMemcpyDeviceToHost, s);
     if (e != cudaSuccess) return e;
+  } else if (const uint32_t lanes = batch_lanes(b)) {
+    return enqueue_lanes(b, lanes, n, heat_passes, dt, s);
   } else {
     for (int k = 0; k < n; k++) {
       const bool last = (k == n - 1);
@@ -286,6 +365,10 @@ int wt_batch_destroy(wt_batch* b) {
   for (auto& g : b->graphs)
     if (g.exec) cudaGraphExecDestroy(g.exec);
   for (auto* c : b->lat) wt_destroy(c);
+  for (auto& st : b->side)
+    if (st) cudaStreamDestroy(st);
+  for (auto& ev : b->joined)
+    if (ev) cudaEventDestroy(ev);
   if (b->d_args) cudaFree(b->d_args);
   if (b->d_tiles) cudaFree(b->d_tiles);
   if (b->d_reduce) cudaFree(b->d_reduce);
@@ -314,9 +397,15 @@ int wt_batch_step(wt_batch* b, int n_lbm_steps, int heat_passes, float heat_dt) 
   const float dt = heat_dt > 0.0f ? heat_dt : (float)n_lbm_steps / 2.0f;
   for (auto* c : b->lat)
     if ((rc = flush_forces(c))) return bfail(b, rc, c->err);
-  if ((rc = run_graphed(b, b->graphs, b->version, n_lbm_steps, heat_passes, dt, 0u,
-                        [&](cudaStream_t s) { return enqueue_batch(b, n_lbm_steps, heat_passes, dt, s); })))
+  const auto enqueue = [&](cudaStream_t s) { return enqueue_batch(b, n_lbm_steps, heat_passes, dt, s); };
+  if (!b->persist && batch_lanes(b) && (uint64_t)n_lbm_steps * b->lat.size() > 8192) {
+    // a graph of every lattice's steps would be instantiated for longer than it saves;
+    // the direct launches are far enough ahead of the lattices' kernels
+    cudaError_t e = enqueue(b->stream);
+    if (e != cudaSuccess) return bfail(b, WT_ERR_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e));
+  } else if ((rc = run_graphed(b, b->graphs, b->version, n_lbm_steps, heat_passes, dt, 0u, enqueue))) {
     return rc;
+  }
   for (auto* c : b->lat) {
     c->steps_total += n_lbm_steps;
     c->steps_since_read += n_lbm_steps;

@@ -15,6 +15,7 @@
 #include "wt_internal.h"
 
 #define WT_ASYNC_SLOTS 16  // force readbacks in flight per context
+#define WT_BATCH_LANES 8   // lattices of a batch that step side by side at most
 
 struct wt_renderer;
 struct wt_mesh;
@@ -112,6 +113,9 @@ struct wt_batch {
   uint32_t persist_grid = 0;
   unsigned int* d_sync = nullptr;
   unsigned int* h_flag = nullptr;
+  // side streams of the lattices' step chains and the events that fork and join them
+  cudaStream_t side[WT_BATCH_LANES] = {};
+  cudaEvent_t joined[WT_BATCH_LANES + 1] = {};
   uint64_t version = ~0ull;                // sum of member versions the device tables were built for
   std::vector<wt_ctx::Graph> graphs;
   std::string err;

@@ -416,9 +416,9 @@ class AeroEngine:
 
 
 class AeroBatch:
-    """Many lattices advanced together by one kernel launch per step, or by one
-    persistent launch per up to 64 steps (the aero-map sweep of
-    src/ui/aeromap.ts:73-114 run as concurrent cases).
+    """Many lattices advanced together, by side-by-side chains of launches, by one
+    kernel launch per step (small lattices) or by one persistent launch per up to 64
+    steps (the aero-map sweep of src/ui/aeromap.ts:73-114 run as concurrent cases).
     `lattices[i]` is an AeroEngine view of lattice i for voxelize/read calls."""
 
     def __init__(self, grids, sim=None, lib=None):

@@ -490,9 +490,10 @@ int wt_tune(wt_ctx* ctx, uint32_t* bx, uint32_t* by, float* ms_per_step);
  * No single reference function: the reference runs one lattice and sweeps the
  * aero map point by point (src/ui/aeromap.ts:73-114, re-voxelizing per point
  * through engine.ts:469).  A batch holds `count` lattices of any sizes with the
- * same simulation parameters; one kernel launch per LBM step covers every
- * lattice's blocks, and the launches of a wt_batch_step call are captured once
- * into a CUDA graph and replayed.  Each lattice is an ordinary wt_ctx
+ * same simulation parameters; a wt_batch_step call runs every lattice's steps as a
+ * chain of launches of its own, as many chains side by side as fill the device, or,
+ * for small lattices, one kernel launch per LBM step over every lattice's blocks, and
+ * a repeated call replays them as a CUDA graph.  Each lattice is an ordinary wt_ctx
  * (wt_batch_lattice): voxelize, reset, read forces and fields with the single-
  * lattice calls; do not wt_destroy it. */
 typedef struct wt_batch wt_batch;
@@ -502,13 +503,13 @@ uint32_t wt_batch_count(const wt_batch* batch);
 wt_ctx* wt_batch_lattice(wt_batch* batch, uint32_t index);
 /* n_lbm_steps / heat_passes / heat_dt as wt_step, for every lattice. */
 int wt_batch_step(wt_batch* batch, int n_lbm_steps, int heat_passes, float heat_dt);
-/* Autotuner over the block shapes for the whole batch, each timed with one
- * launch per LBM step and with the persistent launch (state saved and
+/* Autotuner over the block shapes for the whole batch, each timed with launches
+ * per LBM step and with the persistent launch (state saved and
  * restored).  The environment variable WT_BATCH_PERSIST=0/1, read at
  * wt_batch_create, fixes the launch kind instead. */
 int wt_batch_tune(wt_batch* batch, uint32_t* bx, uint32_t* by, float* ms_per_step);
 /* Grid of the batch's persistent launch (blocks resident at once), or 0 when the
- * batch launches its kernel once per LBM step.  In the persistent launch, one
+ * batch launches kernels per LBM step.  In the persistent launch, one
  * cooperative kernel advances every lattice by up to 64 steps (the force-record
  * capacity), with a grid barrier between steps; the barrier's wait is bounded,
  * and an expired wait is reported as WT_ERR_CUDA by the next wt_batch_step. */
