@@ -36,11 +36,14 @@ __host__ __device__ constexpr float Wd(int i) { return i == 0 ? 0.33333334f : (i
 //   bit 19     belt contact: floor speed 0 under this y=0 cell (wgsl.ts:192-197)
 //   bit 20     duct cell (emit < 0): no force, axial velocity relaxation (wgsl.ts:201,248)
 //   bit 21     at least one force-carrying link (non-mirrored, not a duct cell)
+//   bits 22-23 the solid group that all of the cell's non-mirrored links bounce off,
+//              0 where they differ
 constexpr uint32_t CW_SOLID = 1u;
 constexpr uint32_t CW_LINKS = 0x7fffeu;
 constexpr uint32_t CW_BELT = 1u << 19;
 constexpr uint32_t CW_DUCT = 1u << 20;
 constexpr uint32_t CW_FORCE = 1u << 21;
+constexpr uint32_t CW_GROUP_SHIFT = 22;
 
 // Compile-time loop: f(std::integral_constant<int, I>) for I = 0..N-1.
 template <int... Is, class F>

@@ -511,36 +511,37 @@ __device__ __forceinline__ void step_tile(const StepArgs& a, const Ofs& ofs, For
         }
       });
     } else {
+      // All 19 loads first, each from a selected slot (directions whose value comes
+      // from a boundary condition load the cell's own slot), then the boundary values:
+      // with the loads inside the precedence's branches each waited for its own round
+      // trip to the L2, 3 us of a launch's critical path.
       sfor<19>([&](auto I) {
         constexpr int i = I;
         constexpr int cx = CXd(i), cy = CYd(i), cz = CZd(i);
-        if constexpr (i == 0) {
-          f[0] = ldr<St, !LOOP>(a.pop, 0, np, idx);
-        } else {
-          float v;
-          if (cx > 0 && x == 0) {
-            v = R::feq_in(a, i);
-          } else if (cx < 0 && x == nx - 1) {
-            v = R::template outlet<i>(pu.x, pu.y, pu.z);
-          } else if (cy > 0 && y == 0) {
-            v = ldr<St, !LOOP>(a.pop, i, np, idx);
-            if constexpr (cx != 0) v = v + R::floor_k(a, i) * floor_u;
-          } else if ((cy < 0 && y == ny - 1) || (cz < 0 && z == nz - 1)) {
-            v = R::feq_in(a, i);
-          } else if (GATHER) {
-            if ((cw >> i) & 1u) {
-              v = ldr<St, !LOOP>(a.pop, i, np, idx);
-            } else if (cz > 0 && z == 0) {
-              v = ldr<St, !LOOP>(a.pop, OPPd(ZMIRd(i)), np, (uint32_t)((int)idx - cx - cy * (int)nx));
-            } else {
-              const int off = cx + cy * (int)nx + cz * (int)nxy;
-              v = ldr<St, !LOOP>(a.pop, OPPd(i), np, (uint32_t)((int)idx - off));
-            }
-          } else {
-            v = ldr<St, !LOOP>(a.pop, i, np, idx);
-          }
-          f[i] = v;
+        uint32_t slot = (uint32_t)i * np + idx;
+        if constexpr (GATHER && i != 0) {
+          const bool own = ((cw >> i) & 1u) || (cx > 0 && x == 0) || (cx < 0 && x == nx - 1) || (cy > 0 && y == 0) ||
+                           (cy < 0 && y == ny - 1) || (cz < 0 && z == nz - 1);
+          const int off = cx + cy * (int)nx + cz * (int)nxy;
+          uint32_t from = (uint32_t)OPPd(i) * np + (uint32_t)((int)idx - off);
+          if constexpr (cz > 0)
+            if (z == 0) from = (uint32_t)OPPd(ZMIRd(i)) * np + (uint32_t)((int)idx - cx - cy * (int)nx);
+          slot = own ? slot : from;
         }
+        f[i] = R::ld(P + slot, i);
+      });
+      sfor<19>([&](auto I) {
+        constexpr int i = I;
+        constexpr int cx = CXd(i), cy = CYd(i), cz = CZd(i);
+        if constexpr (cy < 0 || cz < 0)
+          if ((cy < 0 && y == ny - 1) || (cz < 0 && z == nz - 1 && !(cy > 0 && y == 0))) f[i] = R::feq_in(a, i);
+        if constexpr (cy > 0 && cx != 0)
+          if (y == 0) f[i] = f[i] + R::floor_k(a, i) * floor_u;
+        if constexpr (cx < 0) {
+          const float e = R::template outlet<i>(pu.x, pu.y, pu.z);
+          f[i] = (x == nx - 1) ? e : f[i];
+        }
+        if constexpr (cx > 0) f[i] = (x == 0) ? R::feq_in(a, i) : f[i];
       });
     }
     if (!yzface) {  // inlet / outlet directions of the x-face lanes (wgsl.ts:207-210)
@@ -561,19 +562,37 @@ __device__ __forceinline__ void step_tile(const StepArgs& a, const Ofs& ofs, For
     }
 
     // ---------------------------------------------------------------- forces
+    // Blocks with force links and face rows set the latency of a step: a lattice of any
+    // size waited 6 us for the links' dependent flag loads and the FP64 trees of all
+    // nine sums, and 3 us for the faces' serial loads.  Group in the cell word, trees per
+    // group present and loads ahead of the boundary cases: 168x50x38 f32 18.5 -> 14.1 us
+    // a step, 128x48x40 f16 15.6 -> 9.0, 256x96x80 f32 / f16 56.6 / 42.9 -> 53.3 / 37.5,
+    // 512x192x160 f16 315 -> 301.
     if (cw & CW_FORCE) {
-      sfor<19>([&](auto I) {
-        constexpr int i = I;
-        if constexpr (i != 0) {
-          constexpr int cx = CXd(i), cy = CYd(i), cz = CZd(i);
-          const bool mirrored = (cz > 0) && (z == 0);
-          if (((cw >> i) & 1u) && !mirrored) {
-            const int off = cx + cy * (int)nx + cz * (int)nxy;
-            const uint32_t grp = __ldg(solid_u8 + (uint32_t)((int)idx - off));
-            link_force<i, R>(f[i], grp, gf);
+      const uint32_t group = (cw >> CW_GROUP_SHIFT) & 3u;
+      if (group) {  // every force link of this cell bounces off one group: no flags to read
+        float tf[9] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        sfor<19>([&](auto I) {
+          constexpr int i = I;
+          if constexpr (i != 0)
+            if (((cw >> i) & 1u) && !(CZd(i) > 0 && z == 0)) link_force<i, R>(f[i], 1u, tf);
+        });
+#pragma unroll
+        for (int k = 0; k < 9; k++) gf[k] = group == (uint32_t)(k / 3 + 1) ? tf[k % 3] : 0.0f;
+      } else {
+        sfor<19>([&](auto I) {
+          constexpr int i = I;
+          if constexpr (i != 0) {
+            constexpr int cx = CXd(i), cy = CYd(i), cz = CZd(i);
+            const bool mirrored = (cz > 0) && (z == 0);
+            if (((cw >> i) & 1u) && !mirrored) {
+              const int off = cx + cy * (int)nx + cz * (int)nxy;
+              const uint32_t grp = __ldg(solid_u8 + (uint32_t)((int)idx - off));
+              link_force<i, R>(f[i], grp, gf);
+            }
           }
-        }
-      });
+        });
+      }
     }
 
     // ---------------------------------------------------------------- collide
@@ -661,51 +680,43 @@ __device__ __forceinline__ void step_tile(const StepArgs& a, const Ofs& ofs, For
   if (slot < 0) return;  // no force-carrying link in this block: no barrier, no record
   __shared__ double s_f[9][8];
   __shared__ int32_t s_r[6][8];
-  bool any_force = false;
+  // Per group with a force in this warp (mostly one or none): three FP64 shuffle trees,
+  // the i32 sums by one reduction instruction each.
 #pragma unroll
-  for (int q = 0; q < 9; q++) any_force |= (gf[q] != 0.0f);
-  if (!__any_sync(0xffffffffu, any_force)) {  // no force in this warp: zero record, no FP64 shuffles
-    if (lane < 9) s_f[lane][warp] = 0.0;
-    if (lane < 6) s_r[lane][warp] = 0;
-  } else {
-    double d[9];
-    int32_t r[6];
+  for (int g = 0; g < 3; g++) {
+    const float fx = gf[3 * g], fy = gf[3 * g + 1], fz = gf[3 * g + 2];
+    if (!__any_sync(0xffffffffu, fx != 0.0f || fy != 0.0f || fz != 0.0f)) {
+      if (lane < 3) s_f[3 * g + lane][warp] = 0.0;
+      if (lane < 2) s_r[2 * g + lane][warp] = 0;
+    } else {
+      double d[3] = {(double)fx, (double)fy, (double)fz};
+      const int32_t rx = (fx != 0.0f) ? __float2int_rn(fx * 10000.0f) : 0, ry = (fy != 0.0f) ? __float2int_rn(fy * 10000.0f) : 0;
+      const uint32_t sx = __reduce_add_sync(0xffffffffu, (uint32_t)rx), sy = __reduce_add_sync(0xffffffffu, (uint32_t)ry);
 #pragma unroll
-    for (int q = 0; q < 9; q++) d[q] = (double)gf[q];
+      for (int s = 16; s > 0; s >>= 1) {
 #pragma unroll
-    for (int g = 0; g < 3; g++) {
-      r[2 * g] = (gf[3 * g] != 0.0f) ? __float2int_rn(gf[3 * g] * 10000.0f) : 0;
-      r[2 * g + 1] = (gf[3 * g + 1] != 0.0f) ? __float2int_rn(gf[3 * g + 1] * 10000.0f) : 0;
-    }
+        for (int q = 0; q < 3; q++) d[q] += __shfl_down_sync(0xffffffffu, d[q], s);
+      }
+      if (lane == 0) {
 #pragma unroll
-    for (int s = 16; s > 0; s >>= 1) {
-#pragma unroll
-      for (int q = 0; q < 9; q++) d[q] += __shfl_down_sync(0xffffffffu, d[q], s);
-#pragma unroll
-      for (int q = 0; q < 6; q++) r[q] = (int32_t)((uint32_t)r[q] + (uint32_t)__shfl_down_sync(0xffffffffu, r[q], s));
-    }
-    if (lane == 0) {
-#pragma unroll
-      for (int q = 0; q < 9; q++) s_f[q][warp] = d[q];
-#pragma unroll
-      for (int q = 0; q < 6; q++) s_r[q][warp] = r[q];
+        for (int q = 0; q < 3; q++) s_f[3 * g + q][warp] = d[q];
+        s_r[2 * g][warp] = (int32_t)sx;
+        s_r[2 * g + 1][warp] = (int32_t)sy;
+      }
     }
   }
   __syncthreads();
-  if (threadIdx.x == 0 && threadIdx.y == 0) {
-    ForceSlot& out = slots[slot];
-    for (int q = 0; q < 9; q++) {
-      double tt = 0.0;
-      for (uint32_t w = 0; w < nwarps; w++) tt += s_f[q][w];
-      out.f[q] = tt;
-    }
-    for (int q = 0; q < 6; q++) {
-      uint32_t tt = 0;
-      for (uint32_t w = 0; w < nwarps; w++) tt += (uint32_t)s_r[q][w];
-      out.raw[q] = (int32_t)tt;
-    }
+  const uint32_t tid = threadIdx.x + blockDim.x * threadIdx.y;  // one thread per sum, the warps in order
+  if (tid < 9) {
+    double tt = 0.0;
+    for (uint32_t w = 0; w < nwarps; w++) tt += s_f[tid][w];
+    slots[slot].f[tid] = tt;
+  } else if (tid < 15) {
+    uint32_t tt = 0;
+    for (uint32_t w = 0; w < nwarps; w++) tt += (uint32_t)s_r[tid - 9][w];
+    slots[slot].raw[tid - 9] = (int32_t)tt;
   }
-  if constexpr (LOOP) __syncthreads();  // thread 0 has read s_f / s_r before the next tile writes them
+  if constexpr (LOOP) __syncthreads();  // s_f / s_r have been read before the next tile writes them
 }
 
 // Consecutive collide-stream launches are chained by programmatic dependent

@@ -74,6 +74,7 @@ __global__ void cell_words_kernel(const uint8_t* __restrict__ solid, const float
   uint32_t w = 0u;
   const bool duct = emit[idx] < 0.0f;
   bool force = false;
+  uint32_t groups = 0u;  // bit g: a non-mirrored link off group g
   sfor<19>([&](auto I) {
     constexpr int i = I;
     if constexpr (i != 0) {
@@ -81,9 +82,13 @@ __global__ void cell_words_kernel(const uint8_t* __restrict__ solid, const float
       const int sx = (int)x - cx, sy = (int)y - cy, sz = (int)z - cz;
       // precedence of wgsl.ts:207-221: inlet, outlet, floor, far field come first
       if (sx < 0 || sx >= (int)nx || sy < 0 || sy >= (int)ny || sz >= (int)nz) return;
-      if (tile[lz - cz][ly - cy][lx - cx]) {  // z = -1 reads the clamped (mirrored) z = 0 flag
+      const uint32_t g = tile[lz - cz][ly - cy][lx - cx];
+      if (g) {  // z = -1 reads the clamped (mirrored) z = 0 flag
         w |= 1u << i;
-        if (!(sz < 0)) force = true;
+        if (!(sz < 0)) {
+          force = true;
+          groups |= 1u << g;
+        }
       }
     }
   });
@@ -94,6 +99,7 @@ __global__ void cell_words_kernel(const uint8_t* __restrict__ solid, const float
   }
   if (duct) w |= CW_DUCT;
   if (force && !duct) w |= CW_FORCE;
+  if (groups == 2u || groups == 4u || groups == 8u) w |= (groups == 2u ? 1u : groups == 4u ? 2u : 3u) << CW_GROUP_SHIFT;
   cellw[idx] = w;
 }
 
