@@ -117,6 +117,7 @@ ReduceArgs reduce_args(const wt_ctx* c) {
   r.nmass = c->geom.nblocks * warps_per_block(c->geom);
   r.mass_out = c->totals + 9;
   r.counter = c->counters + 1;
+  r.guard = c->counters;
   r.part = c->red_part;
   return r;
 }
@@ -521,11 +522,17 @@ int wt_read_forces_async(wt_ctx* c, int reset, uint64_t* ticket) {
     WT_CUDA(c, cudaHostGetDevicePointer((void**)&c->fpinned_dev, c->fpinned, 0));
     for (cudaEvent_t& ev : c->fevent) WT_CUDA(c, cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
   }
-  if ((rc = flush_forces(c))) return rc;
   const uint32_t slot = (uint32_t)(c->fticket % WT_ASYNC_SLOTS);
   if (c->fticket >= WT_ASYNC_SLOTS) WT_CUDA(c, cudaEventSynchronize(c->fevent[slot]));  // slot reused
-  WT_CUDA(c, launch_force_readback(c->totals, c->raw_totals, c->counters, c->fpinned_dev + slot, c->steps_since_read,
-                                   reset, c->stream));
+  if (c->pending || c->mass_pending) {  // the pending reduction hands its results over itself
+    WT_CUDA(c, launch_force_reduce(c->d_reduce, 1, c->pending, c->mass_pending, c->stream, c->fpinned_dev + slot,
+                                   c->steps_since_read, reset));
+    c->pending = 0;
+    c->mass_pending = false;
+  } else {
+    WT_CUDA(c, launch_force_readback(c->totals, c->raw_totals, c->counters, c->fpinned_dev + slot, c->steps_since_read,
+                                     reset, c->stream));
+  }
   WT_CUDA(c, cudaEventRecord(c->fevent[slot], c->stream));
   if (reset) c->steps_since_read = 0;
   *ticket = c->fticket++;

@@ -130,10 +130,13 @@ struct ReduceArgs {
   uint32_t nmass;
   double* mass_out;
   unsigned int* counter;
+  unsigned int* guard;  // cells reset by the divergence guard
   double* part;  // WT_RED_PART doubles: chunk sums of the force records, then of the mass
 };
+// out (one lattice, host-mapped): also hand the accumulators over and, with reset, zero
+// them, as launch_force_readback does where nothing is pending.
 cudaError_t launch_force_reduce(const ReduceArgs* args, uint32_t count, uint32_t nsteps, bool with_mass,
-                                cudaStream_t s);
+                                cudaStream_t s, wt_forces* out = nullptr, uint64_t steps = 0, int reset = 0);
 // The force accumulators (FP64 totals[10]: sums and mass, raw i32[12], guard
 // counter) into *out, a wt_forces in host-mapped memory; zeroed after if reset.
 cudaError_t launch_force_readback(double* totals, int32_t* raw, unsigned int* counters, wt_forces* out,

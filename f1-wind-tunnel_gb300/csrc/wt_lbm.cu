@@ -986,11 +986,6 @@ __global__ void coarse_average_kernel(const float4* __restrict__ fields, const u
                   : make_float4(0.0f, 0.0f, 0.0f, 1.0f);
 }
 
-// Deterministic reduction of the pending steps' partial records: block s < nsteps
-// sums step s's records (each thread a fixed strided subset with all 15
-// components in registers, then a fixed shuffle tree and the warps in order)
-// into the history ring; block nsteps sums the mass partials; the last block to
-// finish folds the steps into the running totals in step order.
 constexpr uint32_t RED_THREADS = 256;
 constexpr uint32_t RED_FCHUNKS = WT_RED_FCHUNKS, RED_MCHUNKS = WT_RED_MCHUNKS;
 
@@ -1007,59 +1002,88 @@ __device__ __forceinline__ double block_sum_d(double v, double* sm) {
   return t;
 }
 
+// Where a reduction that a readback asked for leaves its results (host-mapped memory;
+// out null: no readback).
+struct Readback {
+  wt_forces* out;
+  uint64_t steps;
+  int reset;
+};
+
 // Pending steps' per-block force records into per-step history records and the
 // totals, and the per-warp mass partials into the mass.  Each step's records
 // are split into RED_FCHUNKS fixed ranges and the mass partials into
 // RED_MCHUNKS, one block each; the last block to finish combines the chunk sums
-// in chunk order.  The order of every sum is fixed, so the result is the same
-// on every run.
+// and, for a readback, hands the totals over.  The order of every sum is fixed, so
+// the result is the same on every run.
+// A readback waits for this kernel, so it is its latency that counts: FP64 additions
+// run at 1/64 of the FP32 rate, so records go through shared memory and are summed by
+// RED_PARTS threads per component (a warp tree spends 32 lanes on each of its sums, and
+// issues five additions for nine components), and so are the totals over the steps.
+// A frame of 8 steps with its readback, beyond the steps: 168x50x38 26.5 -> 20.1 us,
+// 232x68x52 36.3 -> 31.8 (the heat passes, 10 and 19 us, are part of both); the reduce of 8 steps
+// takes 10.3 us where it and a readback launch of its own took 14 and 2.
+constexpr uint32_t RED_PARTS = 16;
+static_assert(9 * RED_PARTS <= RED_THREADS && RED_THREADS >= 64 + WT_PENDING_MAX / 2, "force_reduce_kernel's shared rows");
+
 __global__ void __launch_bounds__(RED_THREADS) force_reduce_kernel(const ReduceArgs* __restrict__ all, uint32_t nsteps,
-                                                                   uint32_t with_mass) {
+                                                                   uint32_t with_mass, Readback rb) {
   // chained like the step kernels: the next launch may be scheduled now; wait
   // for the steps whose records this reads
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
   __shared__ double sm[RED_THREADS / 32];
-  __shared__ double smf[9][RED_THREADS / 32];
+  __shared__ double rec[9][RED_THREADS + 1];                   // this block's records; later the steps' sums
+  __shared__ double part[9][RED_PARTS + 1];
   __shared__ uint32_t smr[6][RED_THREADS / 32];
   __shared__ bool last;
   const ReduceArgs& ra = all[blockIdx.y];
   const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
-  const uint64_t hist_base = *ra.hist_pos;
   const uint32_t nforce = nsteps * RED_FCHUNKS;
   double* const mpart = ra.part + (size_t)WT_PENDING_MAX * RED_FCHUNKS * 16;
   if (blockIdx.x < nforce) {
     const uint32_t step = blockIdx.x / RED_FCHUNKS, chunk = blockIdx.x % RED_FCHUNKS;
     const uint32_t per = (ra.nslots + RED_FCHUNKS - 1) / RED_FCHUNKS;
-    const uint32_t s0 = chunk * per, s1 = min(s0 + per, ra.nslots);
+    const uint32_t s0 = min(chunk * per, ra.nslots), s1 = min(s0 + per, ra.nslots);
     const ForceSlot* base = ra.slots + (size_t)step * ra.nslots;
     double acc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
     uint32_t racc[6] = {0, 0, 0, 0, 0, 0};
-    for (uint32_t s = s0 + t; s < s1; s += RED_THREADS) {
+    if (s0 + t < s1) {
+      const ForceSlot r = base[s0 + t];
+#pragma unroll
+      for (int k = 0; k < 9; k++) acc[k] = r.f[k];
+#pragma unroll
+      for (int k = 0; k < 6; k++) racc[k] = (uint32_t)r.raw[k];
+    }
+    for (uint32_t s = s0 + t + RED_THREADS; s < s1; s += RED_THREADS) {
       const ForceSlot r = base[s];
 #pragma unroll
       for (int k = 0; k < 9; k++) acc[k] += r.f[k];
 #pragma unroll
       for (int k = 0; k < 6; k++) racc[k] += (uint32_t)r.raw[k];
     }
-    double* out = ra.part + (size_t)blockIdx.x * 16;
-    // the nine FP64 sums and six integer sums together: warp trees (as
-    // block_sum_d forms them), one barrier, then the warps in order
 #pragma unroll
-    for (int s = 16; s > 0; s >>= 1) {
+    for (int k = 0; k < 9; k++) rec[k][t] = acc[k];
 #pragma unroll
-      for (int k = 0; k < 9; k++) acc[k] += __shfl_down_sync(0xffffffffu, acc[k], s);
-#pragma unroll
-      for (int k = 0; k < 6; k++) racc[k] += __shfl_down_sync(0xffffffffu, racc[k], s);
-    }
-    if (lane == 0) {
-      for (int k = 0; k < 9; k++) smf[k][warp] = acc[k];
-      for (int k = 0; k < 6; k++) smr[k][warp] = racc[k];
+    for (int k = 0; k < 6; k++) {
+      const uint32_t v = __reduce_add_sync(0xffffffffu, racc[k]);
+      if (lane == 0) smr[k][warp] = v;
     }
     __syncthreads();
-    if (t < 9) {
+    const uint32_t n = min(s1 - s0, RED_THREADS);  // records in shared memory
+    if (t < 9 * RED_PARTS) {
+      const uint32_t k = t / RED_PARTS, p = t % RED_PARTS;
       double v = 0.0;
-      for (uint32_t w = 0; w < RED_THREADS / 32; w++) v += smf[t][w];
+      if (p < n) v = rec[k][p];
+      for (uint32_t s = p + RED_PARTS; s < n; s += RED_PARTS) v += rec[k][s];
+      part[k][p] = v;
+    }
+    __syncthreads();
+    double* out = ra.part + (size_t)blockIdx.x * 16;
+    if (t < 9) {
+      double v = part[t][0];
+#pragma unroll
+      for (uint32_t p = 1; p < RED_PARTS; p++) v += part[t][p];
       out[t] = v;
     } else if (t < 15) {
       uint32_t v = 0;
@@ -1080,41 +1104,72 @@ __global__ void __launch_bounds__(RED_THREADS) force_reduce_kernel(const ReduceA
   __syncthreads();
   if (!last) return;
   __threadfence();
+  const uint64_t hist_base = *ra.hist_pos % ra.hist_cap;
   for (uint32_t i = t; i < nsteps * 16; i += RED_THREADS) {  // per-step records, chunks in order
     const uint32_t step = i / 16, k = i % 16;
     if (k >= 15) continue;
     const double* in = ra.part + (size_t)step * RED_FCHUNKS * 16 + k;
-    double* rec = ra.hist + ((hist_base + step) % ra.hist_cap) * 16;
+    uint64_t at = hist_base + step;
+    if (at >= ra.hist_cap) at -= ra.hist_cap;
+    double* h = ra.hist + at * 16;
+    double c[RED_FCHUNKS];
+#pragma unroll
+    for (uint32_t q = 0; q < RED_FCHUNKS; q++) c[q] = in[(size_t)q * 16];
     if (k < 9) {
-      double v = 0.0;
-      for (uint32_t c = 0; c < RED_FCHUNKS; c++) v += in[(size_t)c * 16];
-      rec[k] = v;
+      double v = c[0];
+#pragma unroll
+      for (uint32_t q = 1; q < RED_FCHUNKS; q++) v += c[q];
+      h[k] = v;
+      rec[k][step] = v;
     } else {
       uint32_t v = 0;
-      for (uint32_t c = 0; c < RED_FCHUNKS; c++) v += (uint32_t)in[(size_t)c * 16];
-      rec[k] = (double)(int32_t)v;
+#pragma unroll
+      for (uint32_t q = 0; q < RED_FCHUNKS; q++) v += (uint32_t)c[q];
+      h[k] = (double)(int32_t)v;
+      // column 64 on: the steps' i32 sums (nsteps <= 64)
+      reinterpret_cast<uint32_t*>(&rec[k - 9][64])[step] = v;
     }
   }
+  double mass = 0.0;
   if (with_mass && t == 0) {
-    double v = 0.0;
-    for (uint32_t c = 0; c < RED_MCHUNKS; c++) v += mpart[c];
-    *ra.mass_out = v;
+    for (uint32_t c = 0; c < RED_MCHUNKS; c++) mass += mpart[c];
+    *ra.mass_out = mass;
   }
   __syncthreads();
-  // the totals: one thread per component, the steps in order
+  // the totals: RED_PARTS threads per component over the steps
+  if (t < 9 * RED_PARTS) {
+    const uint32_t k = t / RED_PARTS, p = t % RED_PARTS;
+    double v = 0.0;
+    if (p < nsteps) v = rec[k][p];
+    for (uint32_t s = p + RED_PARTS; s < nsteps; s += RED_PARTS) v += rec[k][s];
+    part[k][p] = v;
+  }
+  __syncthreads();
   if (t < 9) {
+    const uint32_t np = min(nsteps, RED_PARTS);
     double v = ra.totals[t];
-    for (uint32_t s = 0; s < nsteps; s++) v += ra.hist[((hist_base + s) % ra.hist_cap) * 16 + t];
-    ra.totals[t] = v;
+    for (uint32_t p = 0; p < np; p++) v += part[t][p];
+    ra.totals[t] = rb.out && rb.reset ? 0.0 : v;
+    if (rb.out) rb.out->sum[t] = v;
   } else if (t < 15) {
     const uint32_t g = (t - 9) / 2, comp = (t - 9) % 2;  // raw x / y of group g
+    const uint32_t* r = reinterpret_cast<const uint32_t*>(&rec[t - 9][64]);
     uint32_t v = (uint32_t)ra.raw_totals[3 * g + comp];
-    for (uint32_t s = 0; s < nsteps; s++)
-      v += (uint32_t)(int32_t)ra.hist[((hist_base + s) % ra.hist_cap) * 16 + 9 + 2 * g + comp];
-    ra.raw_totals[3 * g + comp] = (int32_t)v;
+    for (uint32_t s = 0; s < nsteps; s++) v += r[s];
+    ra.raw_totals[3 * g + comp] = rb.out && rb.reset ? 0 : (int32_t)v;
+    if (rb.out) rb.out->raw[3 * g + comp] = (int32_t)v;
+  } else if (t < 21 && rb.out) {  // the accumulator's words without a sum
+    const uint32_t w = t < 18 ? 3 * (t - 15) + 2 : t - 9;
+    rb.out->raw[w] = ra.raw_totals[w];
+    if (rb.reset) ra.raw_totals[w] = 0;
+  } else if (t == 21 && rb.out) {
+    rb.out->guarded = *ra.guard;
+    rb.out->steps = rb.steps;
+    if (rb.reset) *ra.guard = 0u;
   }
   if (t == 0) {
-    *ra.hist_pos = hist_base + nsteps;
+    if (rb.out) rb.out->mass = with_mass ? mass : *ra.mass_out;
+    *ra.hist_pos += nsteps;
     *ra.counter = 0u;
   }
 }
@@ -1274,10 +1329,10 @@ cudaError_t launch_batch_persist(uint32_t storage, dim3 block, uint32_t grid, ui
 }
 
 cudaError_t launch_force_reduce(const ReduceArgs* args, uint32_t count, uint32_t nsteps, bool with_mass,
-                                cudaStream_t s) {
+                                cudaStream_t s, wt_forces* out, uint64_t steps, int reset) {
   if ((nsteps == 0 && !with_mass) || count == 0) return cudaSuccess;
   return launch_chained(force_reduce_kernel, dim3(nsteps * RED_FCHUNKS + (with_mass ? RED_MCHUNKS : 0u), count),
-                        dim3(RED_THREADS), s, args, nsteps, with_mass ? 1u : 0u);
+                        dim3(RED_THREADS), s, args, nsteps, with_mass ? 1u : 0u, Readback{out, steps, reset});
 }
 
 // The force readout in one launch: the accumulators into a wt_forces record
