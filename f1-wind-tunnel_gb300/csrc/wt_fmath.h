@@ -94,6 +94,16 @@ WT_HD float cosf(float x) {
   return ((q + 1) & 2) ? -v : v;
 }
 
+// Both with one reduction; the bits of sinf and cosf.
+WT_HD void sincosf(float x, float* sn, float* cs) {
+  int q;
+  float r = reduce_pio2(x, &q);
+  float s = sin_poly(r), c = cos_poly(r);
+  float a = (q & 1) ? c : s, b = (q & 1) ? s : c;
+  *sn = (q & 2) ? -a : a;
+  *cs = ((q + 1) & 2) ? -b : b;
+}
+
 WT_HD float atan_poly(float t) {
   float z = t * t;
   float p = -0x1.642c86p-5f;          // -1/23

@@ -16,8 +16,42 @@
 namespace wt {
 namespace {
 
+// The F1's parts as tables of operands, formed from the shape on the host (f1_tables) by
+// the operations the reference writes at each part.  One copy of each primitive reads them
+// (sd_taper and on): the scene as straight-line code is some 2500 instructions whose
+// fetches were the bound (a 1280x720 frame issued in 15 % of its cycles and waited for an
+// instruction in 26 of every 30; half of the requests missed the first instruction cache).
+// With the parts left out that cannot matter (beyond): frame 3.15 -> 1.81 ms, voxelizing
+// 168x50x38 cells 75 -> 48 us.  A loop over the parts as a list of operations fetches
+// better still (96 % hits) and issues twice the instructions: 3.4 ms.
+// Quads of floats:
+//   taper    x0 dx mid half | r0 r1 - - | c0 c1 | s0 s1      capsule  a, r | b - a, |b - a|^2
+//   box      centre, r | half - r                           ellipsoid  centre | r | r * r
+//   wing     le.x le.y chord ang | thick z0 z1 rise | taper curl - -
+//   around   low corner, factor | high corner, addend
+enum : uint32_t { T_MID, T_NOSE, T_SCUTTLE, T_COVER, T_KEEL, T_POD, T_TAIL, T_COUNT };
+enum : uint32_t { C_HALO = 0, C_SUSF = 4, C_SUSR = 10, C_MIRROR = 15, C_EXHAUST, C_BORE, C_EDGE, C_POST, C_CARVE, C_COUNT = C_CARVE + 2 };
+enum : uint32_t {
+  B_BODY, B_FLOOR, B_FRONT, B_REAR, B_WHEEL,  // the groups' own boxes (two wheels)
+  B_PYLON = B_WHEEL + 2, B_AIRBOX, B_COCKPIT, B_MIRROR, B_FIN, B_LIGHT, B_CARVE, B_FENCE, B_STRAKE = B_FENCE + 2,
+  B_FOOT = B_STRAKE + 2, B_POST, B_DUCT, B_COUNT = B_DUCT + 2
+};
+enum : uint32_t { E_NOSE, E_AIR, E_HELMET, E_COUNT };
+enum : uint32_t {  // boxes around parts (beyond)
+  K_SCUTTLE, K_NOSE, K_COVER, K_KEEL, K_POD, K_AIRBOX, K_COCKPIT, K_CABIN, K_HELMET, K_HALO, K_MIRROR, K_SUSF, K_SUSR,
+  K_TAIL, K_FIN, K_LIGHT, K_FENCE, K_STRAKE, K_EDGE, K_COUNT
+};
+struct F1Tables {
+  float4 taper[T_COUNT][4], cap[C_COUNT][2], box[B_COUNT][2], ell[E_COUNT][3], wing[6][3],
+      around[K_COUNT][2];
+  float pod_k[3];      // the sidepod's carvings: capsules, then the box
+  uint32_t pod_caps, front_wings, pylon;
+  float ep[5];         // front endplate: centre x, y, half x, y, radius
+};
+
 // Shape plus host-computed shape-wide constants.
 struct Scene {
+  F1Tables f1;                // kind 0
   wt_shape s;
   CarView car;                // the W17 model (kind 5)
   float rake_c, rake_s;       // cos/sin of the rake angle (f1.ts:37-40)
@@ -47,15 +81,6 @@ __device__ float sd_rrect(V2 p, V2 b, float r) {
 __device__ float op_extrude(float d2, float dz) {
   return mn(mx(d2, dz), 0.0f) + len2(v2(mx(d2, 0.0f), mx(dz, 0.0f)));
 }
-__device__ float sd_taper(V3 p, float x0, float x1, V2 c0, V2 c1, V2 s0, V2 s1, float r0, float r1) {
-  const float t = clmp(dv(p.x - x0, x1 - x0), 0.0f, 1.0f);
-  const V2 c = mix2(c0, c1, t);
-  const V2 s = mix2(s0, s1, t);
-  const float r = mn(mixf(r0, r1, t), mn(s.x, s.y));
-  const float d2 = sd_rrect(v2(p.y, p.z) - c, s, r);
-  const float dx = ab(p.x - 0.5f * (x0 + x1)) - 0.5f * (x1 - x0);
-  return op_extrude(d2, dx) * 0.8f;
-}
 __device__ float sd_uneven_capsule(V2 p0, float r1, float r2, float hh) {
   const V2 p = v2(ab(p0.x), p0.y);
   const float b = dv(r1 - r2, hh);
@@ -75,7 +100,9 @@ __device__ float sd_wing_cs(V3 p, V2 le, float chord, float c, float s, float th
   return op_extrude(d2, ab(p.z - 0.5f * (z0 + z1)) - 0.5f * (z1 - z0));
 }
 __device__ float sd_wing(V3 p, V2 le, float chord, float ang, float thick, float z0, float z1) {
-  return sd_wing_cs(p, le, chord, wtm::cosf(ang), wtm::sinf(ang), thick, z0, z1);
+  float s, c;
+  wtm::sincosf(ang, &s, &c);
+  return sd_wing_cs(p, le, chord, c, s, thick, z0, z1);
 }
 __device__ __forceinline__ V2 op_u(V2 a, V2 b) { return (b.x < a.x) ? b : a; }
 
@@ -92,27 +119,47 @@ __device__ V3 body_frame(const Scene& S, V3 pw) {
   }
   return v3(x, p.y, dv(p.z, BODY_Z));
 }
-__device__ float smin(float a, float b, float k) {
+__device__ __noinline__ float smin(float a, float b, float k) {
   const float h = dv(mx(k - ab(a - b), 0.0f), k);
   return mn(a, b) - h * h * k * 0.25f;
 }
-__device__ float smax(float a, float b, float k) { return -smin(-a, -b, k); }
-__device__ float sd_ellipsoid(V3 p, V3 r) {
-  const float k0 = len3(v3(dv(p.x, r.x), dv(p.y, r.y), dv(p.z, r.z)));
-  const V3 rr = v3(r.x * r.x, r.y * r.y, r.z * r.z);
-  const float k1 = len3(v3(dv(p.x, rr.x), dv(p.y, rr.y), dv(p.z, rr.z)));
+__device__ __forceinline__ float smax(float a, float b, float k) { return -smin(-a, -b, k); }
+__device__ __noinline__ float sd_taper(const float4* q, V3 p) {
+  const float4 q0 = q[0], q1 = q[1], q2 = q[2], q3 = q[3];
+  const float t = clmp(dv(p.x - q0.x, q0.y), 0.0f, 1.0f);
+  const V2 c = mix2(v2(q2.x, q2.y), v2(q2.z, q2.w), t);
+  const V2 s = mix2(v2(q3.x, q3.y), v2(q3.z, q3.w), t);
+  const float r = mn(mixf(q1.x, q1.y, t), mn(s.x, s.y));
+  const float d2 = sd_rrect(v2(p.y, p.z) - c, s, r);
+  return op_extrude(d2, ab(p.x - q0.z) - q0.w) * 0.8f;
+}
+__device__ __noinline__ float sd_cap(const float4* q, V3 p) {
+  const float4 q0 = q[0], q1 = q[1];
+  const V3 pa = p - v3(q0.x, q0.y, q0.z), ba = v3(q1.x, q1.y, q1.z);
+  const float hh = clmp(dv(dot3(pa, ba), q1.w), 0.0f, 1.0f);
+  return len3(pa - ba * hh) - q0.w;
+}
+__device__ __noinline__ float sd_rb(const float4* q, V3 p) {
+  const float4 q0 = q[0], q1 = q[1];
+  return sd_box(p - v3(q0.x, q0.y, q0.z), v3(q1.x, q1.y, q1.z)) - q0.w;
+}
+__device__ __noinline__ float sd_ellipsoid(const float4* q, V3 pw) {
+  const float4 q0 = q[0], q1 = q[1], q2 = q[2];
+  const V3 p = pw - v3(q0.x, q0.y, q0.z);
+  const float k0 = len3(v3(dv(p.x, q1.x), dv(p.y, q1.y), dv(p.z, q1.z)));
+  const float k1 = len3(v3(dv(p.x, q2.x), dv(p.y, q2.y), dv(p.z, q2.z)));
   return dv(k0 * (k0 - 1.0f), mx(k1, 1e-5f));
 }
-__device__ float sd_cyl_z(V3 p, float r, float hz) {
+__device__ __noinline__ float sd_cyl_z(V3 p, float r, float hz) {
   const float dx = len2(v2(p.x, p.y)) - r, dz = ab(p.z) - hz;
   return mn(mx(dx, dz), 0.0f) + len2(v2(mx(dx, 0.0f), mx(dz, 0.0f)));
 }
-// Out of line (as is wheel_set): sixteen call sites would otherwise each carry a
-// copy, with its sin/cos, and the SDF's code would outgrow the instruction cache.
-__device__ __noinline__ float sd_wing_z(V3 p, V2 le, float chord, float ang, float thick, float z0, float z1, float rise,
-                           float taper, float curl) {
-  const float s = sstep(curl, z1, p.z);
-  return sd_wing(p, le + v2(0.0f, rise * s), chord * (1.0f - taper * s), ang + rise * s * 0.6f, thick, z0, z1) *
+__device__ __noinline__ float sd_wing_z(const float4* q, V3 p) {
+  const float4 q0 = q[0], q1 = q[1], q2 = q[2];
+  const float z1 = q1.z, rise = q1.w;
+  const float s = sstep(q2.y, z1, p.z);
+  return sd_wing(p, v2(q0.x, q0.y) + v2(0.0f, rise * s), q0.z * (1.0f - q2.x * s), q0.w + rise * s * 0.6f, q1.x, q1.y,
+                 z1) *
          0.85f;
 }
 __device__ float tunnel_roof(float x, float b) {
@@ -120,196 +167,159 @@ __device__ float tunnel_roof(float x, float b) {
   if (x < 3.8f) return b + 0.05f;
   return mixf(b + 0.05f, b + 0.25f, sstep(3.8f, 4.98f, x));
 }
-__device__ float sd_floor(V3 p, float b) {
-  const float roof = tunnel_roof(p.x, b);
+__device__ float sd_slab(V3 p, float b, float roof) {
   const float zlim = mixf(0.80f, 0.58f, sstep(3.6f, 4.15f, p.x));
   const float top = (ab(p.z - 0.40f) < 0.28f) ? roof + 0.03f : b + 0.05f;
   const float slab = mx(mx(b - p.y, p.y - top), mx(ab(p.x - 3.265f) - 1.715f, p.z - zlim));
   const float tunnel = mx(p.y - roof, ab(p.z - 0.40f) - 0.255f);
-  float d = mx(slab, -tunnel) * 0.8f;
-#pragma unroll
-  for (int i = 0; i < 2; i++) {
-    const float fz = 0.26f + (float)i * 0.16f;
-    const float fence = sd_box(p - v3(1.84f, b + 0.08f, fz), v3(0.28f, 0.08f, 0.012f));
-    d = mn(d, mx(fence, p.y - roof - 0.02f));
-  }
-#pragma unroll
-  for (int i = 0; i < 2; i++) {
-    const float sz = 0.30f + (float)i * 0.20f;
-    const float strake = sd_box(p - v3(4.62f, b + 0.17f, sz), v3(0.34f, 0.17f, 0.008f));
-    d = mn(d, mx(strake, p.y - roof));
-  }
-  d = mn(d, sd_capsule(p, v3(2.25f, b + 0.065f, 0.79f), v3(3.85f, b + 0.05f, 0.78f), 0.02f));
-  return d;
+  return mx(slab, -tunnel) * 0.8f;
 }
 __device__ float sd_tyre(V3 p, V3 c, float hw) {
   const V3 q = p - c;
   return sd_rrect(v2(len2(v2(q.x, q.y)) - 0.2925f, q.z), v2(0.0625f, hw), 0.06f);
 }
-__device__ float sd_wheel_cover(V3 p, V3 c, float hw) {
-  const V3 q = p - c;
-  float d = sd_cyl_z(q, 0.234f, hw - 0.028f);
-  d = mn(d, sd_cyl_z(q - v3(0.0f, 0.0f, hw - 0.02f), 0.045f, 0.02f));
+// A part cannot change a point's result when its distance as computed is at least what it
+// joins: mn(d, part) is exactly d when part >= d, smin(d, part, k) exactly d when
+// part >= d + k.  The distance as computed is bounded below by a factor (1 for boxes,
+// capsules and cylinders, 0.8 for tapers, min/max radius for ellipsoids) times the
+// distance to a box around the part; beyond() tests that against r.  Its margin covers
+// the roundings (relative 1e-3, and 0.1 mm of a model in metres); points and parts that
+// are not finite are never beyond.
+// r = factor * (d + addend) is the distance to the box that leaves d as it is.
+__device__ __noinline__ bool beyond(const float4* q, V3 p, float d) {
+  const float4 lo = q[0], hi = q[1];
+  const float x = fmaxf(fmaxf(lo.x - p.x, p.x - hi.x), 0.0f), y = fmaxf(fmaxf(lo.y - p.y, p.y - hi.y), 0.0f),
+              z = fmaxf(fmaxf(lo.z - p.z, p.z - hi.z), 0.0f);
+  const float r = lo.w * (d + hi.w), m = (fmaxf(r, 0.0f) + 1e-4f) * 1.001f, d2 = fmaf(x, x, fmaf(y, y, z * z));
+  return d2 > m * m && d2 < 1e12f && r < 1e6f;
+}
+// The same with the test along x, where most parts fail, in line.
+__device__ __forceinline__ bool beyond_x(const float4* q, V3 p, float lo, float hi, float factor, float addend, float d) {
+  const float gap = fmaxf(lo - p.x, p.x - hi), r = fmaxf(factor * (d + addend), 0.0f);
+  return (gap > r * 1.001f + 2e-4f && gap < 1e6f) || beyond(q, p, d);
+}
+// The body's own distance.  The chain is smin(smin(nose, scuttle), cockpit) and on: the
+// cockpit's part comes first, and what stands before it only where it can reach it (a
+// smin lowers the smaller value by at most k / 4; the nose's ellipsoid has radii 1 : 2).
+__device__ float sd_bodywork(const F1Tables& F, V3 p) {
+  const float mid = sd_taper(F.taper[T_MID], p);
+  float d = mid;
+  if (!beyond_x(F.around[K_SCUTTLE], p, 1.20f, 2.24f, 1.25f, 0.08f, mid) ||
+      !beyond_x(F.around[K_NOSE], p, -0.06f, 1.26f, 2.0f, 0.09f, mid)) {
+    d = sd_taper(F.taper[T_NOSE], p);
+    d = smin(d, sd_ellipsoid(F.ell[E_NOSE], p), 0.04f);
+    if (F.pylon) d = mn(d, sd_rb(F.box[B_PYLON], p));
+    d = smin(d, sd_taper(F.taper[T_SCUTTLE], p), 0.08f);
+    d = smin(d, mid, 0.06f);
+  }
+#pragma unroll 1
+  for (uint32_t i = 0; i < 3; i++) {  // engine cover, keel, sidepods; each joins with its box's addend
+    if (beyond(F.around[K_COVER + i], p, d)) continue;
+    float v = sd_taper(F.taper[T_COVER + i], p);
+    if (i == 2) {
+#pragma unroll 1
+      for (uint32_t j = 0; j <= F.pod_caps; j++) {
+        const float c = j < F.pod_caps ? sd_cap(F.cap[C_CARVE + j], p) : sd_rb(F.box[B_CARVE], p);
+        v = smax(v, -c, F.pod_k[j < F.pod_caps ? j : 2]);
+      }
+    }
+    d = smin(d, v, F.around[K_COVER + i][1].w);
+  }
+  if (!beyond(F.around[K_AIRBOX], p, d))
+    d = smin(d, smax(sd_rb(F.box[B_AIRBOX], p), -sd_ellipsoid(F.ell[E_AIR], p), 0.015f), 0.10f);
+  // smax(d, -x, k) is exactly d when x >= k - d
+  if (!beyond(F.around[K_COCKPIT], p, d))
+    d = smax(d, -sd_rb(F.box[B_COCKPIT], p), 0.03f);
   return d;
 }
-__device__ __noinline__ V2 wheel_set(V3 p, V2 res, V3 c, float hw, float inboard) {
-  if (sd_box(p - c, v3(WR26 + 0.02f, WR26 + 0.02f, hw + 0.2f)) > res.x) return res;
-  res = op_u(res, v2(sd_tyre(p, c, hw), 2.0f));
-  res = op_u(res, v2(sd_wheel_cover(p, c, hw), 9.0f));
-  const float duct = sd_cyl_z(p - v3(c.x, c.y, c.z - hw - inboard * 0.5f), 0.17f, inboard * 0.5f);
-  const float duct_wing = sd_rbox(p - v3(c.x - 0.04f, c.y + 0.21f, c.z - hw - 0.05f), v3(0.16f, 0.012f, 0.05f), 0.006f);
-  return op_u(res, v2(mn(duct, duct_wing), 10.0f));
-}
-__device__ float sd_suspension(V3 p, float b) {
-  const float fz = FWZ - FHW - 0.05f, rz = RWZ - RHW - 0.05f;
-  float d = sd_capsule(p, v3(1.10f, b + 0.43f, 0.17f), v3(FA + 0.02f, WR + 0.16f, fz), 0.017f);
-  d = mn(d, sd_capsule(p, v3(1.42f, b + 0.40f, 0.17f), v3(FA + 0.02f, WR + 0.16f, fz), 0.017f));
-  d = mn(d, sd_capsule(p, v3(0.98f, b + 0.19f, 0.15f), v3(FA, WR - 0.13f, fz), 0.017f));
-  d = mn(d, sd_capsule(p, v3(1.38f, b + 0.17f, 0.15f), v3(FA, WR - 0.13f, fz), 0.017f));
-  d = mn(d, sd_capsule(p, v3(FA + 0.03f, WR - 0.10f, FWZ - FHW - 0.07f), v3(1.20f, b + 0.47f, 0.16f), 0.014f));
-  d = mn(d, sd_capsule(p, v3(0.86f, b + 0.29f, 0.16f), v3(0.88f, WR + 0.02f, fz), 0.013f));
-  d = mn(d, sd_capsule(p, v3(4.30f, b + 0.42f, 0.20f), v3(RA, WR + 0.17f, rz), 0.017f));
-  d = mn(d, sd_capsule(p, v3(4.78f, b + 0.40f, 0.16f), v3(RA, WR + 0.17f, rz), 0.017f));
-  d = mn(d, sd_capsule(p, v3(4.28f, b + 0.16f, 0.24f), v3(RA, WR - 0.14f, rz), 0.017f));
-  d = mn(d, sd_capsule(p, v3(4.82f, b + 0.15f, 0.18f), v3(RA, WR - 0.14f, rz), 0.017f));
-  d = mn(d, sd_capsule(p, v3(RA - 0.03f, WR + 0.14f, RWZ - RHW - 0.07f), v3(4.40f, b + 0.18f, 0.22f), 0.014f));
+__device__ __noinline__ float cap_min(const float4 (*q)[2], uint32_t n, V3 p, float d) {
+#pragma unroll 1
+  for (uint32_t i = 0; i < n; i++) d = mn(d, sd_cap(q[i], p));
   return d;
 }
-__device__ float sd_nose(const Scene& S, V3 p, float b) {
-  const uint32_t v = variant(S.s.nose);
-  const float x0 = (v == 1u) ? 0.34f : 0.10f;
-  const float y0 = b + ((v == 2u) ? 0.25f : 0.17f);
-  V2 s0 = v2(0.055f, 0.11f);
-  if (v == 1u) s0 = v2(0.075f, 0.15f);
-  if (v == 2u) s0 = v2(0.045f, 0.075f);
-  float d = sd_taper(p, x0, 1.26f, v2(y0, 0.0f), v2(b + 0.36f, 0.0f), s0, v2(0.15f, 0.17f), 0.04f, 0.12f);
-  d = smin(d, sd_ellipsoid(p - v3(x0 + 0.02f, y0, 0.0f), v3(0.09f, s0.x, s0.y)), 0.04f);
-  if (v != 0u) {
-    const float yw = 0.19f + b * 0.45f;
-    const float pylon = sd_rbox(p - v3(x0 + 0.06f, 0.5f * (yw + y0), 0.09f), v3(0.09f, 0.5f * (y0 - yw) + 0.02f, 0.006f), 0.004f);
-    d = mn(d, pylon);
-  }
+// near: the point's distance so far; what is not below it need not be exact.
+__device__ float sd_carbon(const F1Tables& F, V3 p, float near) {
+  float d = 1e30f;
+  if (!beyond_x(F.around[K_SUSF], p, 0.84f, 1.44f, 1.0f, 0.0f, near))
+    d = cap_min(F.cap + C_SUSF, 6u, p, d);
+  if (!beyond_x(F.around[K_SUSR], p, 4.26f, 4.84f, 1.0f, 0.0f, fminf(d, near)))
+    d = cap_min(F.cap + C_SUSR, 5u, p, d);
+  if (!beyond_x(F.around[K_TAIL], p, 4.78f, 5.42f, 1.25f, 0.0f, fminf(d, near)))
+    d = mn(d, sd_taper(F.taper[T_TAIL], p));
+  if (!beyond_x(F.around[K_FIN], p, 3.40f, 4.50f, 1.0f, 0.0f, fminf(d, near)))
+    d = mn(d, sd_rb(F.box[B_FIN], p));
   return d;
 }
-__device__ float sd_engine_cover(const Scene& S, V3 p, float b) {
-  const uint32_t v = variant(S.s.cover);
-  if (v == 1u) return sd_taper(p, 2.96f, 4.86f, v2(b + 0.60f, 0.0f), v2(b + 0.40f, 0.0f), v2(0.32f, 0.31f), v2(0.12f, 0.13f), 0.15f, 0.08f);
-  if (v == 2u) return sd_taper(p, 2.96f, 4.70f, v2(b + 0.57f, 0.0f), v2(b + 0.34f, 0.0f), v2(0.29f, 0.19f), v2(0.06f, 0.05f), 0.12f, 0.04f);
-  return sd_taper(p, 2.96f, 4.86f, v2(b + 0.58f, 0.0f), v2(b + 0.36f, 0.0f), v2(0.30f, 0.24f), v2(0.08f, 0.07f), 0.14f, 0.06f);
-}
-__device__ float sd_sidepods(const Scene& S, V3 p, float b) {
-  const uint32_t v = variant(S.s.sidepod);
-  float pod;
-  if (v == 1u) {
-    pod = sd_taper(p, 2.30f, 4.05f, v2(b + 0.40f, 0.36f), v2(b + 0.24f, 0.24f), v2(0.16f, 0.08f), v2(0.07f, 0.05f), 0.06f, 0.04f);
-    return smax(pod, -sd_rbox(p - v3(2.27f, b + 0.42f, 0.38f), v3(0.06f, 0.12f, 0.05f), 0.03f), 0.02f);
-  }
-  if (v == 2u) {
-    pod = sd_taper(p, 2.30f, 4.25f, v2(b + 0.41f, 0.52f), v2(b + 0.24f, 0.30f), v2(0.18f, 0.28f), v2(0.08f, 0.11f), 0.10f, 0.05f);
-    pod = smax(pod, -sd_capsule(p, v3(2.30f, b + 0.13f, 0.84f), v3(3.70f, b + 0.08f, 0.58f), 0.15f), 0.05f);
-    pod = smax(pod, -sd_capsule(p, v3(2.55f, b + 0.66f, 0.52f), v3(4.00f, b + 0.40f, 0.36f), 0.11f), 0.04f);
-    return smax(pod, -sd_rbox(p - v3(2.28f, b + 0.47f, 0.57f), v3(0.06f, 0.10f, 0.17f), 0.05f), 0.02f);
-  }
-  if (v == 3u) {
-    pod = sd_taper(p, 2.30f, 4.25f, v2(b + 0.47f, 0.52f), v2(b + 0.26f, 0.28f), v2(0.15f, 0.25f), v2(0.07f, 0.10f), 0.12f, 0.05f);
-    pod = smax(pod, -sd_capsule(p, v3(2.25f, b + 0.17f, 0.86f), v3(3.70f, b + 0.10f, 0.56f), 0.22f), 0.05f);
-    return smax(pod, -sd_rbox(p - v3(2.28f, b + 0.52f, 0.55f), v3(0.06f, 0.07f, 0.17f), 0.04f), 0.02f);
-  }
-  pod = sd_taper(p, 2.30f, 4.25f, v2(b + 0.41f, 0.52f), v2(b + 0.22f, 0.28f), v2(0.18f, 0.25f), v2(0.07f, 0.10f), 0.12f, 0.05f);
-  pod = smax(pod, -sd_capsule(p, v3(2.30f, b + 0.13f, 0.82f), v3(3.70f, b + 0.08f, 0.56f), 0.16f), 0.05f);
-  return smax(pod, -sd_rbox(p - v3(2.28f, b + 0.47f, 0.57f), v3(0.06f, 0.10f, 0.17f), 0.05f), 0.02f);
-}
-__device__ float sd_bodywork(const Scene& S, V3 p, float b) {
-  float d = sd_nose(S, p, b);
-  d = smin(d, sd_taper(p, 1.20f, 2.24f, v2(b + 0.36f, 0.0f), v2(b + 0.42f, 0.0f), v2(0.15f, 0.17f), v2(0.25f, 0.29f), 0.12f, 0.16f), 0.08f);
-  d = smin(d, sd_taper(p, 2.20f, 3.06f, v2(b + 0.42f, 0.0f), v2(b + 0.42f, 0.0f), v2(0.25f, 0.30f), v2(0.25f, 0.34f), 0.16f, 0.16f), 0.06f);
-  d = smin(d, sd_engine_cover(S, p, b), 0.10f);
-  const float keel = sd_taper(p, 1.30f, 4.70f, v2(b + 0.22f, 0.0f), v2(b + 0.20f, 0.0f), v2(0.19f, 0.19f), v2(0.17f, 0.14f), 0.06f, 0.05f);
-  d = smin(d, keel, 0.08f);
-  d = smin(d, sd_sidepods(S, p, b), 0.12f);
-  float airbox = sd_rbox(p - v3(3.02f, b + 0.84f, 0.0f), v3(0.17f, 0.11f, 0.12f), 0.08f);
-  airbox = smax(airbox, -sd_ellipsoid(p - v3(2.85f, b + 0.86f, 0.0f), v3(0.09f, 0.066f, 0.078f)), 0.015f);
-  d = smin(d, airbox, 0.10f);
-  return smax(d, -sd_rbox(p - v3(2.62f, b + 0.72f, 0.0f), v3(0.42f, 0.13f, 0.215f), 0.10f), 0.03f);
-}
-__device__ float sd_halo(V3 p, float b) {
-  float d = sd_capsule(p, v3(2.17f, b + 0.62f, 0.0f), v3(2.36f, b + 0.90f, 0.0f), 0.034f);
-  d = smin(d, sd_capsule(p, v3(2.36f, b + 0.90f, 0.0f), v3(2.52f, b + 0.92f, 0.20f), 0.031f), 0.03f);
-  d = smin(d, sd_capsule(p, v3(2.52f, b + 0.92f, 0.20f), v3(2.82f, b + 0.88f, 0.26f), 0.031f), 0.03f);
-  return smin(d, sd_capsule(p, v3(2.82f, b + 0.88f, 0.26f), v3(3.02f, b + 0.74f, 0.25f), 0.033f), 0.03f);
-}
-__device__ float sd_front_wing(const Scene& S, V3 p, float yw) {
-  const float ff = S.s.front_flap;
-  const uint32_t v = variant(S.s.front_wing);
-  float d, ep;
-  if (v == 1u) {
-    d = sd_wing_z(p, v2(-0.03f, yw), 0.31f, 2.0f * DEG + ff * 0.1f, 0.034f, 0.0f, 0.94f, 0.03f, 0.2f, 0.5f);
-    d = mn(d, sd_wing_z(p, v2(0.21f, yw + 0.036f), 0.17f, 9.0f * DEG + ff * 0.45f, 0.024f, 0.0f, 0.94f, 0.15f, 0.35f, 0.3f));
-    d = mn(d, sd_wing_z(p, v2(0.335f, yw + 0.075f + ff * 0.03f), 0.14f, 17.0f * DEG + ff * 0.75f, 0.020f, 0.10f, 0.94f, 0.19f, 0.35f, 0.25f));
-    d = mn(d, sd_wing_z(p, v2(0.425f, yw + 0.118f + ff * 0.07f), 0.12f, 26.0f * DEG + ff, 0.018f, 0.12f, 0.94f, 0.22f, 0.4f, 0.25f));
-    ep = sd_rrect(v2(p.x - 0.25f, p.y - (yw + 0.17f)), v2(0.29f, 0.20f), 0.08f);
-  } else if (v == 2u) {
-    d = sd_wing_z(p, v2(-0.03f, yw), 0.31f, 3.0f * DEG + ff * 0.1f, 0.034f, 0.0f, 0.94f, -0.02f, 0.15f, 0.55f);
-    d = mn(d, sd_wing_z(p, v2(0.21f, yw + 0.04f), 0.19f, 13.0f * DEG + ff * 0.45f, 0.024f, 0.0f, 0.94f, -0.04f, 0.35f, 0.35f));
-    d = mn(d, sd_wing_z(p, v2(0.35f, yw + 0.085f + ff * 0.03f), 0.16f, 22.0f * DEG + ff * 0.75f, 0.020f, 0.06f, 0.94f, -0.06f, 0.4f, 0.35f));
-    d = mn(d, sd_wing_z(p, v2(0.45f, yw + 0.13f + ff * 0.07f), 0.13f, 31.0f * DEG + ff, 0.018f, 0.08f, 0.94f, -0.08f, 0.45f, 0.35f));
-    ep = sd_rrect(v2(p.x - 0.25f, p.y - (yw + 0.06f)), v2(0.29f, 0.10f), 0.06f);
-  } else if (v == 3u) {
-    d = sd_wing_z(p, v2(-0.03f, yw), 0.30f, 1.0f * DEG + ff * 0.05f, 0.030f, 0.0f, 0.94f, 0.0f, 0.1f, 0.6f);
-    d = mn(d, sd_wing_z(p, v2(0.20f, yw + 0.03f), 0.16f, 4.0f * DEG + ff * 0.3f, 0.022f, 0.0f, 0.94f, 0.02f, 0.2f, 0.5f));
-    ep = sd_rrect(v2(p.x - 0.22f, p.y - (yw + 0.05f)), v2(0.26f, 0.085f), 0.05f);
-  } else {
-    d = sd_wing_z(p, v2(-0.03f, yw), 0.31f, 2.0f * DEG + ff * 0.1f, 0.034f, 0.0f, 0.94f, 0.06f, 0.2f, 0.5f);
-    d = mn(d, sd_wing_z(p, v2(0.21f, yw + 0.036f), 0.17f, 9.0f * DEG + ff * 0.45f, 0.024f, 0.0f, 0.94f, 0.09f, 0.25f, 0.45f));
-    d = mn(d, sd_wing_z(p, v2(0.335f, yw + 0.075f + ff * 0.03f), 0.14f, 17.0f * DEG + ff * 0.75f, 0.020f, 0.10f, 0.94f, 0.11f, 0.25f, 0.4f));
-    d = mn(d, sd_wing_z(p, v2(0.425f, yw + 0.118f + ff * 0.07f), 0.12f, 26.0f * DEG + ff, 0.018f, 0.12f, 0.94f, 0.13f, 0.25f, 0.4f));
-    ep = sd_rrect(v2(p.x - 0.25f, p.y - (yw + 0.085f)), v2(0.29f, 0.115f), 0.07f);
-  }
-  const float span = 0.94f;
-  d = mn(d, mx(ep, ab(p.z - (span + 0.012f)) - 0.010f));
-  return mn(d, sd_rbox(p - v3(0.22f, yw - 0.008f, span - 0.04f), v3(0.30f, 0.006f, 0.06f), 0.004f));
-}
-__device__ float sd_rear_wing(const Scene& S, V3 p, float b, float yr) {
-  float d = sd_wing_z(p, v2(4.98f, yr), S.chord_m, S.ang_m, 0.05f, 0.0f, 0.50f, S.rise_m, 0.12f, 0.22f);
-  const V2 te = (v2(4.98f, yr) + v2(S.rear_c, S.rear_s) * (S.chord_m - 0.01f)) + v2(-0.03f, 0.035f);
-  d = mn(d, sd_wing_z(p, te, S.chord_f, S.ang_f, 0.03f, 0.0f, 0.49f, S.rise_m * 0.8f, 0.10f, 0.28f));
-  d = mn(d, sd_capsule(p, v3(5.26f, yr + 0.05f, 0.0f), v3(5.30f, yr + 0.12f, 0.0f), 0.024f));
-  const float ep = sd_rrect(v2(p.x - 5.25f, p.y - (yr - 0.03f)), v2(S.ep_hx, S.ep_hy), 0.13f);
-  d = mn(d, mx(ep, ab(p.z - 0.513f) - 0.012f));
-  return mn(d, sd_rbox(p - v3(5.09f, 0.5f * (b + 0.36f + yr + 0.06f), 0.06f), v3(0.07f, 0.5f * (yr + 0.06f - b - 0.36f), 0.008f), 0.006f));
+__device__ float sd_floor(const F1Tables& F, V3 p, float b, float near) {
+  const float roof = tunnel_roof(p.x, b);
+  float d = sd_slab(p, b, roof);
+  if (!beyond(F.around[K_FENCE], p, fminf(d, near)))
+#pragma unroll 1
+    for (uint32_t i = 0; i < 2; i++) d = mn(d, mx(sd_rb(F.box[B_FENCE + i], p), p.y - roof - 0.02f));
+  if (!beyond(F.around[K_STRAKE], p, fminf(d, near)))
+#pragma unroll 1
+    for (uint32_t i = 0; i < 2; i++) d = mn(d, mx(sd_rb(F.box[B_STRAKE + i], p), p.y - roof));
+  if (!beyond(F.around[K_EDGE], p, fminf(d, near)))
+    d = mn(d, sd_cap(F.cap[C_EDGE], p));
+  return d;
 }
 __device__ V2 sd_f1(const Scene& S, V3 pw) {
+  const F1Tables& F = S.f1;
   const V3 pworld = v3(pw.x, pw.y, ab(pw.z));
   const V3 p = body_frame(S, pworld);
   const float b = S.s.ride_h;
-  const float yw = 0.19f + b * 0.45f;
-  const float yr = b + 0.80f;
   V2 res = v2(1e3f, 0.0f);
-  if (sd_box(p - v3(2.72f, b + 0.52f, 0.0f), v3(2.74f, 0.62f, 0.95f)) < res.x) {
-    res = op_u(res, v2(sd_bodywork(S, p, b), 0.0f));
-    res = op_u(res, v2(sd_ellipsoid(p - v3(2.67f, b + 0.71f, 0.0f), v3(0.15f, 0.13f, 0.12f)), 3.0f));
-    res = op_u(res, v2(sd_halo(p, b), 4.0f));
-    float mirror = sd_rbox(p - v3(2.32f, b + 0.67f, 0.60f), v3(0.035f, 0.035f, 0.085f), 0.02f);
-    mirror = mn(mirror, sd_capsule(p, v3(2.36f, b + 0.66f, 0.53f), v3(2.45f, b + 0.50f, 0.46f), 0.011f));
-    res = op_u(res, v2(mirror, 0.0f));
-    float carbon = sd_suspension(p, b);
-    carbon = mn(carbon, sd_taper(p, 4.78f, 5.40f, v2(b + 0.33f, 0.0f), v2(b + 0.33f, 0.0f), v2(0.07f, 0.065f), v2(0.045f, 0.045f), 0.04f, 0.03f));
-    carbon = mn(carbon, sd_rbox(p - v3(3.95f, b + 0.74f, 0.0f), v3(0.55f, 0.10f, 0.008f), 0.006f));
-    res = op_u(res, v2(carbon, 1.0f));
-    res = op_u(res, v2(sd_rbox(p - v3(5.405f, b + 0.33f, 0.0f), v3(0.012f, 0.028f, 0.05f), 0.006f), 11.0f));
-    float exhaust = sd_capsule(p, v3(4.95f, b + 0.44f, 0.0f), v3(5.13f, b + 0.45f, 0.0f), 0.042f);
-    exhaust = mx(exhaust, -sd_capsule(p, v3(5.0f, b + 0.44f, 0.0f), v3(5.2f, b + 0.45f, 0.0f), 0.028f));
-    res = op_u(res, v2(exhaust, 10.0f));
+  if (sd_rb(F.box[B_BODY], p) < res.x) {
+    res = op_u(res, v2(sd_bodywork(F, p), 0.0f));
+    // cockpit: helmet, halo (its smins lower it by at most 0.0225), mirror
+    if (!beyond_x(F.around[K_CABIN], p, 2.13f, 3.06f, 1.25f, 0.018f, res.x)) {
+      if (!beyond(F.around[K_HELMET], p, res.x))
+        res = op_u(res, v2(sd_ellipsoid(F.ell[E_HELMET], p), 3.0f));
+      if (!beyond(F.around[K_HALO], p, res.x)) {
+        float d = sd_cap(F.cap[C_HALO], p);
+#pragma unroll 1
+        for (uint32_t i = 1; i < 4; i++) d = smin(d, sd_cap(F.cap[C_HALO + i], p), 0.03f);
+        res = op_u(res, v2(d, 4.0f));
+      }
+      if (!beyond(F.around[K_MIRROR], p, res.x))
+        res = op_u(res, v2(mn(sd_rb(F.box[B_MIRROR], p), sd_cap(F.cap[C_MIRROR], p)), 0.0f));
+    }
+    res = op_u(res, v2(sd_carbon(F, p, res.x), 1.0f));
+    if (!beyond_x(F.around[K_LIGHT], p, 4.90f, 5.42f, 1.0f, 0.0f, res.x)) {
+      res = op_u(res, v2(sd_rb(F.box[B_LIGHT], p), 11.0f));
+      res = op_u(res, v2(mx(sd_cap(F.cap[C_EXHAUST], p), -sd_cap(F.cap[C_BORE], p)), 10.0f));
+    }
   }
-  if (sd_box(p - v3(3.26f, b + 0.2f, 0.4f), v3(1.75f, 0.22f, 0.42f)) < res.x) res = op_u(res, v2(sd_floor(p, b), 1.0f));
+  if (sd_rb(F.box[B_FLOOR], p) < res.x) res = op_u(res, v2(sd_floor(F, p, b, res.x), 1.0f));
   const float lip = BODY_LIP * BODY_X;
   res.x = res.x * lip;
-  if (sd_box(p - v3(0.24f, yw + 0.17f, 0.48f), v3(0.36f, 0.34f, 0.50f)) < dv(res.x, lip))
-    res = op_u(res, v2(sd_front_wing(S, p, yw) * BODY_LIP * BODY_X, 7.0f));  // (d * LIP) * X, as written
-  if (sd_box(p - v3(5.20f, b + 0.64f, 0.27f), v3(0.46f, 0.56f, 0.29f)) < dv(res.x, lip))
-    res = op_u(res, v2(sd_rear_wing(S, p, b, yr) * BODY_LIP * BODY_X, 8.0f));
-  res = wheel_set(pworld, res, v3(FA, WR26, FWZ * BODY_Z), FHW26, 0.10f);
-  res = wheel_set(pworld, res, v3(RA26, WR26, RWZ * BODY_Z), RHW26, 0.08f);
+#pragma unroll 1
+  for (uint32_t w = 0; w < 2; w++) {  // front, rear wing
+    if (!(sd_rb(F.box[B_FRONT + w], p) < dv(res.x, lip))) continue;
+    const uint32_t i0 = w ? 4u : 0u, i1 = w ? 6u : F.front_wings;
+    float d = sd_wing_z(F.wing[i0], p);
+#pragma unroll 1
+    for (uint32_t i = i0 + 1; i < i1; i++) d = mn(d, sd_wing_z(F.wing[i], p));
+    const float4 e = w ? make_float4(5.25f, (b + 0.80f) - 0.03f, S.ep_hx, S.ep_hy) : make_float4(F.ep[0], F.ep[1], F.ep[2], F.ep[3]);
+    const float ep = sd_rrect(v2(p.x - e.x, p.y - e.y), v2(e.z, e.w), w ? 0.13f : F.ep[4]);
+    if (w) d = mn(d, sd_cap(F.cap[C_POST], p));
+    d = mn(d, mx(ep, w ? ab(p.z - 0.513f) - 0.012f : ab(p.z - (0.94f + 0.012f)) - 0.010f));
+    d = mn(d, sd_rb(F.box[B_FOOT + w], p));
+    res = op_u(res, v2(d * BODY_LIP * BODY_X, w ? 8.0f : 7.0f));  // (d * LIP) * X, as written
+  }
+#pragma unroll 1
+  for (uint32_t w = 0; w < 2; w++) {  // wheels, in the world's frame
+    if (sd_rb(F.box[B_WHEEL + w], pworld) > res.x) continue;
+    const float4 c4 = F.box[B_WHEEL + w][0];
+    const V3 c = v3(c4.x, c4.y, c4.z);
+    const float hw = w ? RHW26 : FHW26, inboard = w ? 0.08f : 0.10f;
+    res = op_u(res, v2(sd_tyre(pworld, c, hw), 2.0f));
+    const V3 q = pworld - c;
+    const float cover = mn(sd_cyl_z(q, 0.234f, hw - 0.028f), sd_cyl_z(q - v3(0.0f, 0.0f, hw - 0.02f), 0.045f, 0.02f));
+    res = op_u(res, v2(cover, 9.0f));
+    const float duct = sd_cyl_z(pworld - v3(c.x, c.y, c.z - hw - inboard * 0.5f), 0.17f, inboard * 0.5f);
+    res = op_u(res, v2(mn(duct, sd_rb(F.box[B_DUCT + w], pworld)), 10.0f));
+  }
   return res;
 }
 __device__ float f1_emission(const Scene& S, V3 pw) {
@@ -500,6 +510,181 @@ __device__ V2 scene_sdf(const Scene& S, V3 p) {
   }
 }
 
+uint32_t host_variant(float v) {  // u32(v + 0.5), saturating
+  const float t = v + 0.5f;
+  return (t == t && t > 0.0f) ? (t >= 4294967296.0f ? 4294967295u : (uint32_t)t) : 0u;
+}
+// The parts of f1.ts:42-320.
+void f1_tables(Scene& S) {
+  F1Tables& F = S.f1;
+  const float b = S.s.ride_h, yw = 0.19f + b * 0.45f, yr = b + 0.80f, ff = S.s.front_flap;
+  auto f4 = [](float x, float y, float z, float w) { return make_float4(x, y, z, w); };
+  auto at = [&](float x, float y, float z) { return v3(x, b + y, z); };
+  auto taper = [&](uint32_t i, float x0, float x1, V2 c0, V2 c1, V2 s0, V2 s1, float r0, float r1) {
+    float4* q = F.taper[i];
+    q[0] = f4(x0, x1 - x0, 0.5f * (x0 + x1), 0.5f * (x1 - x0));
+    q[1] = f4(r0, r1, 0.0f, 0.0f);
+    q[2] = f4(c0.x, c0.y, c1.x, c1.y);
+    q[3] = f4(s0.x, s0.y, s1.x, s1.y);
+  };
+  auto cap = [&](uint32_t i, V3 a, V3 e, float r) {
+    const float x = e.x - a.x, y = e.y - a.y, z = e.z - a.z;
+    F.cap[i][0] = f4(a.x, a.y, a.z, r);
+    F.cap[i][1] = f4(x, y, z, x * x + y * y + z * z);
+  };
+  auto box = [&](uint32_t i, V3 c, V3 h, float r) {
+    F.box[i][0] = f4(c.x, c.y, c.z, r);
+    F.box[i][1] = f4(h.x - r, h.y - r, h.z - r, 0.0f);
+  };
+  auto ell = [&](uint32_t i, V3 c, V3 r) {
+    F.ell[i][0] = f4(c.x, c.y, c.z, 0.0f);
+    F.ell[i][1] = f4(r.x, r.y, r.z, 0.0f);
+    F.ell[i][2] = f4(r.x * r.x, r.y * r.y, r.z * r.z, 0.0f);
+  };
+  auto wing = [&](uint32_t i, float lx, float ly, float chord, float ang, float thick, float z0, float z1, float rise,
+                  float tap, float curl) {
+    F.wing[i][0] = f4(lx, ly, chord, ang);
+    F.wing[i][1] = f4(thick, z0, z1, rise);
+    F.wing[i][2] = f4(tap, curl, 0.0f, 0.0f);
+  };
+  auto y0z = [&](float y) { return v2(b + y, 0.0f); };
+  auto around = [&](uint32_t i, V3 lo, V3 hi, float factor, float addend) {
+    F.around[i][0] = f4(lo.x, lo.y, lo.z, factor);
+    F.around[i][1] = f4(hi.x, hi.y, hi.z, addend);
+  };
+  around(K_SCUTTLE, at(1.20f, 0.17f, -0.29f), at(2.24f, 0.67f, 0.29f), 1.25f, 0.08f);
+  around(K_NOSE, v3(-0.06f, fminf(b, yw - 0.02f), -0.17f), v3(1.26f, fmaxf(b + 0.51f, yw + 0.02f), 0.17f), 2.0f, 0.09f);
+  around(K_COVER, at(2.96f, 0.28f, -0.31f), at(4.86f, 0.92f, 0.31f), 1.25f, 0.10f);
+  around(K_KEEL, at(1.30f, 0.03f, -0.19f), at(4.70f, 0.41f, 0.19f), 1.25f, 0.08f);
+  around(K_POD, at(2.30f, 0.15f, 0.18f), at(4.25f, 0.62f, 0.80f), 1.25f, 0.12f);
+  around(K_AIRBOX, at(2.85f, 0.73f, -0.12f), at(3.19f, 0.95f, 0.12f), 1.0f, 0.10f);
+  around(K_COCKPIT, at(2.20f, 0.59f, -0.215f), at(3.04f, 0.85f, 0.215f), -1.0f, -0.03f);
+  around(K_CABIN, at(2.13f, 0.48f, -0.15f), at(3.06f, 0.96f, 0.69f), 1.25f, 0.018f);
+  around(K_HELMET, at(2.52f, 0.56f, -0.15f), at(2.82f, 0.86f, 0.15f), 1.25f, 0.0f);
+  around(K_HALO, at(2.13f, 0.58f, -0.04f), at(3.06f, 0.96f, 0.30f), 1.0f, 0.0225f);
+  around(K_MIRROR, at(2.28f, 0.48f, 0.44f), at(2.47f, 0.71f, 0.69f), 1.0f, 0.0f);
+  around(K_SUSF, v3(0.84f, fminf(b + 0.15f, 0.21f), 0.13f), v3(1.44f, fmaxf(b + 0.49f, 0.54f), 0.66f), 1.0f, 0.0f);
+  around(K_SUSR, v3(4.26f, fminf(b + 0.13f, 0.20f), 0.14f), v3(4.84f, fmaxf(b + 0.44f, 0.55f), 0.57f), 1.0f, 0.0f);
+  around(K_TAIL, at(4.78f, 0.26f, -0.07f), at(5.42f, 0.50f, 0.07f), 1.25f, 0.0f);
+  around(K_FIN, at(3.40f, 0.64f, -0.008f), at(4.50f, 0.84f, 0.008f), 1.0f, 0.0f);
+  around(K_LIGHT, at(4.90f, 0.26f, -0.07f), at(5.42f, 0.50f, 0.07f), 1.0f, 0.0f);
+  around(K_FENCE, at(1.56f, 0.0f, 0.248f), at(2.12f, 0.16f, 0.432f), 1.0f, 0.0f);
+  around(K_STRAKE, at(4.28f, 0.0f, 0.292f), at(4.96f, 0.34f, 0.508f), 1.0f, 0.0f);
+  around(K_EDGE, at(2.23f, 0.03f, 0.76f), at(3.87f, 0.085f, 0.81f), 1.0f, 0.0f);
+
+  box(B_BODY, at(2.72f, 0.52f, 0.0f), v3(2.74f, 0.62f, 0.95f), 0.0f);
+  taper(T_MID, 2.20f, 3.06f, y0z(0.42f), y0z(0.42f), v2(0.25f, 0.30f), v2(0.25f, 0.34f), 0.16f, 0.16f);
+  const uint32_t nose = host_variant(S.s.nose);
+  const float x0 = (nose == 1u) ? 0.34f : 0.10f, y0 = b + ((nose == 2u) ? 0.25f : 0.17f);
+  const V2 s0 = nose == 1u ? v2(0.075f, 0.15f) : (nose == 2u ? v2(0.045f, 0.075f) : v2(0.055f, 0.11f));
+  taper(T_NOSE, x0, 1.26f, v2(y0, 0.0f), y0z(0.36f), s0, v2(0.15f, 0.17f), 0.04f, 0.12f);
+  ell(E_NOSE, v3(x0 + 0.02f, y0, 0.0f), v3(0.09f, s0.x, s0.y));
+  F.pylon = nose != 0u;
+  box(B_PYLON, v3(x0 + 0.06f, 0.5f * (yw + y0), 0.09f), v3(0.09f, 0.5f * (y0 - yw) + 0.02f, 0.006f), 0.004f);
+  taper(T_SCUTTLE, 1.20f, 2.24f, y0z(0.36f), y0z(0.42f), v2(0.15f, 0.17f), v2(0.25f, 0.29f), 0.12f, 0.16f);
+  const uint32_t cover = host_variant(S.s.cover);
+  if (cover == 1u) taper(T_COVER, 2.96f, 4.86f, y0z(0.60f), y0z(0.40f), v2(0.32f, 0.31f), v2(0.12f, 0.13f), 0.15f, 0.08f);
+  else if (cover == 2u) taper(T_COVER, 2.96f, 4.70f, y0z(0.57f), y0z(0.34f), v2(0.29f, 0.19f), v2(0.06f, 0.05f), 0.12f, 0.04f);
+  else taper(T_COVER, 2.96f, 4.86f, y0z(0.58f), y0z(0.36f), v2(0.30f, 0.24f), v2(0.08f, 0.07f), 0.14f, 0.06f);
+  taper(T_KEEL, 1.30f, 4.70f, y0z(0.22f), y0z(0.20f), v2(0.19f, 0.19f), v2(0.17f, 0.14f), 0.06f, 0.05f);
+  const uint32_t pod = host_variant(S.s.sidepod);
+  F.pod_k[0] = 0.05f; F.pod_k[1] = 0.04f; F.pod_k[2] = 0.02f;
+  F.pod_caps = pod == 1u ? 0u : (pod == 2u ? 2u : 1u);
+  cap(C_CARVE + 1, at(2.55f, 0.66f, 0.52f), at(4.00f, 0.40f, 0.36f), 0.11f);
+  if (pod == 1u) {
+    taper(T_POD, 2.30f, 4.05f, v2(b + 0.40f, 0.36f), v2(b + 0.24f, 0.24f), v2(0.16f, 0.08f), v2(0.07f, 0.05f), 0.06f, 0.04f);
+    cap(C_CARVE, v3(0.0f, 0.0f, 0.0f), v3(1.0f, 0.0f, 0.0f), 0.0f);
+    box(B_CARVE, at(2.27f, 0.42f, 0.38f), v3(0.06f, 0.12f, 0.05f), 0.03f);
+  } else if (pod == 2u) {
+    taper(T_POD, 2.30f, 4.25f, v2(b + 0.41f, 0.52f), v2(b + 0.24f, 0.30f), v2(0.18f, 0.28f), v2(0.08f, 0.11f), 0.10f, 0.05f);
+    cap(C_CARVE, at(2.30f, 0.13f, 0.84f), at(3.70f, 0.08f, 0.58f), 0.15f);
+    box(B_CARVE, at(2.28f, 0.47f, 0.57f), v3(0.06f, 0.10f, 0.17f), 0.05f);
+  } else if (pod == 3u) {
+    taper(T_POD, 2.30f, 4.25f, v2(b + 0.47f, 0.52f), v2(b + 0.26f, 0.28f), v2(0.15f, 0.25f), v2(0.07f, 0.10f), 0.12f, 0.05f);
+    cap(C_CARVE, at(2.25f, 0.17f, 0.86f), at(3.70f, 0.10f, 0.56f), 0.22f);
+    box(B_CARVE, at(2.28f, 0.52f, 0.55f), v3(0.06f, 0.07f, 0.17f), 0.04f);
+  } else {
+    taper(T_POD, 2.30f, 4.25f, v2(b + 0.41f, 0.52f), v2(b + 0.22f, 0.28f), v2(0.18f, 0.25f), v2(0.07f, 0.10f), 0.12f, 0.05f);
+    cap(C_CARVE, at(2.30f, 0.13f, 0.82f), at(3.70f, 0.08f, 0.56f), 0.16f);
+    box(B_CARVE, at(2.28f, 0.47f, 0.57f), v3(0.06f, 0.10f, 0.17f), 0.05f);
+  }
+  box(B_AIRBOX, at(3.02f, 0.84f, 0.0f), v3(0.17f, 0.11f, 0.12f), 0.08f);
+  ell(E_AIR, at(2.85f, 0.86f, 0.0f), v3(0.09f, 0.066f, 0.078f));
+  box(B_COCKPIT, at(2.62f, 0.72f, 0.0f), v3(0.42f, 0.13f, 0.215f), 0.10f);
+  ell(E_HELMET, at(2.67f, 0.71f, 0.0f), v3(0.15f, 0.13f, 0.12f));
+  cap(C_HALO, at(2.17f, 0.62f, 0.0f), at(2.36f, 0.90f, 0.0f), 0.034f);
+  cap(C_HALO + 1, at(2.36f, 0.90f, 0.0f), at(2.52f, 0.92f, 0.20f), 0.031f);
+  cap(C_HALO + 2, at(2.52f, 0.92f, 0.20f), at(2.82f, 0.88f, 0.26f), 0.031f);
+  cap(C_HALO + 3, at(2.82f, 0.88f, 0.26f), at(3.02f, 0.74f, 0.25f), 0.033f);
+  box(B_MIRROR, at(2.32f, 0.67f, 0.60f), v3(0.035f, 0.035f, 0.085f), 0.02f);
+  cap(C_MIRROR, at(2.36f, 0.66f, 0.53f), at(2.45f, 0.50f, 0.46f), 0.011f);
+  const float fz = FWZ - FHW - 0.05f, rz = RWZ - RHW - 0.05f;
+  cap(C_SUSF, at(1.10f, 0.43f, 0.17f), v3(FA + 0.02f, WR + 0.16f, fz), 0.017f);
+  cap(C_SUSF + 1, at(1.42f, 0.40f, 0.17f), v3(FA + 0.02f, WR + 0.16f, fz), 0.017f);
+  cap(C_SUSF + 2, at(0.98f, 0.19f, 0.15f), v3(FA, WR - 0.13f, fz), 0.017f);
+  cap(C_SUSF + 3, at(1.38f, 0.17f, 0.15f), v3(FA, WR - 0.13f, fz), 0.017f);
+  cap(C_SUSF + 4, v3(FA + 0.03f, WR - 0.10f, FWZ - FHW - 0.07f), at(1.20f, 0.47f, 0.16f), 0.014f);
+  cap(C_SUSF + 5, at(0.86f, 0.29f, 0.16f), v3(0.88f, WR + 0.02f, fz), 0.013f);
+  cap(C_SUSR, at(4.30f, 0.42f, 0.20f), v3(RA, WR + 0.17f, rz), 0.017f);
+  cap(C_SUSR + 1, at(4.78f, 0.40f, 0.16f), v3(RA, WR + 0.17f, rz), 0.017f);
+  cap(C_SUSR + 2, at(4.28f, 0.16f, 0.24f), v3(RA, WR - 0.14f, rz), 0.017f);
+  cap(C_SUSR + 3, at(4.82f, 0.15f, 0.18f), v3(RA, WR - 0.14f, rz), 0.017f);
+  cap(C_SUSR + 4, v3(RA - 0.03f, WR + 0.14f, RWZ - RHW - 0.07f), at(4.40f, 0.18f, 0.22f), 0.014f);
+  taper(T_TAIL, 4.78f, 5.40f, y0z(0.33f), y0z(0.33f), v2(0.07f, 0.065f), v2(0.045f, 0.045f), 0.04f, 0.03f);
+  box(B_FIN, at(3.95f, 0.74f, 0.0f), v3(0.55f, 0.10f, 0.008f), 0.006f);
+  box(B_LIGHT, at(5.405f, 0.33f, 0.0f), v3(0.012f, 0.028f, 0.05f), 0.006f);
+  cap(C_EXHAUST, at(4.95f, 0.44f, 0.0f), at(5.13f, 0.45f, 0.0f), 0.042f);
+  cap(C_BORE, at(5.0f, 0.44f, 0.0f), at(5.2f, 0.45f, 0.0f), 0.028f);
+  box(B_FLOOR, at(3.26f, 0.2f, 0.4f), v3(1.75f, 0.22f, 0.42f), 0.0f);
+  for (int i = 0; i < 2; i++) {
+    box(B_FENCE + i, at(1.84f, 0.08f, 0.26f + (float)i * 0.16f), v3(0.28f, 0.08f, 0.012f), 0.0f);
+    box(B_STRAKE + i, at(4.62f, 0.17f, 0.30f + (float)i * 0.20f), v3(0.34f, 0.17f, 0.008f), 0.0f);
+  }
+  cap(C_EDGE, at(2.25f, 0.065f, 0.79f), at(3.85f, 0.05f, 0.78f), 0.02f);
+  box(B_FRONT, v3(0.24f, yw + 0.17f, 0.48f), v3(0.36f, 0.34f, 0.50f), 0.0f);
+  box(B_REAR, at(5.20f, 0.64f, 0.27f), v3(0.46f, 0.56f, 0.29f), 0.0f);
+  const uint32_t fw = host_variant(S.s.front_wing);
+  auto plate = [&](float x, float y, float hx, float hy, float r) {
+    F.ep[0] = x; F.ep[1] = y; F.ep[2] = hx; F.ep[3] = hy; F.ep[4] = r;
+  };
+  F.front_wings = fw == 3u ? 2u : 4u;
+  if (fw == 1u) {
+    wing(0, -0.03f, yw, 0.31f, 2.0f * DEG + ff * 0.1f, 0.034f, 0.0f, 0.94f, 0.03f, 0.2f, 0.5f);
+    wing(1, 0.21f, yw + 0.036f, 0.17f, 9.0f * DEG + ff * 0.45f, 0.024f, 0.0f, 0.94f, 0.15f, 0.35f, 0.3f);
+    wing(2, 0.335f, yw + 0.075f + ff * 0.03f, 0.14f, 17.0f * DEG + ff * 0.75f, 0.020f, 0.10f, 0.94f, 0.19f, 0.35f, 0.25f);
+    wing(3, 0.425f, yw + 0.118f + ff * 0.07f, 0.12f, 26.0f * DEG + ff, 0.018f, 0.12f, 0.94f, 0.22f, 0.4f, 0.25f);
+    plate(0.25f, yw + 0.17f, 0.29f, 0.20f, 0.08f);
+  } else if (fw == 2u) {
+    wing(0, -0.03f, yw, 0.31f, 3.0f * DEG + ff * 0.1f, 0.034f, 0.0f, 0.94f, -0.02f, 0.15f, 0.55f);
+    wing(1, 0.21f, yw + 0.04f, 0.19f, 13.0f * DEG + ff * 0.45f, 0.024f, 0.0f, 0.94f, -0.04f, 0.35f, 0.35f);
+    wing(2, 0.35f, yw + 0.085f + ff * 0.03f, 0.16f, 22.0f * DEG + ff * 0.75f, 0.020f, 0.06f, 0.94f, -0.06f, 0.4f, 0.35f);
+    wing(3, 0.45f, yw + 0.13f + ff * 0.07f, 0.13f, 31.0f * DEG + ff, 0.018f, 0.08f, 0.94f, -0.08f, 0.45f, 0.35f);
+    plate(0.25f, yw + 0.06f, 0.29f, 0.10f, 0.06f);
+  } else if (fw == 3u) {
+    wing(0, -0.03f, yw, 0.30f, 1.0f * DEG + ff * 0.05f, 0.030f, 0.0f, 0.94f, 0.0f, 0.1f, 0.6f);
+    wing(1, 0.20f, yw + 0.03f, 0.16f, 4.0f * DEG + ff * 0.3f, 0.022f, 0.0f, 0.94f, 0.02f, 0.2f, 0.5f);
+    plate(0.22f, yw + 0.05f, 0.26f, 0.085f, 0.05f);
+  } else {
+    wing(0, -0.03f, yw, 0.31f, 2.0f * DEG + ff * 0.1f, 0.034f, 0.0f, 0.94f, 0.06f, 0.2f, 0.5f);
+    wing(1, 0.21f, yw + 0.036f, 0.17f, 9.0f * DEG + ff * 0.45f, 0.024f, 0.0f, 0.94f, 0.09f, 0.25f, 0.45f);
+    wing(2, 0.335f, yw + 0.075f + ff * 0.03f, 0.14f, 17.0f * DEG + ff * 0.75f, 0.020f, 0.10f, 0.94f, 0.11f, 0.25f, 0.4f);
+    wing(3, 0.425f, yw + 0.118f + ff * 0.07f, 0.12f, 26.0f * DEG + ff, 0.018f, 0.12f, 0.94f, 0.13f, 0.25f, 0.4f);
+    plate(0.25f, yw + 0.085f, 0.29f, 0.115f, 0.07f);
+  }
+  box(B_FOOT, v3(0.22f, yw - 0.008f, 0.94f - 0.04f), v3(0.30f, 0.006f, 0.06f), 0.004f);
+  wing(4, 4.98f, yr, S.chord_m, S.ang_m, 0.05f, 0.0f, 0.50f, S.rise_m, 0.12f, 0.22f);
+  wing(5, (4.98f + S.rear_c * (S.chord_m - 0.01f)) + -0.03f, (yr + S.rear_s * (S.chord_m - 0.01f)) + 0.035f, S.chord_f,
+       S.ang_f, 0.03f, 0.0f, 0.49f, S.rise_m * 0.8f, 0.10f, 0.28f);
+  cap(C_POST, v3(5.26f, yr + 0.05f, 0.0f), v3(5.30f, yr + 0.12f, 0.0f), 0.024f);
+  box(B_POST, v3(5.09f, 0.5f * (b + 0.36f + yr + 0.06f), 0.06f), v3(0.07f, 0.5f * (yr + 0.06f - b - 0.36f), 0.008f), 0.006f);
+  for (int i = 0; i < 2; i++) {
+    const V3 c = i == 0 ? v3(FA, WR26, FWZ * BODY_Z) : v3(RA26, WR26, RWZ * BODY_Z);
+    const float hw = i == 0 ? FHW26 : RHW26;
+    box(B_WHEEL + i, c, v3(WR26 + 0.02f, WR26 + 0.02f, hw + 0.2f), 0.0f);
+    box(B_DUCT + i, v3(c.x - 0.04f, c.y + 0.21f, c.z - hw - 0.05f), v3(0.16f, 0.012f, 0.05f), 0.006f);
+  }
+}
+
 // Shape plus its shape-wide constants.
 Scene make_scene(const wt_shape& shape, const CarView& car = CarView{}) {
   Scene S;
@@ -523,6 +708,8 @@ Scene make_scene(const wt_shape& shape, const CarView& car = CarView{}) {
   }
   S.rear_c = wtm::cosf(S.ang_m);
   S.rear_s = wtm::sinf(S.ang_m);
+  S.f1 = F1Tables{};
+  if (shape.kind == WT_KIND_F1) f1_tables(S);
   return S;
 }
 

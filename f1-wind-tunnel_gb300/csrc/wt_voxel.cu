@@ -22,7 +22,7 @@
 namespace wt {
 namespace {
 
-__global__ void voxelize_kernel(Scene S, uint32_t nx, uint32_t ny, uint32_t nz, float ox, float oy, float oz, float h,
+__global__ void voxelize_kernel(const __grid_constant__ Scene S, uint32_t nx, uint32_t ny, uint32_t nz, float ox, float oy, float oz, float h,
                                 uint8_t* __restrict__ solid, float* __restrict__ emit) {
   const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t y = blockIdx.y * blockDim.y + threadIdx.y;
@@ -182,7 +182,7 @@ __global__ void solid_from_u32_kernel(const uint32_t* __restrict__ in, uint8_t* 
 }  // namespace
 
 // Scene distance at the cell centres of `grid` (the first component of sceneSdf).
-__global__ void sdf_sample_kernel(Scene S, uint32_t nx, uint32_t ny, uint32_t nz, float ox, float oy, float oz,
+__global__ void sdf_sample_kernel(const __grid_constant__ Scene S, uint32_t nx, uint32_t ny, uint32_t nz, float ox, float oy, float oz,
                                   float h, float* __restrict__ out) {
   const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t y = blockIdx.y * blockDim.y + threadIdx.y;
