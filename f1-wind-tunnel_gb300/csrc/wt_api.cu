@@ -183,6 +183,8 @@ StepArgs step_args(const wt_ctx* c) {
     a.dev_guard[i] = (c->feq_guard[i] - Wd(i)) * S;
   }
   a.guard_uu = guard_threshold();
+  a.plus2 = make_float2(1.0f, 1.0f);
+  a.minus2 = make_float2(-1.0f, -1.0f);
   fill_slot_offsets(a);
   a.prefetch_ahead = c->prefetch_ahead;
   a.pop_bytes = 19ull * c->np * c->elem;

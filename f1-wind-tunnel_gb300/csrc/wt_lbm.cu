@@ -72,10 +72,32 @@ __device__ __forceinline__ float cdot(float ux, float uy, float uz) {
 
 __device__ __forceinline__ bool is_bad(float x) { return (__float_as_uint(x) & 0x7f800000u) == 0x7f800000u; }
 
+// Two FP32 operations in one instruction, each correctly rounded.  The compiler contracts
+// a product that feeds x2_add into one rounding (whatever the instructions' rounding
+// modifiers and -fmad say), and sees through a product with a constant 1: where the two
+// roundings matter the sum is x2_fma(product, one, other) with a 1 that it cannot know
+// (StepArgs::plus2).
+// The step issues in 70 % of its cycles (534 instructions a cell in f16, 755 in f32), so
+// what the directions have alike is done for two pairs of opposite directions at
+// once: f32 256x96x80 51.6 -> 50.6 us a step, 512x192x160 417 -> 403; f16 37.7 -> 36.0
+// and 302 -> 292.5, 128x48x40 7.9 -> 7.25.  (Sums and differences of the pairs too: f16
+// 512x192x160 299, more moves than operations saved.)
+struct X2 { uint64_t v; };
+__device__ __forceinline__ X2 x2(float a, float b) {
+  X2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void x2_get(X2 a, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(a.v)); }
+__device__ __forceinline__ X2 x2_add(X2 a, X2 b) { X2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
+__device__ __forceinline__ X2 x2_mul(X2 a, X2 b) { X2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
+__device__ __forceinline__ X2 x2_fma(X2 a, X2 b, X2 c) { X2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v)); return r; }
+
 // Moments, divergence guard, duct relaxation, regularized + Smagorinsky collision
 // (wgsl.ts:231-272).  f[] in, fo[] out.
 __device__ __forceinline__ CellOut collide(const float (&f)[19], float (&fo)[19], float tau0, float u_in, float ks2,
-                                           bool duct, const float (&feq_guard)[19], float guard_uu) {
+                                           bool duct, const float (&feq_guard)[19], float guard_uu,
+                                           float2 plus2, float2 minus2) {
   CellOut o;
   float rho = 0.0f, mx = 0.0f, my = 0.0f, mz = 0.0f;
   sfor<19>([&](auto I) {
@@ -127,7 +149,7 @@ __device__ __forceinline__ CellOut collide(const float (&f)[19], float (&fo)[19]
   const float uu = ux * ux + uy * uy + uz * uz;
   const float uu15 = 1.5f * uu;
   const float wr0 = Wd(0) * rho, wr1 = Wd(1) * rho, wr2 = Wd(7) * rho;
-  float eq[19];
+  float eq[19], ne[19];
   float pxx = 0.0f, pyy = 0.0f, pzz = 0.0f, pxy = 0.0f, pxz = 0.0f, pyz = 0.0f;
   // Pi^neq accumulated as each equilibrium is formed, directions in order 0..18
   // (every sum keeps the reference's order), so each incoming population dies
@@ -135,31 +157,48 @@ __device__ __forceinline__ CellOut collide(const float (&f)[19], float (&fo)[19]
   auto acc = [&](auto I) {
     constexpr int i = I;
     constexpr int cx = CXd(i), cy = CYd(i), cz = CZd(i);
-    const float ne = g[i] - eq[i];
-    if constexpr (cx != 0) pxx = pxx + ne;
-    if constexpr (cy != 0) pyy = pyy + ne;
-    if constexpr (cz != 0) pzz = pzz + ne;
-    if constexpr (cx * cy > 0) pxy = pxy + ne;
-    if constexpr (cx * cy < 0) pxy = pxy - ne;
-    if constexpr (cx * cz > 0) pxz = pxz + ne;
-    if constexpr (cx * cz < 0) pxz = pxz - ne;
-    if constexpr (cy * cz > 0) pyz = pyz + ne;
-    if constexpr (cy * cz < 0) pyz = pyz - ne;
+    const float ne_i = ne[i];
+    if constexpr (cx != 0) pxx = pxx + ne_i;
+    if constexpr (cy != 0) pyy = pyy + ne_i;
+    if constexpr (cz != 0) pzz = pzz + ne_i;
+    if constexpr (cx * cy > 0) pxy = pxy + ne_i;
+    if constexpr (cx * cy < 0) pxy = pxy - ne_i;
+    if constexpr (cx * cz > 0) pxz = pxz + ne_i;
+    if constexpr (cx * cz < 0) pxz = pxz - ne_i;
+    if constexpr (cy * cz > 0) pyz = pyz + ne_i;
+    if constexpr (cy * cz < 0) pyz = pyz - ne_i;
   };
   // Opposite directions share 3 c.u (exact negation) and 4.5 (c.u)^2 (identical bits).
   eq[0] = wr0 * (1.0f + 3.0f * 0.0f + 4.5f * 0.0f * 0.0f - uu15);
+  ne[0] = g[0] - eq[0];
   acc(std::integral_constant<int, 0>{});
-  sfor<9>([&](auto P) {
-    constexpr int i = 2 * P + 1;  // odd member of the pair (i, i + 1)
-    const float cu = cdot<i>(ux, uy, uz);
-    const float t3 = 3.0f * cu;
-    const float t45 = 4.5f * cu * cu;
-    const float wr = (i < 7 ? wr1 : wr2);
-    eq[i] = wr * (1.0f + t3 + t45 - uu15);
-    eq[i + 1] = wr * (1.0f - t3 + t45 - uu15);
+  const X2 one = x2(plus2.x, plus2.y), minus = x2(minus2.x, minus2.y), muu15 = x2(-uu15, -uu15), wr1v = x2(wr1, wr1), wr2v = x2(wr2, wr2);
+  auto two = [&](auto I) {  // the pairs (i, i + 1) and (i + 2, i + 3)
+    constexpr int i = I;
+    const X2 cu = x2(cdot<i>(ux, uy, uz), cdot<i + 2>(ux, uy, uz));
+    const X2 t3 = x2_mul(x2(3.0f, 3.0f), cu);
+    const X2 t45 = x2_mul(x2_mul(x2(4.5f, 4.5f), cu), cu);
+    const X2 wr = (i < 7 ? wr1v : wr2v);
+    const X2 ea = x2_mul(wr, x2_add(x2_fma(t45, one, x2_fma(t3, one, one)), muu15));
+    const X2 eb = x2_mul(wr, x2_add(x2_fma(t45, one, x2_fma(t3, minus, one)), muu15));
+    x2_get(ea, eq[i], eq[i + 2]);
+    x2_get(eb, eq[i + 1], eq[i + 3]);
+    x2_get(x2_fma(ea, minus, x2(g[i], g[i + 2])), ne[i], ne[i + 2]);
+    x2_get(x2_fma(eb, minus, x2(g[i + 1], g[i + 3])), ne[i + 1], ne[i + 3]);
+    sfor<4>([&](auto J) { acc(std::integral_constant<int, i + J>{}); });
+  };
+  two(std::integral_constant<int, 1>{});
+  {
+    constexpr int i = 5;  // z
+    const float t3 = 3.0f * uz, t45 = 4.5f * uz * uz;
+    eq[i] = wr1 * (1.0f + t3 + t45 - uu15);
+    eq[i + 1] = wr1 * (1.0f - t3 + t45 - uu15);
+    ne[i] = g[i] - eq[i];
+    ne[i + 1] = g[i + 1] - eq[i + 1];
     acc(std::integral_constant<int, i>{});
     acc(std::integral_constant<int, i + 1>{});
-  });
+  }
+  sfor<3>([&](auto Q) { two(std::integral_constant<int, 7 + 4 * Q>{}); });
   const float q = __fsqrt_rn(pxx * pxx + pyy * pyy + pzz * pzz + 2.0f * (pxy * pxy + pxz * pxz + pyz * pyz));
   // ks2 q / rho with rho in [0.3, 3] (or 1 after the guard) and rcp = RN(1/rho):
   // IEEE-exact for ks2 q >= 2^-60; below that the quotient (< 2^-58) vanishes in
@@ -175,6 +214,7 @@ __device__ __forceinline__ CellOut collide(const float (&f)[19], float (&fo)[19]
   const float a_zz = (1.0f - third) * pzz, b_zz = (0.0f - third) * pzz;
   const float pxy2 = 2.0f * pxy, pxz2 = 2.0f * pxz, pyz2 = 2.0f * pyz;
   fo[0] = eq[0] + k0 * ((b_xx + b_yy) + b_zz);
+  float qps[9];
   sfor<9>([&](auto P) {  // (c_a c_b - delta/3) is the same for i and opp(i)
     constexpr int i = 2 * P + 1;
     constexpr int cx = CXd(i), cy = CYd(i), cz = CZd(i);
@@ -186,10 +226,18 @@ __device__ __forceinline__ CellOut collide(const float (&f)[19], float (&fo)[19]
     if constexpr (cx * cz < 0) qp = qp - pxz2;
     if constexpr (cy * cz > 0) qp = qp + pyz2;
     if constexpr (cy * cz < 0) qp = qp - pyz2;
-    const float kq = (i < 7 ? k1 : k2) * qp;
-    fo[i] = eq[i] + kq;
-    fo[i + 1] = eq[i + 1] + kq;
+    qps[P] = qp;
   });
+  const X2 k1v = x2(k1, k1), k2v = x2(k2, k2);
+  sfor<4>([&](auto Q) {
+    constexpr int P = Q == 0 ? 0 : 2 * Q + 1, i = 2 * P + 1;
+    const X2 kq = x2_mul(i < 7 ? k1v : k2v, x2(qps[P], qps[P + 1]));
+    x2_get(x2_fma(kq, one, x2(eq[i], eq[i + 2])), fo[i], fo[i + 2]);
+    x2_get(x2_fma(kq, one, x2(eq[i + 1], eq[i + 3])), fo[i + 1], fo[i + 3]);
+  });
+  const float kz = k1 * qps[2];
+  fo[5] = eq[5] + kz;
+  fo[6] = eq[6] + kz;
   o.ux = ux; o.uy = uy; o.uz = uz; o.rho = rho; o.guard = guard;
   return o;
 }
@@ -282,16 +330,25 @@ __device__ __forceinline__ CellOut collide_dev(const float (&d)[19], float (&fo)
   const float qd[9] = {qx, qy, qz, fmaf(2.0f, pxy, bxy), fmaf(-2.0f, pxy, bxy), fmaf(2.0f, pxz, bxz),
                        fmaf(-2.0f, pxz, bxz), fmaf(2.0f, pyz, byz), fmaf(-2.0f, pyz, byz)};
   fo[0] = (S * Wd(0)) * fmaf(-k, tr3, a);
-  sfor<9>([&](auto P) {
-    constexpr int i = 2 * P + 1;
-    const float cu = cdot<i>(ux, uy, uz);
-    const float e = fmaf(r45 * cu, cu, fmaf(k, qd[P], a));
+  // pairs (x, y), (+x+y, +x-y), (+x+z, +x-z), (+y+z, +y-z) two at a time
+  const X2 r45v = x2(r45, r45), kv = x2(k, k), av = x2(a, a), r3v = x2(r3, r3);
+  sfor<4>([&](auto Q) {
+    constexpr int P = Q == 0 ? 0 : 2 * Q + 1, i = 2 * P + 1;
     constexpr float W = S * Wd(i);
-    const float ew = W * e;
-    const float lin = r3 * cu;
+    const X2 cu = x2(cdot<i>(ux, uy, uz), cdot<i + 2>(ux, uy, uz));
+    const X2 e = x2_fma(x2_mul(r45v, cu), cu, x2_fma(kv, x2(qd[P], qd[P + 1]), av));
+    const X2 ew = x2_mul(x2(W, W), e), lin = x2_mul(r3v, cu);
+    x2_get(x2_fma(x2(W, W), lin, ew), fo[i], fo[i + 2]);
+    x2_get(x2_fma(x2(-W, -W), lin, ew), fo[i + 1], fo[i + 3]);
+  });
+  {
+    constexpr int i = 5;  // z
+    const float e = fmaf(r45 * uz, uz, fmaf(k, qd[2], a));
+    constexpr float W = S * Wd(i);
+    const float ew = W * e, lin = r3 * uz;
     fo[i] = fmaf(W, lin, ew);
     fo[i + 1] = fmaf(-W, lin, ew);
-  });
+  }
   o.ux = ux; o.uy = uy; o.uz = uz; o.rho = rho; o.guard = guard;
   return o;
 }
@@ -600,7 +657,8 @@ __device__ __forceinline__ void step_tile(const StepArgs& a, const Ofs& ofs, For
     if constexpr (R::dev)
       o = collide_dev<St>(f, fo, __ldg(a.tau0_x + x), a.u_in, a.ks2, (cw & CW_DUCT) != 0, a.guard_uu);
     else
-      o = collide(f, fo, __ldg(a.tau0_x + x), a.u_in, a.ks2, (cw & CW_DUCT) != 0, a.feq_guard, a.guard_uu);
+      o = collide(f, fo, __ldg(a.tau0_x + x), a.u_in, a.ks2, (cw & CW_DUCT) != 0, a.feq_guard, a.guard_uu,
+                  a.plus2, a.minus2);
     if (o.guard) {
 #pragma unroll
       for (int k = 0; k < 9; k++) gf[k] = 0.0f;
