@@ -183,7 +183,7 @@ def run_reference_arm(args, rank, world):
 
 
 def run_aeromap(args, rank, world, dist):
-    """Batched aero map: all cases advanced by one launch per LBM step."""
+    """Batched aero map: all cases advanced by one call."""
     import torch
     import windtunnel
     from windtunnel.workloads import aeromap_cases
@@ -212,7 +212,7 @@ def run_aeromap(args, rank, world, dist):
             "warmup": max(3, args.warmup), "ms_per_step": ms / args.steps, "higher_is_better": True,
             "scaling": "weak", "vs_baseline": None, "dtype": args.storage, "data": "synthetic",
             "config": {"workload": f"batched aero map: {len(cases)} lattices ({cells} cells), 8 LBM steps per step, "
-                                   "one launch per LBM step, CUDA graph", "block": f"{tuned[0]}x{tuned[1]} (autotuned)"},
+                                   "single-lattice launches in chains, CUDA graph", "block": f"{tuned[0]}x{tuned[1]} (autotuned)"},
             "roofline": {"bound": "hbm", "achieved": cells * bpl * 8 * args.steps / (ms / 1e3) / 1e9, "peak": peak,
                          "unit": "GB/s", "peak_source": kind}}
     line["roofline"]["frac"] = line["roofline"]["achieved"] / peak
