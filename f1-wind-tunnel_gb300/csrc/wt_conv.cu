@@ -428,7 +428,8 @@ __global__ void __launch_bounds__(ROW_THREADS) conv_rows_kernel(RowArgs p) {
 // WGRAD: D[co][(dy, ci)] += sum over a tile's voxels of dy[m][co] x[m + off][ci].
 //
 // A block owns one dz and one or all three dx (its accumulators in tensor memory)
-// and a range of tiles (16 numbered rows x 8 XG voxels, as above) for which it
+// and the rows that start in its share of the voxels, in tiles (up to 16 numbered rows x 8 XG
+// voxels, as above) for which it
 // loads the output gradient and, with its halo, the input, into two buffers in
 // turn.  Both operands are M/N-major: 8 channels of a voxel are 16 contiguous
 // bytes, 8 voxels along x one core matrix, and the channel groups of a row are laid
@@ -438,7 +439,7 @@ __global__ void __launch_bounds__(ROW_THREADS) conv_rows_kernel(RowArgs p) {
 // two groups of 8 voxels.  Only rows of the grid are walked: the K steps of a tile
 // are tabulated by the loaders from the rows' validity, an odd group paired with
 // zeros.  Measured, the network's 12 distinct layers at batch 16 / 1 (us in all, with
-// the reduction): 3620 -> 792 / 1390 -> 252 against a gather of every tap's K slices
+// the reduction): 3620 -> 860 / 1390 -> 252 against a gather of every tap's K slices
 // through registers with 2-byte stores.  What bounds it now: on the wide layers the
 // MMAs (cout of 8-16 uses an eighth to a quarter of M), on the others the copies'
 // latency per tile.  M is 64 or 128: rows above cout are computed from whatever follows in
@@ -456,7 +457,9 @@ struct WgradArgs {
   uint32_t gpx, gpy;       // bytes per channel group of a row
   uint32_t xrows;          // rows of the x tile
   uint32_t xofs, buf;      // offset of the x tile in a buffer, bytes per buffer
-  uint32_t xg, ctiles, tiles, splits;
+  uint32_t xg, ctiles, rt; // voxel groups and rows of a tile
+  uint32_t vrows;          // rows of the grid
+  uint64_t k_chunk;        // voxels of a split
   uint32_t groups;         // x groups of a row of the grid
   uint32_t dxs;            // dx per block: 3, or 1 (one also splits cin into chunks)
   uint32_t m, n, bstep;    // M and N of one MMA; bytes between the x operands of an MMA and the next of its K step
@@ -471,7 +474,7 @@ constexpr uint32_t WG_THREADS = ROW_THREADS + 32;                        // load
 // Voxels of the tile's gradient rows and x rows (-1: zeros) and its K steps.
 struct WgTile {
   int32_t yv[ROW_TILE], xv[ROW_TILE + 2];
-  uint32_t steps, pad;
+  uint32_t steps, xl;      // first voxel in x; bit 31: the block's last tile
   uint2 step[WG_STEPS];    // descriptor low words of dy and x
 };
 static_assert(sizeof(WgTile) == 400 && WG_HEAD % 128 == 0, "tables fit the head");
@@ -493,7 +496,14 @@ __global__ void __launch_bounds__(WG_THREADS) conv_wgrad_kernel(WgradArgs p) {
   const uint32_t split = blockIdx.x, tg = blockIdx.y / p.chunks, g0 = (blockIdx.y - tg * p.chunks) * p.cgx;
   const int dz = p.halo ? (int)(p.dxs == 3 ? tg : tg / 3u) - 1 : 0;
   const uint32_t dx0 = p.halo && p.dxs == 1 ? tg % 3u : 0u;  // first dx + 1 of this block
-  const uint32_t tb = (uint32_t)((uint64_t)split * p.tiles / p.splits), te = (uint32_t)((uint64_t)(split + 1) * p.tiles / p.splits);
+  // this block's rows: those that start in its voxels, as numbered rows [rb, re)
+  auto numbered = [&](uint32_t q) {
+    const uint32_t zz = q / p.h, bb = zz / p.d;
+    return (bb * p.dp + zz - bb * p.d) * p.hp + q - zz * p.h;
+  };
+  const uint32_t q0 = (uint32_t)min((uint64_t)p.vrows, split * p.k_chunk / p.w), q1 = (uint32_t)min((uint64_t)p.vrows, (split + 1) * p.k_chunk / p.w);
+  const bool any = q0 < q1;
+  const uint32_t rb = any ? numbered(q0) : 0u, re = any ? numbered(q1 - 1) + 1 : 0u;
   // dx = -1 never reads the last column; where a row's last group reaches past the
   // grid, its gradient there is zero and so has to be x (0 times infinity)
   const uint32_t xlim = p.halo && p.dxs == 1 && dx0 == 0 ? p.w - 1 : p.w;
@@ -533,13 +543,14 @@ __global__ void __launch_bounds__(WG_THREADS) conv_wgrad_kernel(WgradArgs p) {
     uint32_t elected;
     asm volatile("{\n .reg .pred q;\n elect.sync _|q, 0xffffffff;\n selp.u32 %0, 1, 0, q;\n}\n" : "=r"(elected));
     uint32_t acc = 0, kt = 0, b = 0, phase = 0, tab = 0, tphase = 0;
-    for (uint32_t i = tb; i < te; i++, kt++) {
+    for (bool more = any; more; kt++) {
       ok = mbar_wait_or(smem_u32(&tfull[tab]), tphase, stop) && mbar_wait_or(smem_u32(&full[b]), phase, stop);
       if (!__all_sync(0xffffffffu, ok)) {
         ok = false;
         if (elected) *reinterpret_cast<volatile uint32_t*>(stop) = 1u;
         break;
       }
+      more = !(tile[tab].xl >> 31);
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       if (elected) {
@@ -573,9 +584,11 @@ __global__ void __launch_bounds__(WG_THREADS) conv_wgrad_kernel(WgradArgs p) {
       ok = mbar_wait(last, ph, WAIT_LIMIT) && ok;  // before the tensor memory is freed, whatever came before
     }
   } else if (warp == ROW_LOADERS / 32 + 1) {
-    // Rows and K steps of tile i (buffer b), by one warp.
-    auto make_table = [&](uint32_t i, uint32_t b, WgTile& T) {
-      const uint32_t base = s0 + b * p.buf, x0 = (i % p.ctiles) * p.xg * 8u, r0 = (i / p.ctiles) * ROW_TILE;
+    // Rows and K steps of the tile at row r0 and voxel x0 (buffer b), by one warp; the first
+    // row that it leaves.  With an odd number of groups in all, the last row is left to
+    // the next tile: K steps are the 16 voxels that follow one another in the grid.
+    auto make_table = [&](uint32_t r0, uint32_t x0, uint32_t b, WgTile& T) -> uint32_t {
+      const uint32_t base = s0 + b * p.buf;
       const uint32_t ng = min(p.xg, p.groups - (x0 >> 3));
       auto voxel = [&](int64_t R) -> int32_t {
         if (R < 0 || R >= (int64_t)p.rows) return -1;
@@ -583,9 +596,16 @@ __global__ void __launch_bounds__(WG_THREADS) conv_wgrad_kernel(WgradArgs p) {
         return y < p.h && z < p.d ? (int32_t)(((bb * p.d + z) * p.h + y) * p.w) : -1;
       };
       if (lane < p.xrows) T.xv[lane] = voxel((int64_t)r0 + dz * (int)p.hp + lane - p.halo);
-      const int32_t yv = lane < ROW_TILE ? voxel((int64_t)r0 + lane) : -1;
-      if (lane < ROW_TILE) T.yv[lane] = yv;
-      const uint32_t valid = __ballot_sync(0xffffffffu, yv >= 0), units = __popc(valid) * ng;
+      int32_t yv = lane < p.rt && r0 + lane < re ? voxel((int64_t)r0 + lane) : -1;
+      uint32_t valid = __ballot_sync(0xffffffffu, yv >= 0), next = r0 + p.rt;
+      if (p.ctiles == 1 && next < re && (__popc(valid) * ng & 1u) && __popc(valid) > 1) {
+        const uint32_t l = 31u - __clz(valid);
+        valid &= ~(1u << l);
+        next = r0 + l;
+        if (lane == l) yv = -1;
+      }
+      const uint32_t units = __popc(valid) * ng;
+      if (lane < p.rt) T.yv[lane] = yv;
       if (lane == 0) T.steps = (units + 1) / 2;
       const uint32_t u = 2u * lane;
       if (u < units) {
@@ -607,18 +627,25 @@ __global__ void __launch_bounds__(WG_THREADS) conv_wgrad_kernel(WgradArgs p) {
         }
         T.step[lane] = make_uint2((aa >> 4) | ((la >> 4) << 16), (xa >> 4) | ((lx >> 4) << 16));
       }
+      return next;
     };
     // (Formed by a loading warp between its copies a table kept the others waiting for
     // 2300 cycles a tile.)
-    uint32_t kt = 0, b = 0, tab = 0, phase = 1;
-    for (uint32_t i = tb; i < te; i++, kt++) {
+    uint32_t kt = 0, b = 0, tab = 0, phase = 1, r = rb, c = 0;
+    for (bool more = any; more; kt++) {
       if (kt >= WG_TABLES) ok = mbar_wait_or(smem_u32(&tfree[tab]), phase, stop);
       if (!__all_sync(0xffffffffu, ok)) {
         ok = false;
         *reinterpret_cast<volatile uint32_t*>(stop) = 1u;
         break;
       }
-      make_table(i, b, tile[tab]);
+      const uint32_t next = make_table(r, c * p.xg * 8u, b, tile[tab]);
+      if (lane == 0) tile[tab].xl = c * p.xg * 8u | (c + 1 == p.ctiles && next >= re ? 1u << 31 : 0u);
+      if (++c == p.ctiles) {
+        c = 0;
+        r = next;
+        more = r < re;
+      }
       __syncwarp();
       if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&tfull[tab])) : "memory");
       if (++tab == WG_TABLES) {
@@ -629,7 +656,7 @@ __global__ void __launch_bounds__(WG_THREADS) conv_wgrad_kernel(WgradArgs p) {
     }
   } else {
     uint32_t kt = 0, b = 0, phase = 1, tab = 0, tphase = 0;
-    for (uint32_t i = tb; i < te; i++, kt++) {
+    for (bool more = any; more; kt++) {
       const uint32_t base = s0 + b * p.buf;
       ok = mbar_wait_or(smem_u32(&tfull[tab]), tphase, stop) && (kt < p.nbuf || mbar_wait_or(smem_u32(&done[b]), phase, stop));
       if (!ok) {
@@ -637,12 +664,13 @@ __global__ void __launch_bounds__(WG_THREADS) conv_wgrad_kernel(WgradArgs p) {
         break;
       }
       const WgTile& T = tile[tab];
-      const uint32_t x0 = (i % p.ctiles) * p.xg * 8u;
+      const uint32_t x0 = T.xl & 0x7fffffffu;
+      more = !(T.xl >> 31);
       {
         const uint32_t per = 8u * p.xg * p.cgy, q = ROW_LOADERS / per, rem = ROW_LOADERS - q * per;
         uint32_t r = t / per, e = t - r * per;
 #pragma unroll 4
-        for (uint32_t k = t; k < ROW_TILE * per; k += ROW_LOADERS) {
+        for (uint32_t k = t; k < p.rt * per; k += ROW_LOADERS) {
           const int32_t v0 = T.yv[r];
           const uint32_t xx = (e * p.magy) >> 16, g = e - xx * p.cgy, x = x0 + xx;
           const bool in = v0 >= 0 && x < p.w && (uint32_t)v0 + x < p.M;
@@ -911,8 +939,8 @@ int launch_wgrad(const wt_conv_shape* s, const void* x, const void* dy, float* w
   p.cgy = p.cout / 8;
   p.magy = (65536u + p.cgy - 1) / p.cgy;
   p.groups = (p.w + 7) / 8;
-  p.splits = splits;
-  p.xrows = ROW_TILE + 2 * p.halo;
+  p.vrows = p.halo ? batch * p.d * p.h : p.h;
+  p.k_chunk = (((uint64_t)p.M + splits - 1) / splits + 63) / 64 * 64;
   p.stage_wait = g_stage_wait.load();
   p.throttle = p.M / splits > 128 ? 1u : 0u;
   auto r16 = [](uint32_t v) { return (v + 15) / 16 * 16; };
@@ -933,21 +961,29 @@ int launch_wgrad(const wt_conv_shape* s, const void* x, const void* dy, float* w
   p.n = r16((p.halo && !(nm == 3 && p.dxs == 1) ? 3 : 1) * p.cgx * 8);
   p.magx = (65536u + p.cgx - 1) / p.cgx;
   uint32_t smem = 0;
-  for (p.xg = p.groups >= 3 ? 4 : p.groups; ; p.xg /= 2) {
+  // Rows of up to 4 groups, or of 8, whole where they are full: the K steps are then the 16
+  // voxels that follow one another in the grid, in their order, and the sums the same
+  // bits as those of a plain walk over the voxels (a training run amplifies the last bit:
+  // Adam's first steps divide gradients by themselves).  There the tile's rows shrink
+  // until it fits, elsewhere its groups.
+  const bool eight = p.groups == 8 && p.w % 8 == 0, whole = eight || (p.groups <= 4 && p.w % 8 == 0);
+  for (p.xg = eight ? 8 : p.groups >= 3 ? 4 : p.groups, p.rt = eight ? 8 : ROW_TILE; ;) {
+    p.xrows = p.rt + 2 * p.halo;
     p.W = 8 * p.xg + 2 * p.halo;
     p.gpx = pad_pitch(p.W * 16, p.cgx);
     p.gpy = pad_pitch(8 * p.xg * 16, p.cgy);
-    p.xofs = ROW_TILE * p.cgy * p.gpy;
+    p.xofs = p.rt * p.cgy * p.gpy;
     p.buf = (p.xofs + p.xrows * p.cgx * p.gpx + 127) / 128 * 128;
     // after the buffers: the zero row, and what the junk M rows and N columns of the last rows read
     const uint32_t rest = WG_HEAD + 16 * p.gpy + 16 * p.gpx + 2048, most = blocks > SMS ? SMEM_MAX / 2 : SMEM_MAX;
     for (p.nbuf = WG_BUFS; p.nbuf > 2 && rest + p.nbuf * p.buf > most; p.nbuf--) {}
     smem = rest + p.nbuf * p.buf;
-    if (p.xg == 1 || smem <= most) break;
+    if (smem <= most || (p.xg == 1 && (!whole || p.rt == 4))) break;
+    if (whole && p.rt > 4) p.rt /= 2;
+    else p.xg /= 2, p.rt = ROW_TILE;
   }
   p.bstep = p.dxs == 3 ? 16u : p.cgx * p.gpx;
   p.ctiles = (p.groups + p.xg - 1) / p.xg;
-  p.tiles = (p.rows + ROW_TILE - 1) / ROW_TILE * p.ctiles;
   for (p.cols = 32; p.cols < nm * p.n; p.cols *= 2) {}
   const dim3 grid(splits, (p.halo ? (p.dxs == 3 ? 3 : 9) : 1) * p.chunks);
   const auto kernel = nm == 3 ? conv_wgrad_kernel<3> : conv_wgrad_kernel<1>;

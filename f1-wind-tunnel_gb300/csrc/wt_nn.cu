@@ -256,55 +256,42 @@ __global__ void grad_to_bf16_kernel(const float* __restrict__ g, const float* __
 
 // Bias gradient in two passes with a fixed summation order: block b of the first
 // pass sums rows [b * chunk, (b + 1) * chunk) of every channel (each thread the rows
-// of its phase, 8 channels at a time where the rows come in aligned 16-byte chunks,
-// then the block folds its phases in order) into partial[b][c]; the second pass sums
-// the blocks, 32 phases per channel folded in order.  (One thread per channel
-// summed the 512 partials in 10 us a layer, more than the rest of the gradient.)
+// of its phase, the phases folded in order) into partial[b][c]; the second pass sums
+// the blocks in order, which is kept because a training run amplifies the last bit.  Eight
+// channels a thread and 32 phases per channel in the second pass took 103 us of a batch-16
+// step, this 175, one thread per channel over global memory 10 us a layer more.
 constexpr uint32_t BG_BLOCKS = 512;
 
-template <int V>  // channels per thread: 8 or 1; V divides c, c / V divides TB
 __global__ void bias_grad_partial_kernel(const __nv_bfloat16* __restrict__ dy, float* __restrict__ partial,
                                          uint64_t rows, uint32_t c, uint64_t chunk) {
-  __shared__ float red[V][TB];
-  const uint32_t per = c / V, phases = TB / per;
-  const uint32_t k = threadIdx.x % per, ph = threadIdx.x / per;
+  __shared__ float red[TB];
+  const uint32_t phases = TB / c, ch = threadIdx.x % c, ph = threadIdx.x / c;
   const uint64_t r0 = (uint64_t)blockIdx.x * chunk, r1 = min(rows, r0 + chunk);
-  float acc[V] = {};
-#pragma unroll 4
-  for (uint64_t r = r0 + ph; r < r1; r += phases) {
-    if constexpr (V == 8) {
-      const Bf8 v{reinterpret_cast<const uint4*>(dy)[r * per + k]};
-#pragma unroll
-      for (int e = 0; e < 8; e++) acc[e] += v.get(e);
-    } else {
-      acc[0] += __bfloat162float(dy[r * c + k]);
-    }
-  }
-#pragma unroll
-  for (int e = 0; e < V; e++) red[e][threadIdx.x] = acc[e];
+  float acc = 0.0f;
+#pragma unroll 8
+  for (uint64_t r = r0 + ph; r < r1; r += phases) acc += __bfloat162float(dy[r * c + ch]);
+  red[threadIdx.x] = acc;
   __syncthreads();
   if (threadIdx.x < c) {
-    const uint32_t kk = threadIdx.x / V, e = threadIdx.x % V;
     float t = 0.0f;
-    for (uint32_t q = 0; q < phases; q++) t += red[e][q * per + kk];
+    for (uint32_t q = 0; q < phases; q++) t += red[q * c + threadIdx.x];
     partial[(size_t)blockIdx.x * c + threadIdx.x] = t;
   }
 }
-
+// Eight channels to a block: the partial sums through shared memory, then in order (a thread
+// walking them in global memory waits for each load).
 __global__ void bias_grad_final_kernel(const float* __restrict__ partial, float* __restrict__ db, uint32_t nblocks,
                                        uint32_t c) {
-  __shared__ float red[TB];
-  const uint32_t ch = blockIdx.x * 8 + (threadIdx.x & 7u), ph = threadIdx.x >> 3;
-  float t = 0.0f;
-  if (ch < c)
-#pragma unroll 4
-    for (uint32_t b = ph; b < nblocks; b += TB / 8) t += partial[(size_t)b * c + ch];
-  red[threadIdx.x] = t;
+  __shared__ float sh[BG_BLOCKS * 8];
+  const uint32_t c0 = blockIdx.x * 8, n = min(8u, c - c0);
+  for (uint32_t i = threadIdx.x; i < nblocks * 8; i += TB)
+    if ((i & 7u) < n) sh[i] = partial[(size_t)(i >> 3) * c + c0 + (i & 7u)];
   __syncthreads();
-  if (threadIdx.x < 8 && ch < c) {
-    float v = 0.0f;
-    for (uint32_t q = 0; q < TB / 8; q++) v += red[8 * q + threadIdx.x];
-    db[ch] = v;
+  if (threadIdx.x < n) {
+    float t = 0.0f;
+#pragma unroll 8
+    for (uint32_t b = 0; b < nblocks; b++) t += sh[8 * b + threadIdx.x];
+    db[c0 + threadIdx.x] = t;
   }
 }
 
@@ -533,10 +520,7 @@ int wt_nn_bias_grad(const void* dy, float* db, uint64_t rows, uint32_t c, void* 
     return bad("wt_nn_bias_grad scratch");
   const uint64_t chunk = rows ? (rows + BG_BLOCKS - 1) / BG_BLOCKS : 1;
   const uint32_t nb = (uint32_t)(rows ? (rows + chunk - 1) / chunk : 1);
-  if (c % 8 == 0 && aligned16(dy))
-    bias_grad_partial_kernel<8><<<nb, TB, 0, S(stream)>>>(static_cast<const bf*>(dy), partial, rows, c, chunk);
-  else
-    bias_grad_partial_kernel<1><<<nb, TB, 0, S(stream)>>>(static_cast<const bf*>(dy), partial, rows, c, chunk);
+  bias_grad_partial_kernel<<<nb, TB, 0, S(stream)>>>(static_cast<const bf*>(dy), partial, rows, c, chunk);
   bias_grad_final_kernel<<<(c + 7) / 8, TB, 0, S(stream)>>>(partial, db, nb, c);
   return done("wt_nn_bias_grad");
 }
