@@ -47,16 +47,9 @@ std::atomic<uint32_t> g_stage_wait{WAIT_LIMIT};
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
-// Shared-memory matrix descriptor (tcgen05): start address, leading (K-direction)
-// and stride (M/N-direction) byte offsets, all >> 4; bits 46-47 = 1 (the
-// descriptor version of this architecture); no swizzle, base offset 0.
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
-  uint64_t d = (uint64_t)((addr >> 4) & 0x3FFFu);
-  d |= (uint64_t)((lbo >> 4) & 0x3FFFu) << 16;
-  d |= (uint64_t)((sbo >> 4) & 0x3FFFu) << 32;
-  d |= (uint64_t)1 << 46;
-  return d;
-}
+// Shared-memory matrix descriptors (tcgen05) are start address (bits 0-13), leading and
+// stride byte offsets (16-29, 32-45), all >> 4; bits 46-47 = 1 (the descriptor version of this
+// architecture); no swizzle, base offset 0.
 
 // Instruction descriptor of kind::f16: D FP32 (bits 4-5 = 1), A and B BF16
 // (bits 7-9 = 1, 10-12 = 1), both K-major (bits 15, 16 = 0) or both M/N-major (1),
