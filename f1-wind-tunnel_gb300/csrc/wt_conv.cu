@@ -21,6 +21,7 @@
 
 #include <string>
 
+#include "wt_conv_plan.h"
 #include "wt_internal.h"
 #include "wt_net.h"
 
@@ -126,7 +127,6 @@ struct RowArgs {
   uint32_t stage_wait;
 };
 
-constexpr uint32_t ROW_TILE = 16, ROW_ROWS = 3 * (ROW_TILE + 2), ROW_HEAD = 512;  // ROW_HEAD: barriers, slot, ROW_ROWS row voxels
 // Bytes of the head and of the MMAs' tables.
 __host__ __device__ constexpr uint32_t row_tables(uint32_t units) { return (ROW_HEAD + (units + 3) / 4 * 4 * 12 + 127) / 128 * 128; }
 
@@ -146,7 +146,6 @@ __device__ __forceinline__ int32_t row_voxel(const RowArgs& p, int64_t R) {
 // st - depth are done (done[slot], committed by the issuing lane); full[slot]
 // completes when its copies have landed, and the issuing warp makes them visible to
 // the tensor cores.  At most two stages of MMAs are in flight.
-constexpr uint32_t ROW_LOADERS = 256, ROW_THREADS = ROW_LOADERS + 32, ROW_DEPTH_MAX = 16;
 
 // mbar_wait that also ends when the block has been told to stop.
 __device__ __forceinline__ bool mbar_wait_or(uint32_t bar, uint32_t parity, const volatile uint32_t* stop) {
@@ -437,33 +436,6 @@ __global__ void __launch_bounds__(ROW_THREADS) conv_rows_kernel(RowArgs p) {
 // MMAs (cout of 8-16 uses an eighth to a quarter of M), on the others the copies'
 // latency per tile.  M is 64 or 128: rows above cout are computed from whatever follows in
 // shared memory and not read.
-struct WgradArgs {
-  const __nv_bfloat16 *x, *dy;
-  float* ws;               // [split][taps * cin][cout]
-  uint32_t cin, cout, taps;
-  uint32_t d, h, w, M, hp, dp, rows;  // as RowArgs
-  uint32_t cgx, cgy;       // channel groups of x in a block, and of dy
-  uint32_t chunks;         // blocks along cin
-  uint32_t nbuf;           // tile buffers
-  uint32_t magx, magy;     // ceil(2^16 / cgx), ceil(2^16 / cgy)
-  uint32_t halo, W;        // voxels per row of the x tile
-  uint32_t gpx, gpy;       // bytes per channel group of a row
-  uint32_t xrows;          // rows of the x tile
-  uint32_t xofs, buf;      // offset of the x tile in a buffer, bytes per buffer
-  uint32_t xg, ctiles, rt; // voxel groups and rows of a tile
-  uint32_t vrows;          // rows of the grid
-  uint64_t k_chunk;        // voxels of a split
-  uint32_t groups;         // x groups of a row of the grid
-  uint32_t dxs;            // dx per block: 3, or 1 (one also splits cin into chunks)
-  uint32_t m, n, bstep;    // M and N of one MMA; bytes between the x operands of an MMA and the next of its K step
-  uint32_t cols;           // tensor-memory columns
-  uint32_t stage_wait, throttle;  // throttle: more than two K slices of 64 voxels
-};
-
-constexpr uint32_t WG_STEPS = 32, WG_BUFS = 4, WG_TABLES = WG_BUFS + 2;  // K steps of a tile
-constexpr uint32_t WG_HEAD = 256 + WG_TABLES * 400 + 32;               // barriers, tables
-constexpr uint32_t WG_THREADS = ROW_THREADS + 32;                        // loaders, issuer, table warp
-
 // Voxels of the tile's gradient rows and x rows (-1: zeros) and its K steps.
 struct WgTile {
   int32_t yv[ROW_TILE], xv[ROW_TILE + 2];
@@ -792,28 +764,10 @@ int check_shape(const wt_conv_shape* s, const char* what) {
   return WT_OK;
 }
 
-constexpr uint32_t WGRAD_SPLITS_MAX = 64;
-
-uint32_t wgrad_splits(uint64_t voxels) {
-  // about 4096 voxels (64 slices of 64) per split, at most WGRAD_SPLITS_MAX
-  uint64_t s = (voxels + 4095) / 4096;
-  if (s < 1) s = 1;
-  if (s > WGRAD_SPLITS_MAX) s = WGRAD_SPLITS_MAX;
-  return (uint32_t)s;
-}
-
 // Tiling of conv_rows_kernel.  Wide tiles (xg groups of 8 voxels along x) share
 // their halo and their weights; narrow ones and a split of N give a small grid
 // enough blocks.  Shared memory of a block stays below a third of an SM's where it
 // can, so that several blocks overlap their loads, MMAs and epilogues.
-constexpr uint32_t SMS = 152, SMEM_MAX = 227 * 1024, SMEM_THIRD = 74 * 1024;
-
-// A channel group's pitch such that eight successive 16-byte copies (channel groups
-// fastest, then voxels) fall in different banks: 64, 32 or 16 mod 128 bytes.
-uint32_t pad_pitch(uint32_t bytes, uint32_t cg) {
-  const uint32_t want = cg >= 8 ? 16u : cg >= 4 ? 32u : cg >= 2 ? 64u : 0u;
-  return bytes + (want + 128u - bytes % 128u) % 128u;
-}
 
 template <int MODE, int XG>
 int launch_rows_xg(const RowArgs& p, uint32_t smem, dim3 grid, cudaStream_t st) {
@@ -905,79 +859,14 @@ int launch_rows(const wt_conv_shape* s, const void* a, const void* b, const floa
   return launch_rows_xg<MODE, 1>(p, smem, grid, st);
 }
 
-// Tiling of conv_wgrad_kernel.  A block takes all three dx where their accumulators
-// fit the tensor memory (9 cin columns), the splits alone give every SM a block and
-// rows end with a group of 8; otherwise one dx, for a finer grid, and where that
-// still leaves SMs idle, cin in chunks (16 channels at least).  The workspace bounds
-// the splits.
 int launch_wgrad(const wt_conv_shape* s, const void* x, const void* dy, float* ws, uint32_t splits, cudaStream_t st) {
   WgradArgs p = {};
   p.x = static_cast<const __nv_bfloat16*>(x);
   p.dy = static_cast<const __nv_bfloat16*>(dy);
   p.ws = ws;
-  p.cin = s->cin, p.cout = s->cout, p.taps = s->taps;
-  p.M = s->batch * s->d * s->h * s->w;
-  p.halo = s->taps == 27 ? 1u : 0u;
-  uint32_t batch = s->batch;
-  if (p.halo) {
-    p.d = s->d, p.h = s->h, p.w = s->w;
-    p.hp = p.h + 1, p.dp = p.d + 1;
-  } else {
-    batch = 1, p.d = 1, p.w = 32, p.h = (p.M + 31) / 32;
-    p.hp = p.h, p.dp = 1;
-  }
-  const uint64_t rows = ((uint64_t)batch * p.dp - p.halo) * p.hp - p.halo;  // up to the last row of the grid
-  if (rows >= (1ull << 31)) return nfail(WT_ERR_ARG, "convolution: grid too large");
-  p.rows = (uint32_t)rows;
-  p.cgy = p.cout / 8;
-  p.magy = (65536u + p.cgy - 1) / p.cgy;
-  p.groups = (p.w + 7) / 8;
-  p.vrows = p.halo ? batch * p.d * p.h : p.h;
-  p.k_chunk = (((uint64_t)p.M + splits - 1) / splits + 63) / 64 * 64;
   p.stage_wait = g_stage_wait.load();
-  p.throttle = p.M / splits > 128 ? 1u : 0u;
-  auto r16 = [](uint32_t v) { return (v + 15) / 16 * 16; };
-  const uint32_t cg = p.cin / 8, n3 = r16(3 * p.cin);
-  uint32_t nm = 1, blocks = splits * (p.halo ? 9 : 1);
-  p.cgx = cg;
-  p.dxs = 1;
-  if (p.halo && 3 * n3 <= 512 && 3 * splits >= SMS && p.w % 8 == 0) {
-    p.dxs = nm = 3;
-    blocks = 3 * splits;
-  } else {
-    while (p.cgx > 2 && blocks * ((cg + p.cgx - 1) / p.cgx) < SMS) p.cgx = (p.cgx + 1) / 2;
-    if (p.halo && 3 * p.cgx * 8 > 256) nm = 3;  // one MMA per dy
-  }
-  p.chunks = (cg + p.cgx - 1) / p.cgx;
-  blocks *= p.chunks;
-  p.m = p.cout <= 64 ? 64 : 128;  // (N 48: 29 and 44 cycles an MMA)
-  p.n = r16((p.halo && !(nm == 3 && p.dxs == 1) ? 3 : 1) * p.cgx * 8);
-  p.magx = (65536u + p.cgx - 1) / p.cgx;
-  uint32_t smem = 0;
-  // Rows of up to 4 groups, or of 8, whole where they are full: the K steps are then the 16
-  // voxels that follow one another in the grid, in their order, and the sums the same
-  // bits as those of a plain walk over the voxels (a training run amplifies the last bit:
-  // Adam's first steps divide gradients by themselves).  There the tile's rows shrink
-  // until it fits, elsewhere its groups.
-  const bool eight = p.groups == 8 && p.w % 8 == 0, whole = eight || (p.groups <= 4 && p.w % 8 == 0);
-  for (p.xg = eight ? 8 : p.groups >= 3 ? 4 : p.groups, p.rt = eight ? 8 : ROW_TILE; ;) {
-    p.xrows = p.rt + 2 * p.halo;
-    p.W = 8 * p.xg + 2 * p.halo;
-    p.gpx = pad_pitch(p.W * 16, p.cgx);
-    p.gpy = pad_pitch(8 * p.xg * 16, p.cgy);
-    p.xofs = p.rt * p.cgy * p.gpy;
-    p.buf = (p.xofs + p.xrows * p.cgx * p.gpx + 127) / 128 * 128;
-    // after the buffers: the zero row, and what the junk M rows and N columns of the last rows read
-    const uint32_t rest = WG_HEAD + 16 * p.gpy + 16 * p.gpx + 2048, most = blocks > SMS ? SMEM_MAX / 2 : SMEM_MAX;
-    for (p.nbuf = WG_BUFS; p.nbuf > 2 && rest + p.nbuf * p.buf > most; p.nbuf--) {}
-    smem = rest + p.nbuf * p.buf;
-    if (smem <= most || (p.xg == 1 && (!whole || p.rt == 4))) break;
-    if (whole && p.rt > 4) p.rt /= 2;
-    else p.xg /= 2, p.rt = ROW_TILE;
-  }
-  p.bstep = p.dxs == 3 ? 16u : p.cgx * p.gpx;
-  p.ctiles = (p.groups + p.xg - 1) / p.xg;
-  for (p.cols = 32; p.cols < nm * p.n; p.cols *= 2) {}
+  uint32_t nm = 0, smem = 0;
+  if (!plan_wgrad(*s, splits, p, nm, smem)) return nfail(WT_ERR_ARG, "convolution: grid too large");
   const dim3 grid(splits, (p.halo ? (p.dxs == 3 ? 3 : 9) : 1) * p.chunks);
   const auto kernel = nm == 3 ? conv_wgrad_kernel<3> : conv_wgrad_kernel<1>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX);
