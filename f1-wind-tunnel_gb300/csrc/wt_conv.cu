@@ -11,6 +11,7 @@
 // shared memory and runs all 27 taps on it; a tap is a shift of the matrix
 // descriptor's start address, so every input value is fetched once per tile
 // instead of once per tap.  WGRAD (conv_wgrad_kernel) does the same with voxels as K.
+// Grids too narrow for such tiles are gathered voxel by voxel (conv_gather_kernel).
 // The accumulators live in tensor memory; the epilogues read them with
 // tcgen05.ld (warp w owns lanes 32w..32w+31).  Every mbarrier wait is bounded:
 // on expiry the kernel raises g_conv_error, still waits (bounded) for its own
@@ -39,7 +40,7 @@ namespace {
 constexpr uint32_t BM = 128;
 constexpr uint32_t WAIT_LIMIT = 1u << 21;
 
-enum Mode { FWD = 0, DGRAD = 1 };
+enum Mode { FWD = 0, DGRAD = 1, WGRAD = 2 };
 
 // Poll budget of the pipeline's stage waits for the next launches (see
 // wt_net_set_stage_wait_limit); the drain before tensor memory is freed always
@@ -107,29 +108,6 @@ __device__ __forceinline__ int tap_dx(uint32_t t, uint32_t taps) { return taps =
 // in one MMA (FWD); other odd plane counts, and DGRAD with 8, pair their last plane
 // with a plane of zeros.  Weights come in stages of `ups` MMAs of K through a ring of
 // D stages (cp.async).
-struct RowArgs {
-  const __nv_bfloat16* a;  // FWD x, DGRAD dy
-  const __nv_bfloat16* b;  // FWD w, DGRAD wt: [N][taps][C]
-  const float* bias;
-  void* out;               // FWD bf16 y[M][N], DGRAD f32 dx[M][N]
-  uint32_t C, N, K, taps;  // input channels, output channels, taps * C
-  uint32_t d, h, w, M;     // grid (one batch item) and voxels in all
-  uint32_t hp, dp, rows;   // rows per plane and planes per item with their zero row / plane; rows in all
-  uint32_t cg, planes;     // channel groups; planes in shared memory (the last one zero if cg is odd)
-  uint32_t W, nrows, pitch;  // shared-memory tile: voxels per row, rows, bytes per plane
-  uint32_t halo, run;      // 1 for 27 taps; 1 when the rows are one run
-  uint32_t band0, zstep;   // shared-memory row of tile row 0 for dz = -1, and from one dz to the next
-  uint32_t ctiles;         // tiles along x
-  uint32_t nt, units, ups, upt;  // N per block; MMAs of K; MMAs per stage; MMAs per tap where K is padded per tap, else 0
-  uint32_t depth;            // stages in the weight ring
-  uint32_t cg_magic;       // ceil(2^16 / cg)
-  int relu, vec;           // vec: out is 16-byte aligned and N a multiple of 8
-  uint32_t stage_wait;
-};
-
-// Bytes of the head and of the MMAs' tables.
-__host__ __device__ constexpr uint32_t row_tables(uint32_t units) { return (ROW_HEAD + (units + 3) / 4 * 4 * 12 + 127) / 128 * 128; }
-
 __device__ __forceinline__ void cp16(uint32_t dst, const void* src, bool ok) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16u : 0u) : "memory");
 }
@@ -729,6 +707,272 @@ __global__ void __launch_bounds__(WG_THREADS) conv_wgrad_kernel(WgradArgs p) {
   }
 }
 
+// ---------------------------------------------------------------------------
+// All three gathered voxel by voxel: the grids whose rows fill too little of a tile of
+// numbered rows (one voxel a row: 1 of 8, and a zero row for each where planes have one
+// row), and those whose numbered rows pass 31 bits.  gather_is_cheaper (wt_conv_plan.h)
+// says which.
+//
+// A block: 128 threads, a 128 x N tile (N <= 128).  K runs in slices of 64 through two
+// shared-memory stages: all threads gather a slice of A (128 rows) and B (N rows) into
+// the K-major core-matrix layout (8 rows x 16 bytes; core matrices 128 B apart along K,
+// 1024 B along M/N), one thread issues four MMAs (K = 16 each) and commits them to the
+// stage's mbarrier, and the next slice is gathered into the other stage meanwhile.  What
+// bounds it is that chain, 1.5 us and up a slice.
+constexpr int GA_K = 64, GA_THREADS = 128;
+constexpr uint32_t GA_STAGE = BM * GA_K * 2;          // one operand slice, 16 KB
+constexpr uint32_t GA_SMEM = 4 * GA_STAGE + 64;       // A0 A1 B0 B1, barriers, tensor-memory slot
+constexpr uint32_t GA_COLS = 128;
+
+struct GatherArgs {
+  uint32_t d, h, w;
+  uint32_t cin, cout, taps;
+  uint32_t M, N, K;        // GEMM extents
+  uint32_t k_chunk;        // K per split (WGRAD; a multiple of GA_K), K otherwise
+  const __nv_bfloat16* a;  // FWD x, DGRAD dy, WGRAD x
+  const __nv_bfloat16* b;  // FWD w, DGRAD wt, WGRAD dy
+  const float* bias;
+  void* out;               // FWD bf16 y[M][cout], DGRAD f32 dx[M][cin], WGRAD f32 ws[split][M][N]
+  int relu;
+  uint32_t stage_wait;
+};
+
+// Shared-memory matrix descriptor from byte offsets.
+__device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
+  return (uint64_t)(addr >> 4) | (uint64_t)(lbo >> 4) << 16 | (uint64_t)(sbo >> 4) << 32 | (uint64_t)1 << 46;
+}
+
+// Byte offset of 16-byte chunk (row r, k-group g) in the core-matrix layout.
+__device__ __forceinline__ uint32_t chunk_off(uint32_t r, uint32_t g) { return ((r >> 3) * 8u + g) * 128u + (r & 7u) * 16u; }
+
+__device__ __forceinline__ uint4 ld16(const __nv_bfloat16* p) { return __ldg(reinterpret_cast<const uint4*>(p)); }
+
+// Grid position of a voxel (x fastest, then y, z, batch item).
+struct VoxPos {
+  int x, y, z;
+  int64_t vox;
+  bool ok;
+};
+
+__device__ __forceinline__ VoxPos vox_pos(const GatherArgs& p, uint32_t m, uint32_t end) {
+  VoxPos r;
+  r.ok = m < end;
+  const uint32_t mm = r.ok ? m : 0u;
+  r.x = (int)(mm % p.w);
+  r.y = (int)((mm / p.w) % p.h);
+  r.z = (int)((mm / (p.w * p.h)) % p.d);
+  r.vox = mm;
+  return r;
+}
+
+// Index of the voxel r + (dz, dy, dx) in the same batch item, or -1 outside the grid.
+__device__ __forceinline__ int64_t nbr(const GatherArgs& p, const VoxPos& r, int dz, int dy, int dx) {
+  const int xx = r.x + dx, yy = r.y + dy, zz = r.z + dz;
+  if ((unsigned)xx >= p.w || (unsigned)yy >= p.h || (unsigned)zz >= p.d) return -1;
+  return r.vox + ((int64_t)dz * p.h + dy) * p.w + dx;
+}
+
+// Gather K slice [k0, k0 + 64) of both operands into the stage buffers sa, sb.
+//   FWD / DGRAD: thread t owns A row t (a voxel, position precomputed in `row`)
+//   and B row t (a weight row); each 16-byte chunk is 8 consecutive channels of
+//   one tap, one vector load.
+//   WGRAD: K runs over voxels; thread t owns voxel k0 + (t & 63) and half
+//   (t >> 6) of the A rows (taps x channels) and B rows (output channels); it
+//   loads 8 channels of its voxel with one vector load and stores them into 8
+//   rows of the K-major tile (2-byte stores).
+// Rows past the MMA's N (B) are never read and not written; K past the range
+// is zero in both operands.
+template <int MODE>
+__device__ __forceinline__ void gather(const GatherArgs& p, const VoxPos& row, uint32_t tile_m, uint32_t n_mma,
+                                       uint32_t k0, uint32_t k_end, uint8_t* sa, uint8_t* sb) {
+  const uint32_t t = threadIdx.x;
+  if constexpr (MODE == FWD || MODE == DGRAD) {
+    const uint32_t C = (MODE == FWD) ? p.cin : p.cout;
+    const int sg = (MODE == FWD) ? 1 : -1;
+    uint32_t tap = k0 / C, c = k0 % C;
+#pragma unroll
+    for (uint32_t g = 0; g < 8; g++) {
+      const uint32_t k = k0 + 8 * g;
+      uint4 v = make_uint4(0u, 0u, 0u, 0u);
+      if (row.ok && k < k_end) {
+        const int64_t sv = nbr(p, row, sg * tap_dz(tap, p.taps), sg * tap_dy(tap, p.taps), sg * tap_dx(tap, p.taps));
+        if (sv >= 0) v = ld16(p.a + (size_t)sv * C + c);
+      }
+      *reinterpret_cast<uint4*>(sa + chunk_off(t, g)) = v;
+      c += 8;
+      if (c >= C) {
+        c = 0;
+        tap++;
+      }
+    }
+    if (t < n_mma) {
+#pragma unroll
+      for (uint32_t g = 0; g < 8; g++) {
+        const uint32_t k = k0 + 8 * g;
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (t < p.N && k < k_end) v = ld16(p.b + (size_t)t * p.K + k);
+        *reinterpret_cast<uint4*>(sb + chunk_off(t, g)) = v;
+      }
+    }
+  } else {
+    const uint32_t j = t & 63u, half = t >> 6;
+    const VoxPos m = vox_pos(p, k0 + j, k_end);
+    const uint32_t jo = (j & 7u) * 2u, jg = j >> 3;
+    // A rows half*64 .. +63 = (tap, ci) rows tile_m + ...
+#pragma unroll
+    for (uint32_t q = 0; q < 8; q++) {
+      const uint32_t r0 = half * 64u + 8u * q, R0 = tile_m + r0;
+      uint4 v = make_uint4(0u, 0u, 0u, 0u);
+      if (m.ok && R0 < p.M) {
+        const uint32_t tap = R0 / p.cin, ci = R0 % p.cin;
+        const int64_t sv = nbr(p, m, tap_dz(tap, p.taps), tap_dy(tap, p.taps), tap_dx(tap, p.taps));
+        if (sv >= 0) v = ld16(p.a + (size_t)sv * p.cin + ci);
+      }
+      const uint32_t w4[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int e = 0; e < 8; e++)
+        *reinterpret_cast<uint16_t*>(sa + chunk_off(r0 + e, jg) + jo) = (uint16_t)(w4[e >> 1] >> ((e & 1) * 16));
+    }
+    // B rows (output channels) half*64 .. +63, only those the MMA reads
+#pragma unroll
+    for (uint32_t q = 0; q < 8; q++) {
+      const uint32_t r0 = half * 64u + 8u * q;
+      if (r0 >= n_mma) break;
+      uint4 v = make_uint4(0u, 0u, 0u, 0u);
+      if (m.ok && r0 < p.N) v = ld16(p.b + (size_t)m.vox * p.cout + r0);
+      const uint32_t w4[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int e = 0; e < 8; e++)
+        *reinterpret_cast<uint16_t*>(sb + chunk_off(r0 + e, jg) + jo) = (uint16_t)(w4[e >> 1] >> ((e & 1) * 16));
+    }
+  }
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(GA_THREADS, 1) conv_gather_kernel(GatherArgs p) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  // stage s: A at smem + s * GA_STAGE, B at smem + (2 + s) * GA_STAGE
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 4 * GA_STAGE);  // [2]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + 4 * GA_STAGE + 16);
+  const uint32_t t = threadIdx.x, warp = t >> 5;
+  const uint32_t tile_m = blockIdx.x * BM;
+  const uint32_t k_begin = blockIdx.y * p.k_chunk;
+  const uint32_t k_end = min(p.K, k_begin + p.k_chunk);
+  const uint32_t nk = (k_end > k_begin) ? (k_end - k_begin + GA_K - 1) / GA_K : 0;
+  const uint32_t n_mma = ((p.N + 15) / 16) * 16;
+  const uint32_t idesc = idesc_bf16(BM, n_mma);
+
+  if (t == 0) {
+    mbar_init(smem_u32(&bars[0]), 1);
+    mbar_init(smem_u32(&bars[1]), 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                 "r"(GA_COLS)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  }
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *tmem_slot;
+
+  const VoxPos row_pos = vox_pos(p, tile_m + t, p.M);  // FWD / DGRAD: this thread's A row (a voxel)
+  bool ok = true;
+  uint32_t issued = 0;  // K slices whose MMAs were issued (uniform across the block)
+  for (uint32_t kt = 0; kt < nk; kt++) {
+    const uint32_t s = kt & 1u;
+    bool w = true;
+    if (kt >= 2) w = mbar_wait(smem_u32(&bars[s]), ((kt >> 1) - 1) & 1u, p.stage_wait);  // MMAs of slice kt-2 done
+    if (!__syncthreads_and(w)) {  // the block stops together
+      ok = false;
+      break;
+    }
+    uint8_t* const sa = smem + s * GA_STAGE;
+    uint8_t* const sb = smem + (2u + s) * GA_STAGE;
+    gather<MODE>(p, row_pos, tile_m, n_mma, k_begin + kt * GA_K, k_end, sa, sb);
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncthreads();
+    if (t == 0) {
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint32_t a0 = smem_u32(sa), b0 = smem_u32(sb);
+#pragma unroll
+      for (uint32_t kk = 0; kk < GA_K / 16; kk++) {
+        const uint64_t ad = smem_desc(a0 + kk * 256u, 128u, 1024u);
+        const uint64_t bd = smem_desc(b0 + kk * 256u, 128u, 1024u);
+        const uint32_t acc = (kt > 0 || kk > 0) ? 1u : 0u;
+        asm volatile(
+            "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+            " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
+            "l"(ad), "l"(bd), "r"(idesc), "r"(acc)
+            : "memory");
+      }
+      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                       smem_u32(&bars[s]))
+                   : "memory");
+    }
+    issued++;
+  }
+  // All MMAs done: the last commit covers every earlier one of the issuing thread.
+  if (issued > 0) {
+    const uint32_t last = issued - 1;
+    const bool done = mbar_wait(smem_u32(&bars[last & 1u]), (last >> 1) & 1u, WAIT_LIMIT);
+    ok = ok && done;
+  }
+  if (!ok && t == 0) atomicExch(&g_conv_error, 1);
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+
+  // ---- epilogue: lane = row t of the tile, 16 columns per tcgen05.ld
+  const uint32_t row = tile_m + t;
+  const uint32_t taddr = tmem + ((warp * 32u) << 16);
+  for (uint32_t c0 = 0; c0 < n_mma; c0 += 16) {
+    uint32_t r[16];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr + c0)
+        : "memory");
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+    if (!ok || row >= p.M || nk == 0) continue;
+#pragma unroll
+    for (int j = 0; j < 16; j++) {
+      const uint32_t col = c0 + j;
+      if (col >= p.N) break;
+      float v = __uint_as_float(r[j]);
+      if constexpr (MODE == FWD) {
+        if (p.bias) v += p.bias[col];
+        if (p.relu) v = fmaxf(v, 0.0f);
+        reinterpret_cast<__nv_bfloat16*>(p.out)[(size_t)row * p.N + col] = __float2bfloat16_rn(v);
+      } else if constexpr (MODE == DGRAD) {
+        reinterpret_cast<float*>(p.out)[(size_t)row * p.N + col] = v;
+      } else {
+        reinterpret_cast<float*>(p.out)[((size_t)blockIdx.y * p.M + row) * p.N + col] = v;
+      }
+    }
+  }
+  if (nk == 0 && row < p.M) {  // empty K range: the product is zero
+    for (uint32_t col = 0; col < p.N; col++) {
+      if constexpr (MODE == FWD) {
+        float v = p.bias ? p.bias[col] : 0.0f;
+        if (p.relu) v = fmaxf(v, 0.0f);
+        reinterpret_cast<__nv_bfloat16*>(p.out)[(size_t)row * p.N + col] = __float2bfloat16_rn(v);
+      } else if constexpr (MODE == DGRAD) {
+        reinterpret_cast<float*>(p.out)[(size_t)row * p.N + col] = 0.0f;
+      } else {
+        reinterpret_cast<float*>(p.out)[((size_t)blockIdx.y * p.M + row) * p.N + col] = 0.0f;
+      }
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 0) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(GA_COLS) : "memory");
+  }
+}
+
 // dw[co][t][ci] = sum over splits of ws[split][(t, ci)][co]: a block takes 32
 // outputs, its eight warps every eighth split each (in FP64, folded in order).
 __global__ void wgrad_reduce_kernel(const float* __restrict__ ws, float* __restrict__ dw, uint32_t splits,
@@ -764,10 +1008,26 @@ int check_shape(const wt_conv_shape* s, const char* what) {
   return WT_OK;
 }
 
-// Tiling of conv_rows_kernel.  Wide tiles (xg groups of 8 voxels along x) share
-// their halo and their weights; narrow ones and a split of N give a small grid
-// enough blocks.  Shared memory of a block stays below a third of an SM's where it
-// can, so that several blocks overlap their loads, MMAs and epilogues.
+template <int MODE>
+int launch_gather(const GatherArgs& p, uint32_t splits, cudaStream_t st) {
+  cudaError_t e = cudaFuncSetAttribute(conv_gather_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GA_SMEM);
+  if (e != cudaSuccess) return nfail(WT_ERR_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
+  conv_gather_kernel<MODE><<<dim3((p.M + BM - 1) / BM, splits), GA_THREADS, GA_SMEM, st>>>(p);
+  e = cudaGetLastError();
+  if (e != cudaSuccess) return nfail(WT_ERR_CUDA, std::string("conv kernel launch: ") + cudaGetErrorString(e));
+  return WT_OK;
+}
+
+GatherArgs gather_args(const wt_conv_shape* s, const void* a, const void* b, void* out) {
+  GatherArgs p = {};
+  p.d = s->d, p.h = s->h, p.w = s->w;
+  p.cin = s->cin, p.cout = s->cout, p.taps = s->taps;
+  p.a = static_cast<const __nv_bfloat16*>(a);
+  p.b = static_cast<const __nv_bfloat16*>(b);
+  p.out = out;
+  p.stage_wait = g_stage_wait.load();
+  return p;
+}
 
 template <int MODE, int XG>
 int launch_rows_xg(const RowArgs& p, uint32_t smem, dim3 grid, cudaStream_t st) {
@@ -781,82 +1041,29 @@ int launch_rows_xg(const RowArgs& p, uint32_t smem, dim3 grid, cudaStream_t st) 
 
 template <int MODE>
 int launch_rows(const wt_conv_shape* s, const void* a, const void* b, const float* bias, void* out, int relu, void* stream) {
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
   RowArgs p = {};
+  RowPlan q = {};
+  if (!plan_rows(*s, MODE == FWD, p, q) || gather_is_cheaper(p, q)) {
+    GatherArgs ga = gather_args(s, a, b, out);
+    ga.bias = bias;
+    ga.relu = relu;
+    ga.M = s->batch * s->d * s->h * s->w;
+    ga.N = p.N;
+    ga.K = ga.k_chunk = p.K;
+    return launch_gather<MODE>(ga, 1, st);
+  }
   p.a = static_cast<const __nv_bfloat16*>(a);
   p.b = static_cast<const __nv_bfloat16*>(b);
   p.bias = bias;
   p.out = out;
   p.relu = relu;
-  p.C = MODE == FWD ? s->cin : s->cout;
-  p.N = MODE == FWD ? s->cout : s->cin;
-  p.taps = s->taps;
-  p.K = p.taps * p.C;
-  p.M = s->batch * s->d * s->h * s->w;
   p.stage_wait = g_stage_wait.load();
   p.vec = (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
-  p.halo = s->taps == 27 ? 1u : 0u;
-  uint32_t batch = s->batch;
-  if (p.halo) {
-    p.d = s->d, p.h = s->h, p.w = s->w;
-    p.hp = p.h + 1, p.dp = p.d + 1;
-  } else {  // pointwise: the voxels in rows of 32
-    batch = 1, p.d = 1, p.w = 32, p.h = (p.M + 31) / 32;
-    p.hp = p.h, p.dp = 1;
-  }
-  const uint64_t rows = ((uint64_t)batch * p.dp - p.halo) * p.hp - p.halo;  // up to the last row of the grid
-  if (rows >= (1ull << 31)) return nfail(WT_ERR_ARG, "convolution: grid too large");
-  p.rows = (uint32_t)rows;
-  p.cg = p.C / 8;
-  p.planes = p.cg + (p.cg & 1u);
-  p.cg_magic = (65536u + p.cg - 1) / p.cg;
-  const uint32_t halo_rows = p.halo * (p.hp + 1);
-  p.run = !p.halo || ROW_TILE + 2 * halo_rows <= ROW_ROWS;
-  p.nrows = p.run ? ROW_TILE + 2 * halo_rows : ROW_ROWS;
-  p.band0 = p.halo;  // row -1 of the first band is shared-memory row 0
-  p.zstep = !p.halo ? 0 : p.run ? p.hp : ROW_TILE + 2;
-  if (p.cg & 1u) {
-    p.upt = (p.cg + 1) / 2;
-    if (p.cg == 1 && MODE == FWD && p.h > 1) p.upt = 0;  // (planes of one row: the distance of two taps may be negative)
-  }
-  p.units = p.upt ? p.taps * p.upt : (p.K + 15) / 16;
-  const uint32_t rt = (p.rows + ROW_TILE - 1) / ROW_TILE, groups = (p.w + 7) / 8, n16 = (p.N + 15) / 16 * 16;
-  auto tile = [&](uint32_t xg) {
-    p.W = 8 * xg + 2 * p.halo;
-    p.pitch = p.nrows * p.W * 16;
-    p.pitch = pad_pitch(p.pitch, p.cg);
-    p.ctiles = (groups + xg - 1) / xg;
-  };
-  // Longer stages where K is long: an MMA takes 40-70 cycles to issue, a stage's
-  // waits about 400.  (Fewer than 32 MMAs: 4 to a stage, K slices of 64.)
-  auto stage = [&](uint32_t nt) { return p.units < 32 ? 4u : p.units < 64 || nt > 32 ? 8u : 16u; };
-  auto ring = [&](uint32_t nt) { return 2 * stage(nt) * (nt * 16 + 16); };
-  uint32_t xg = 4;
-  for (; xg > 1; xg >>= 1) {
-    tile(xg);
-    if (xg < 2 * groups && p.planes * p.pitch + 4 * ring(n16) <= (xg == 2 ? SMEM_MAX / 2 : SMEM_THIRD) - 4096 && xg * n16 <= 128 &&
-        (uint64_t)rt * p.ctiles >= 2 * SMS)
-      break;
-  }
-  tile(xg);
-  p.nt = n16;
-  while (p.nt > 16 && ((uint64_t)rt * p.ctiles * ((p.N + p.nt - 1) / p.nt) < SMS ||
-                       row_tables(p.units) + p.planes * p.pitch + 4 * ring(p.nt) > SMEM_MAX))
-    p.nt = (p.nt / 2 + 15) / 16 * 16;
-  p.ups = stage(p.nt);
-  const uint32_t nst = (p.units + p.ups - 1) / p.ups, a_bytes = row_tables(p.units) + p.planes * p.pitch;
-  const dim3 grid(rt * p.ctiles, (p.N + p.nt - 1) / p.nt);
-  // A deep ring hides the weights' latency; it must not cost resident blocks.
-  auto per_sm = [&](uint32_t depth) {
-    const uint32_t fit = SMEM_MAX / (a_bytes + depth * ring(p.nt)), have = (grid.x * grid.y + SMS - 1) / SMS;
-    return fit < have ? fit : have;
-  };
-  p.depth = ROW_DEPTH_MAX;
-  while (p.depth > 4 && (p.depth >= 2 * nst || !per_sm(p.depth) || per_sm(p.depth) < per_sm(4))) p.depth /= 2;
-  const uint32_t smem = a_bytes + p.depth * ring(p.nt);
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (xg == 4) return launch_rows_xg<MODE, 4>(p, smem, grid, st);
-  if (xg == 2) return launch_rows_xg<MODE, 2>(p, smem, grid, st);
-  return launch_rows_xg<MODE, 1>(p, smem, grid, st);
+  const dim3 grid(q.blocks, q.nblocks);
+  if (q.xg == 4) return launch_rows_xg<MODE, 4>(p, q.smem, grid, st);
+  if (q.xg == 2) return launch_rows_xg<MODE, 2>(p, q.smem, grid, st);
+  return launch_rows_xg<MODE, 1>(p, q.smem, grid, st);
 }
 
 int launch_wgrad(const wt_conv_shape* s, const void* x, const void* dy, float* ws, uint32_t splits, cudaStream_t st) {
@@ -866,7 +1073,14 @@ int launch_wgrad(const wt_conv_shape* s, const void* x, const void* dy, float* w
   p.ws = ws;
   p.stage_wait = g_stage_wait.load();
   uint32_t nm = 0, smem = 0;
-  if (!plan_wgrad(*s, splits, p, nm, smem)) return nfail(WT_ERR_ARG, "convolution: grid too large");
+  if (!plan_wgrad(*s, splits, p, nm, smem) || gather_is_cheaper(p, splits)) {
+    GatherArgs ga = gather_args(s, x, dy, ws);
+    ga.M = s->taps * s->cin;
+    ga.N = s->cout;
+    ga.K = s->batch * s->d * s->h * s->w;
+    ga.k_chunk = (uint32_t)p.k_chunk;
+    return launch_gather<WGRAD>(ga, splits, st);
+  }
   const dim3 grid(splits, (p.halo ? (p.dxs == 3 ? 3 : 9) : 1) * p.chunks);
   const auto kernel = nm == 3 ? conv_wgrad_kernel<3> : conv_wgrad_kernel<1>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX);

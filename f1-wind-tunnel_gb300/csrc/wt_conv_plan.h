@@ -12,10 +12,32 @@ namespace wt {
 namespace {
 
 constexpr uint32_t SMS = 152, SMEM_MAX = 227 * 1024, SMEM_THIRD = 74 * 1024;
-
 constexpr uint32_t ROW_TILE = 16, ROW_ROWS = 3 * (ROW_TILE + 2), ROW_HEAD = 512;  // ROW_HEAD: barriers, slot, ROW_ROWS row voxels
 // Threads that load, and with the issuing warp; stages of the weight ring at most.
 constexpr uint32_t ROW_LOADERS = 256, ROW_THREADS = ROW_LOADERS + 32, ROW_DEPTH_MAX = 16;
+
+struct RowArgs {
+  const __nv_bfloat16* a;  // FWD x, DGRAD dy
+  const __nv_bfloat16* b;  // FWD w, DGRAD wt: [N][taps][C]
+  const float* bias;
+  void* out;               // FWD bf16 y[M][N], DGRAD f32 dx[M][N]
+  uint32_t C, N, K, taps;  // input channels, output channels, taps * C
+  uint32_t d, h, w, M;     // grid (one batch item) and voxels in all
+  uint32_t hp, dp, rows;   // rows per plane and planes per item with their zero row / plane; rows in all
+  uint32_t cg, planes;     // channel groups; planes in shared memory (the last one zero if cg is odd)
+  uint32_t W, nrows, pitch;  // shared-memory tile: voxels per row, rows, bytes per plane
+  uint32_t halo, run;      // 1 for 27 taps; 1 when the rows are one run
+  uint32_t band0, zstep;   // shared-memory row of tile row 0 for dz = -1, and from one dz to the next
+  uint32_t ctiles;         // tiles along x
+  uint32_t nt, units, ups, upt;  // N per block; MMAs of K; MMAs per stage; MMAs per tap where K is padded per tap, else 0
+  uint32_t depth;            // stages in the weight ring
+  uint32_t cg_magic;       // ceil(2^16 / cg)
+  int relu, vec;           // vec: out is 16-byte aligned and N a multiple of 8
+  uint32_t stage_wait;
+};
+
+// Bytes of the head and of the MMAs' tables.
+constexpr uint32_t row_tables(uint32_t units) { return (ROW_HEAD + (units + 3) / 4 * 4 * 12 + 127) / 128 * 128; }
 
 struct WgradArgs {
   const __nv_bfloat16 *x, *dy;
@@ -61,14 +83,110 @@ uint32_t pad_pitch(uint32_t bytes, uint32_t cg) {
   return bytes + (want + 128u - bytes % 128u) % 128u;
 }
 
+// What plan_rows settles beside the arguments.
+struct RowPlan {
+  uint32_t xg, blocks, nblocks, smem;  // voxel groups of a tile; blocks along the voxels and along N
+};
+
+// Tiling of conv_rows_kernel.  Wide tiles (xg groups of 8 voxels along x) share
+// their halo and their weights; narrow ones and a split of N give a small grid
+// enough blocks.  Shared memory of a block stays below a third of an SM's where it
+// can, so that several blocks overlap their loads, MMAs and epilogues.
+// False: the numbered rows do not fit 31 bits.
+bool plan_rows(const wt_conv_shape& s, bool forward, RowArgs& p, RowPlan& q) {
+  p.C = forward ? s.cin : s.cout;
+  p.N = forward ? s.cout : s.cin;
+  p.taps = s.taps;
+  p.K = p.taps * p.C;
+  p.M = s.batch * s.d * s.h * s.w;
+  p.halo = s.taps == 27 ? 1u : 0u;
+  uint32_t batch = s.batch;
+  if (p.halo) {
+    p.d = s.d, p.h = s.h, p.w = s.w;
+    p.hp = p.h + 1, p.dp = p.d + 1;
+  } else {  // pointwise: the voxels in rows of 32
+    batch = 1, p.d = 1, p.w = 32, p.h = (p.M + 31) / 32;
+    p.hp = p.h, p.dp = 1;
+  }
+  const uint64_t rows = ((uint64_t)batch * p.dp - p.halo) * p.hp - p.halo;  // up to the last row of the grid
+  if (rows >= (1ull << 31)) return false;
+  p.rows = (uint32_t)rows;
+  p.cg = p.C / 8;
+  p.planes = p.cg + (p.cg & 1u);
+  p.cg_magic = (65536u + p.cg - 1) / p.cg;
+  const uint64_t halo_rows = p.halo * ((uint64_t)p.hp + 1);
+  p.run = !p.halo || ROW_TILE + 2 * halo_rows <= ROW_ROWS;
+  p.nrows = p.run ? ROW_TILE + 2 * (uint32_t)halo_rows : ROW_ROWS;
+  p.band0 = p.halo;  // row -1 of the first band is shared-memory row 0
+  p.zstep = !p.halo ? 0 : p.run ? p.hp : ROW_TILE + 2;
+  if (p.cg & 1u) {
+    p.upt = (p.cg + 1) / 2;
+    if (p.cg == 1 && forward && p.h > 1) p.upt = 0;  // (planes of one row: the distance of two taps may be negative)
+  }
+  p.units = p.upt ? p.taps * p.upt : (p.K + 15) / 16;
+  const uint32_t rt = (p.rows + ROW_TILE - 1) / ROW_TILE, groups = (p.w + 7) / 8, n16 = (p.N + 15) / 16 * 16;
+  auto tile = [&](uint32_t xg) {
+    p.W = 8 * xg + 2 * p.halo;
+    p.pitch = p.nrows * p.W * 16;
+    p.pitch = pad_pitch(p.pitch, p.cg);
+    p.ctiles = (groups + xg - 1) / xg;
+  };
+  // Longer stages where K is long: an MMA takes 40-70 cycles to issue, a stage's
+  // waits about 400.  (Fewer than 32 MMAs: 4 to a stage, K slices of 64.)
+  auto stage = [&](uint32_t nt) { return p.units < 32 ? 4u : p.units < 64 || nt > 32 ? 8u : 16u; };
+  auto ring = [&](uint32_t nt) { return 2 * stage(nt) * (nt * 16 + 16); };
+  uint32_t xg = 4;
+  for (; xg > 1; xg >>= 1) {
+    tile(xg);
+    if (xg < 2 * groups && p.planes * p.pitch + 4 * ring(n16) <= (xg == 2 ? SMEM_MAX / 2 : SMEM_THIRD) - 4096 && xg * n16 <= 128 &&
+        (uint64_t)rt * p.ctiles >= 2 * SMS)
+      break;
+  }
+  tile(xg);
+  p.nt = n16;
+  while (p.nt > 16 && ((uint64_t)rt * p.ctiles * ((p.N + p.nt - 1) / p.nt) < SMS ||
+                       row_tables(p.units) + p.planes * p.pitch + 4 * ring(p.nt) > SMEM_MAX))
+    p.nt = (p.nt / 2 + 15) / 16 * 16;
+  p.ups = stage(p.nt);
+  const uint32_t nst = (p.units + p.ups - 1) / p.ups, a_bytes = row_tables(p.units) + p.planes * p.pitch;
+  q.xg = xg, q.blocks = rt * p.ctiles, q.nblocks = (p.N + p.nt - 1) / p.nt;
+  // A deep ring hides the weights' latency; it must not cost resident blocks.
+  auto per_sm = [&](uint32_t depth) {
+    const uint32_t fit = SMEM_MAX / (a_bytes + depth * ring(p.nt)), have = (q.blocks * q.nblocks + SMS - 1) / SMS;
+    return fit < have ? fit : have;
+  };
+  p.depth = ROW_DEPTH_MAX;
+  while (p.depth > 4 && (p.depth >= 2 * nst || !per_sm(p.depth) || per_sm(p.depth) < per_sm(4))) p.depth /= 2;
+  q.smem = a_bytes + p.depth * ring(p.nt);
+  return true;
+}
+
+// Whether a 3x3x3 call is cheaper gathered voxel by voxel than on numbered rows.  Both
+// times are estimated, in us.  A block of rows costs its weights (read anew by every
+// block), its tile and its MMAs whatever part of the tile the grid fills; a block of 128
+// gathered voxels a chain of K slices of 64, several blocks to an SM overlapping theirs.
+// The constants fit 35 grids of rows of 1 to 40 voxels, from 1x1x1 on, at 512 to 262144
+// voxels and 7 pairs of channels, both measured (rows, gather): 65536 of 1x1x1, 16
+// channels 284 and 33, 128 channels 3705 and 434; 4096 of 1x4x4, 128 channels 623 and
+// 477; 512 of 2x2x2, 64 channels 35 and 84.  The estimate picks the faster one there up
+// to 1 % on average and 45 % at worst.
+bool gather_is_cheaper(const RowArgs& p, const RowPlan& q) {
+  if (!p.halo) return false;  // pointwise voxels are packed
+  const double C = p.C, N = p.N, b = (double)((p.M + 127) / 128) / SMS;
+  const double rows = (double)q.blocks * q.nblocks / SMS * (1.8 + 0.002 * C * p.nt + (0.02 + 0.01 * q.xg) * C);
+  const double gather = (double)((p.K + 63) / 64) * (1.5 + (0.85 + 0.007 * N) * b) + 0.05 * N * b;
+  return rows > gather;
+}
+
 // Tiling of conv_wgrad_kernel.  A block takes all three dx where their accumulators
 // fit the tensor memory (9 cin columns), the splits alone give every SM a block and
 // rows end with a group of 8; otherwise one dx, for a finer grid, and where that
 // still leaves SMs idle, cin in chunks (16 channels at least).  The workspace bounds
-// the splits.  False: the numbered rows do not fit 32 bits.
+// the splits.  False: the numbered rows do not fit 31 bits.
 bool plan_wgrad(const wt_conv_shape& s, uint32_t splits, WgradArgs& p, uint32_t& nm, uint32_t& smem) {
   p.cin = s.cin, p.cout = s.cout, p.taps = s.taps;
   p.M = s.batch * s.d * s.h * s.w;
+  p.k_chunk = (((uint64_t)p.M + splits - 1) / splits + 63) / 64 * 64;
   p.halo = s.taps == 27 ? 1u : 0u;
   uint32_t batch = s.batch;
   if (p.halo) {
@@ -85,7 +203,6 @@ bool plan_wgrad(const wt_conv_shape& s, uint32_t splits, WgradArgs& p, uint32_t&
   p.magy = (65536u + p.cgy - 1) / p.cgy;
   p.groups = (p.w + 7) / 8;
   p.vrows = p.halo ? batch * p.d * p.h : p.h;
-  p.k_chunk = (((uint64_t)p.M + splits - 1) / splits + 63) / 64 * 64;
   p.throttle = p.M / splits > 128 ? 1u : 0u;
   auto r16 = [](uint32_t v) { return (v + 15) / 16 * 16; };
   const uint32_t cg = p.cin / 8, n3 = r16(3 * p.cin);
@@ -133,6 +250,22 @@ bool plan_wgrad(const wt_conv_shape& s, uint32_t splits, WgradArgs& p, uint32_t&
   p.ctiles = (p.groups + p.xg - 1) / p.xg;
   for (p.cols = 32; p.cols < nm * p.n; p.cols *= 2) {}
   return true;
+}
+
+// The weight gradient's.  Both walk the voxels of a split as one chain (tiles of rows,
+// slices of 64 voxels), so the tiles per 128 voxels decide: 5.6 of them while an SM has
+// one block, less the more splits read wide tiles at a time; 4.1 where it has several;
+// 3 where the splits would fill the device with three dx to a block but the row width
+// forbids it.  On the same grids and larger ones (to 1048576 voxels) 1 to 2 % off the
+// faster one on average.  Rows, gather: 4096 of 1x1x1, 64 channels 1176 and 247 us; 1024
+// of 4x4x4, 16 channels 160 and 218; 262144 voxels in 3x3x4, 16 channels 412 and 246.
+bool gather_is_cheaper(const WgradArgs& p, uint32_t splits) {
+  if (!p.halo) return false;
+  const double tiles = (double)((p.rows + ROW_TILE - 1) / ROW_TILE) * p.groups, blocks = (double)((p.M + 127) / 128);
+  const double limit = 9 * splits <= SMS                               ? 5.6 - 5e-6 * p.cin * p.cout * splits
+                       : 3 * splits >= SMS && p.w % 8 && p.cin < 64 ? 3.0
+                                                                     : 4.1;
+  return tiles > limit * blocks;
 }
 
 }  // namespace
