@@ -126,9 +126,9 @@ __device__ __forceinline__ int32_t row_voxel(const RowArgs& p, int64_t R) {
 // the tensor cores.  At most two stages of MMAs are in flight.
 
 // mbar_wait that also ends when the block has been told to stop.
-__device__ __forceinline__ bool mbar_wait_or(uint32_t bar, uint32_t parity, const volatile uint32_t* stop) {
-  if (mbar_wait(bar, parity, 1)) return true;
-  for (uint32_t i = 0; i < WAIT_LIMIT && !*stop; i += 16)
+__device__ __forceinline__ bool mbar_wait_or(uint32_t bar, uint32_t parity, const volatile uint32_t* stop, uint32_t limit = WAIT_LIMIT) {
+  if (limit && mbar_wait(bar, parity, 1)) return true;
+  for (uint32_t i = 0; i < limit && !*stop; i += 16)
     if (mbar_wait(bar, parity, 16)) return true;
   return false;
 }
@@ -487,7 +487,7 @@ __global__ void __launch_bounds__(WG_THREADS) conv_wgrad_kernel(WgradArgs p) {
     asm volatile("{\n .reg .pred q;\n elect.sync _|q, 0xffffffff;\n selp.u32 %0, 1, 0, q;\n}\n" : "=r"(elected));
     uint32_t acc = 0, kt = 0, b = 0, phase = 0, tab = 0, tphase = 0;
     for (bool more = any; more; kt++) {
-      ok = mbar_wait_or(smem_u32(&tfull[tab]), tphase, stop) && mbar_wait_or(smem_u32(&full[b]), phase, stop);
+      ok = mbar_wait_or(smem_u32(&tfull[tab]), tphase, stop) && mbar_wait_or(smem_u32(&full[b]), phase, stop, p.stage_wait);
       if (!__all_sync(0xffffffffu, ok)) {
         ok = false;
         if (elected) *reinterpret_cast<volatile uint32_t*>(stop) = 1u;
@@ -523,7 +523,6 @@ __global__ void __launch_bounds__(WG_THREADS) conv_wgrad_kernel(WgradArgs p) {
     if (elected) *nonzero = acc;
     if (kt > 0) {
       const uint32_t last = smem_u32(&done[b ? b - 1 : p.nbuf - 1]), ph = b ? phase : phase ^ 1u;
-      if (p.throttle) ok = mbar_wait(last, ph, p.stage_wait) && ok;
       ok = mbar_wait(last, ph, WAIT_LIMIT) && ok;  // before the tensor memory is freed, whatever came before
     }
   } else if (warp == ROW_LOADERS / 32 + 1) {
@@ -601,7 +600,7 @@ __global__ void __launch_bounds__(WG_THREADS) conv_wgrad_kernel(WgradArgs p) {
     uint32_t kt = 0, b = 0, phase = 1, tab = 0, tphase = 0;
     for (bool more = any; more; kt++) {
       const uint32_t base = s0 + b * p.buf;
-      ok = mbar_wait_or(smem_u32(&tfull[tab]), tphase, stop) && (kt < p.nbuf || mbar_wait_or(smem_u32(&done[b]), phase, stop));
+      ok = mbar_wait_or(smem_u32(&tfull[tab]), tphase, stop) && (kt < p.nbuf || mbar_wait_or(smem_u32(&done[b]), phase, stop, p.stage_wait));
       if (!ok) {
         *reinterpret_cast<volatile uint32_t*>(stop) = 1u;
         break;
@@ -1071,7 +1070,6 @@ int launch_wgrad(const wt_conv_shape* s, const void* x, const void* dy, float* w
   p.x = static_cast<const __nv_bfloat16*>(x);
   p.dy = static_cast<const __nv_bfloat16*>(dy);
   p.ws = ws;
-  p.stage_wait = g_stage_wait.load();
   uint32_t nm = 0, smem = 0;
   if (!plan_wgrad(*s, splits, p, nm, smem) || gather_is_cheaper(p, splits)) {
     GatherArgs ga = gather_args(s, x, dy, ws);
@@ -1081,6 +1079,7 @@ int launch_wgrad(const wt_conv_shape* s, const void* x, const void* dy, float* w
     ga.k_chunk = (uint32_t)p.k_chunk;
     return launch_gather<WGRAD>(ga, splits, st);
   }
+  p.stage_wait = p.M / splits > 128 ? g_stage_wait.load() : WAIT_LIMIT;  // up to two K slices of 64 voxels: no stage to wait for
   const dim3 grid(splits, (p.halo ? (p.dxs == 3 ? 3 : 9) : 1) * p.chunks);
   const auto kernel = nm == 3 ? conv_wgrad_kernel<3> : conv_wgrad_kernel<1>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX);

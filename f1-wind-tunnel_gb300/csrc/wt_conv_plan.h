@@ -59,7 +59,7 @@ struct WgradArgs {
   uint32_t dxs;            // dx per block: 3, or 1 (one also splits cin into chunks)
   uint32_t m, n, bstep;    // M and N of one MMA; bytes between the x operands of an MMA and the next of its K step
   uint32_t cols;           // tensor-memory columns
-  uint32_t stage_wait, throttle;  // throttle: more than two K slices of 64 voxels
+  uint32_t stage_wait;     // polls of the waits for a tile and for its buffer
 };
 
 constexpr uint32_t WG_STEPS = 32, WG_BUFS = 4, WG_TABLES = WG_BUFS + 2;  // K steps of a tile
@@ -203,7 +203,6 @@ bool plan_wgrad(const wt_conv_shape& s, uint32_t splits, WgradArgs& p, uint32_t&
   p.magy = (65536u + p.cgy - 1) / p.cgy;
   p.groups = (p.w + 7) / 8;
   p.vrows = p.halo ? batch * p.d * p.h : p.h;
-  p.throttle = p.M / splits > 128 ? 1u : 0u;
   auto r16 = [](uint32_t v) { return (v + 15) / 16 * 16; };
   const uint32_t cg = p.cin / 8, n3 = r16(3 * p.cin);
   uint32_t blocks = splits * (p.halo ? 9 : 1);

@@ -85,9 +85,10 @@ const char* wt_net_last_error(void);
  * convolution pipeline makes before it gives up (default 2^21), for the
  * launches that follow; returns the previous value.  0 makes every stage wait
  * give up at once, so a convolution with more than two K slices leaves its K
- * loop, reports the expiry through wt_net_check and writes no output.  The
- * wait for the issued MMAs before tensor memory is freed always keeps its full
- * limit.  Not for production use; restore the returned value afterwards. */
+ * loop, reports the expiry through wt_net_check and writes no output (the weight
+ * gradient is then formed from what its workspace held).  The wait for the issued
+ * MMAs before tensor memory is freed always keeps its full limit.  Not for production
+ * use; restore the returned value afterwards. */
 uint32_t wt_net_set_stage_wait_limit(uint32_t polls);
 
 #ifdef __cplusplus
