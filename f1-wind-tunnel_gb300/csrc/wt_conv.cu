@@ -434,7 +434,7 @@ __global__ void __launch_bounds__(WG_THREADS) conv_wgrad_kernel(WgradArgs p) {
   uint32_t* const nonzero = tmem_slot + 2;  // 0: no row of the grid in this block's tiles, the accumulators are unset
   WgTile* const tile = reinterpret_cast<WgTile*>(smem + 256);  // [WG_TABLES]
   const uint32_t s0 = smem_u32(smem) + WG_HEAD;
-  const uint32_t zero = s0 + p.nbuf * p.buf;  // a zero row of the gradient tile
+  const uint32_t zero = s0 + p.nbuf * p.buf;  // a zero row of the gradient tile, and three of the x tile
   const uint32_t t = threadIdx.x, warp = __shfl_sync(0xffffffffu, t >> 5, 0), lane = t & 31u;
   const uint32_t split = blockIdx.x, tg = blockIdx.y / p.chunks, g0 = (blockIdx.y - tg * p.chunks) * p.cgx;
   const int dz = p.halo ? (int)(p.dxs == 3 ? tg : tg / 3u) - 1 : 0;
@@ -471,7 +471,7 @@ __global__ void __launch_bounds__(WG_THREADS) conv_wgrad_kernel(WgradArgs p) {
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   } else if (warp < ROW_LOADERS / 32) {
-    for (uint32_t i = t * 16u; i < rpy; i += ROW_LOADERS * 16u)
+    for (uint32_t i = t * 16u; i < p.zbytes; i += ROW_LOADERS * 16u)
       *reinterpret_cast<uint4*>(smem + WG_HEAD + p.nbuf * p.buf + i) = make_uint4(0u, 0u, 0u, 0u);
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
@@ -561,7 +561,9 @@ __global__ void __launch_bounds__(WG_THREADS) conv_wgrad_kernel(WgradArgs p) {
         uint32_t ra, ga, rb, gb;
         place(u, ra, ga);
         const uint32_t aa = base + ra * rpy + ga * 128u, xa = base + p.xofs + ra * rpx + ga * 128u + (p.halo ? dx0 * 16u : 0u);
-        uint32_t la = zero - aa, lx = 0u;  // zeros against the same x (whose own products are in the first half)
+        // half a step: zeros against zeros (against another x, an infinity would give a NaN): the voxels past
+        // the grid in the same row where the tile has a group of them, else the zero rows
+        uint32_t la = zero - aa, lx = p.dxs == 1 && ng < p.xg ? 144u - 16u * dx0 : zero + rpy - xa;
         if (u + 1 < units) {
           place(u + 1, rb, gb);
           la = (rb - ra) * rpy + gb * 128u - ga * 128u;

@@ -60,6 +60,7 @@ struct WgradArgs {
   uint32_t m, n, bstep;    // M and N of one MMA; bytes between the x operands of an MMA and the next of its K step
   uint32_t cols;           // tensor-memory columns
   uint32_t stage_wait;     // polls of the waits for a tile and for its buffer
+  uint32_t zbytes;         // the zero rows: one of the gradient's tile and, where half a K step may need them, three of the x tile's
 };
 
 constexpr uint32_t WG_STEPS = 32, WG_BUFS = 4, WG_TABLES = WG_BUFS + 2;  // K steps of a tile
@@ -226,8 +227,8 @@ bool plan_wgrad(const wt_conv_shape& s, uint32_t splits, WgradArgs& p, uint32_t&
   // bits as those of a plain walk over the voxels (a training run amplifies the last bit:
   // Adam's first steps divide gradients by themselves).  There the tile's rows shrink
   // until it fits, elsewhere its groups.  A tile of one group that is over a half SM is
-  // taken all the same; 112 channels and more on both sides are over the whole of it
-  // (16 rows: 232576 to 241792 bytes) and take fewer rows.
+  // taken all the same; 104 channels and more on both sides are over the whole of it
+  // and take 14 rows.
   const bool eight = p.groups == 8 && p.w % 8 == 0, whole = eight || (p.groups <= 4 && p.w % 8 == 0);
   for (p.xg = eight ? 8 : p.groups >= 3 ? 4 : p.groups, p.rt = eight ? 8 : ROW_TILE; ;) {
     p.xrows = p.rt + 2 * p.halo;
@@ -236,13 +237,17 @@ bool plan_wgrad(const wt_conv_shape& s, uint32_t splits, WgradArgs& p, uint32_t&
     p.gpy = pad_pitch(8 * p.xg * 16, p.cgy);
     p.xofs = p.rt * p.cgy * p.gpy;
     p.buf = (p.xofs + p.xrows * p.cgx * p.gpx + 127) / 128 * 128;
-    // after the buffers: the zero row, and what the junk M rows and N columns of the last rows read
-    const uint32_t rest = WG_HEAD + 16 * p.gpy + 16 * p.gpx + 2048, most = blocks > SMS ? SMEM_MAX / 2 : SMEM_MAX;
+    const uint32_t zrows = p.xg & 1u || (p.dxs == 3 && p.groups & 1u) ? 3 : 0;
+    // after the buffers: the zero rows, and what the junk M rows and N columns of the last rows read
+    const uint32_t zeros = (p.cgy * p.gpy + (zrows * p.cgx + 1) * p.gpx + 256 + 127) / 128 * 128, junk = 16 * p.gpy + 16 * p.gpx + 2048;
+    const uint32_t rest = WG_HEAD + (zeros > junk ? zeros : junk), most = blocks > SMS ? SMEM_MAX / 2 : SMEM_MAX;
+    p.zbytes = p.cgy * p.gpy + zrows * p.cgx * p.gpx;
     for (p.nbuf = WG_BUFS; p.nbuf > 2 && rest + p.nbuf * p.buf > most; p.nbuf--) {}
     smem = rest + p.nbuf * p.buf;
     if (smem <= most || (p.xg == 1 && smem <= SMEM_MAX && (!whole || p.rt == 4))) break;
-    if ((whole || p.xg == 1) && p.rt > 4) p.rt /= 2;
+    if (whole && p.rt > 4) p.rt /= 2;
     else if (p.xg > 1) p.xg /= 2, p.rt = ROW_TILE;
+    else if (p.rt > 4) p.rt -= 2;
     else break;
   }
   p.bstep = p.dxs == 3 ? 16u : p.cgx * p.gpx;
