@@ -75,23 +75,24 @@ int restore_state(wt_ctx* c, Saved& sv) {
   return WT_OK;
 }
 
-// ms per LBM step of `step(n)` on stream s (events around `reps` calls of 16 steps)
+// ms per LBM step of `step(n)` on stream s (events around three calls of 16 steps).  A
+// sequence is launched directly the first time, captured the second and replayed from
+// then on, which is how a running program has it: two calls go ahead.
 template <class Step>
 float time_steps(cudaStream_t s, Step&& step) {
-  cudaEvent_t a, b;
-  cudaEventCreate(&a);
-  cudaEventCreate(&b);
-  if (step(2) != WT_OK) return -1.0f;  // capture + warm
-  cudaEventRecord(a, s);
-  for (int r = 0; r < 3; r++)
-    if (step(16) != WT_OK) return -1.0f;
-  cudaEventRecord(b, s);
-  cudaEventSynchronize(b);
-  float ms = 0.0f;
-  cudaEventElapsedTime(&ms, a, b);
-  cudaEventDestroy(a);
-  cudaEventDestroy(b);
-  return ms / 48.0f;
+  cudaEvent_t a = nullptr, b = nullptr;
+  float ms = -1.0f;
+  if (cudaEventCreate(&a) == cudaSuccess && cudaEventCreate(&b) == cudaSuccess && step(16) == WT_OK && step(16) == WT_OK) {
+    bool ok = cudaEventRecord(a, s) == cudaSuccess;
+    for (int r = 0; r < 3; r++) ok = ok && step(16) == WT_OK;
+    float t = 0.0f;
+    if (ok && cudaEventRecord(b, s) == cudaSuccess && cudaEventSynchronize(b) == cudaSuccess &&
+        cudaEventElapsedTime(&t, a, b) == cudaSuccess)
+      ms = t / 48.0f;
+  }
+  if (a) cudaEventDestroy(a);
+  if (b) cudaEventDestroy(b);
+  return ms;
 }
 
 }  // namespace
@@ -108,7 +109,11 @@ int wt_tune(wt_ctx* c, uint32_t* bx_out, uint32_t* by_out, float* ms_out) {
   uint32_t bbx = c->bx, bby = c->by;
   for (auto& sh : kShapes) {
     if ((rc = set_geometry(c, sh[0], sh[1]))) return rc;
-    const float ms = time_steps(c->stream, [&](int n) { return wt_step(c, n, 0, 0.0f); });
+    const float ms = time_steps(c->stream, [&](int n) {
+      c->pending = 0;  // every call the same sequence; the trial steps' records are not kept
+      c->mass_pending = false;
+      return wt_step(c, n, 0, 0.0f);
+    });
     if (ms > 0.0f && ms < best) {
       best = ms;
       bbx = c->bx;
