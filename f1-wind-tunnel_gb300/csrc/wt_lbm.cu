@@ -1027,9 +1027,10 @@ __global__ void resample_kernel(const float4* coarse, uint32_t cx, uint32_t cy, 
 // (the FP64 rate is 1/64 of FP32's), so the sums are 64-bit integers on a scale that each
 // coarse cell takes from its own largest magnitude, per component: a first pass over the
 // cell finds it, the second reads the same lines from L1.  A box of up to COARSE_EXACT
-// cells keeps 50 bits below that maximum in every term, which is as close as an FP64 sum
-// of as many terms comes; larger boxes, and boxes with an infinity or a NaN, are summed
-// in FP64.  64x24x20 boxes: of 232x68x52 45 -> 19 us, of 512x192x160 326 -> 185
+// cells keeps every term to a unit of 2^-48 (4096 cells), 2^-49 (2048 and more) or less of
+// that maximum, 62 bits in all, far below the rounding of the average to 32 bits; larger
+// boxes, and boxes with an infinity or a NaN, are summed in FP64.
+// 64x24x20 boxes: of 232x68x52 45 -> 19 us, of 512x192x160 326 -> 185
 // (315 MB read twice, the second time from L1 and L2).
 constexpr uint32_t COARSE_EXACT = 4096;
 
