@@ -15,6 +15,7 @@
 #include "wt_fieldfn.cuh"
 #include "wt_fields.h"
 #include "wt_fmath.h"
+#include "wt_lattice.cuh"
 
 namespace wt {
 namespace {
@@ -105,22 +106,6 @@ __device__ V3 seed_of(const StreamArgs& st, uint32_t line) {
   const float fz = ((float)col + 0.5f) / (float)st.cols;
   return v3(st.smin[0], wmix(st.smin[1], st.smax[1], fy), wmix(st.smin[2], st.smax[2], fz));
 }
-
-// a / b, correctly rounded, from r = RN(1 / b) by Markstein's correction (see
-// div_rcp in wt_lattice.cuh) for b in [2^-20, 2^20] and a = 0 or |a| in [2^-60, 2^60);
-// other operands (`fast` false, or a outside) take the division itself.  The built-in
-// division leaves its short path for a zero numerator too, and the temperatures and
-// the cross velocities of undisturbed air are zeros: 400 cycles instead of 20.
-__device__ __noinline__ float div_slow(float a, float b) { return __fdiv_rn(a, b); }
-__device__ __forceinline__ float div_known(float a, float b, float r, bool fast) {
-  const uint32_t m = __float_as_uint(a) & 0x7fffffffu;
-  float q = __fmul_rn(a, r);
-  const float c = __fmaf_rn(__fmaf_rn(-q, b, a), r, q);
-  q = m ? c : q;
-  if (!fast || (m - 0x21800000u >= 0x5d800000u - 0x21800000u && m != 0u)) q = div_slow(a, b);
-  return q;
-}
-__device__ __forceinline__ bool div_range(float b) { return b >= 0x1p-20f && b <= 0x1p20f; }
 
 // The velocity and fluid weight of sampleFlow (wgsl.ts:332-357) by one warp at one
 // point.  Lane 4 k + c stands for corner k and, with c < 3, axis and component c: it

@@ -66,6 +66,21 @@ __device__ __forceinline__ float div_rcp(float a, float b, float r) {
   return __fmaf_rn(__fmaf_rn(-q, b, a), r, q);
 }
 
+// The same for every operand: by the correction for b in [2^-20, 2^20] and a = 0 or
+// |a| in [2^-60, 2^60); others (`fast` false, or a outside) take the division itself.  The built-in
+// division leaves its short path for a zero numerator too, and the temperatures and
+// the cross velocities of undisturbed air are zeros: 400 cycles instead of 20.
+static __device__ __noinline__ float div_slow(float a, float b) { return __fdiv_rn(a, b); }
+__device__ __forceinline__ float div_known(float a, float b, float r, bool fast) {
+  const uint32_t m = __float_as_uint(a) & 0x7fffffffu;
+  float q = __fmul_rn(a, r);
+  const float c = __fmaf_rn(__fmaf_rn(-q, b, a), r, q);
+  q = m ? c : q;
+  if (!fast || (m - 0x21800000u >= 0x5d800000u - 0x21800000u && m != 0u)) q = div_slow(a, b);
+  return q;
+}
+__device__ __forceinline__ bool div_range(float b) { return b >= 0x1p-20f && b <= 0x1p20f; }
+
 // Population storage.  F32 keeps f_i; F16/BF16 keep f_i - w_i, which is small
 // and keeps the significant bits of the deviation from rest.
 struct StoreF32 {
