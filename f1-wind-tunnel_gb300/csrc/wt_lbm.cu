@@ -1145,6 +1145,32 @@ __global__ void __launch_bounds__(128) coarse_average_kernel(const float4* __res
   reinterpret_cast<float*>(coarse)[4 * (size_t)i + lane] = r;
 }
 
+// The same for small boxes, a thread to each: the lanes of the kernel above would share
+// out a few cells and its fixed part be all of the time.
+__global__ void coarse_average_small_kernel(const float4* __restrict__ fields, const uint32_t* __restrict__ cellw,
+                                            uint32_t nx, uint32_t ny, uint32_t nz, float4* __restrict__ coarse,
+                                            uint32_t cx, uint32_t cy, uint32_t cz) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= cx * cy * cz) return;
+  const uint32_t a = i % cx, b = (i / cx) % cy, c = i / (cx * cy);
+  const uint32_t x0 = (uint32_t)((uint64_t)a * nx / cx), x1 = (uint32_t)((uint64_t)(a + 1) * nx / cx);
+  const uint32_t y0 = (uint32_t)((uint64_t)b * ny / cy), y1 = (uint32_t)((uint64_t)(b + 1) * ny / cy);
+  const uint32_t z0 = (uint32_t)((uint64_t)c * nz / cz), z1 = (uint32_t)((uint64_t)(c + 1) * nz / cz);
+  double sx = 0.0, sy = 0.0, sz = 0.0, sr = 0.0;
+  uint32_t cnt = 0;
+  for (uint32_t z = z0; z < z1; z++)
+    for (uint32_t y = y0; y < y1; y++)
+      for (uint32_t x = x0; x < x1; x++) {
+        const uint32_t idx = x + nx * (y + ny * z);
+        if (cellw[idx] & CW_SOLID) continue;
+        const float4 f = fields[idx];
+        sx += f.x; sy += f.y; sz += f.z; sr += f.w;
+        cnt++;
+      }
+  coarse[i] = cnt ? make_float4((float)(sx / cnt), (float)(sy / cnt), (float)(sz / cnt), (float)(sr / cnt))
+                  : make_float4(0.0f, 0.0f, 0.0f, 1.0f);
+}
+
 constexpr uint32_t RED_THREADS = 256;
 constexpr uint32_t RED_FCHUNKS = WT_RED_FCHUNKS, RED_MCHUNKS = WT_RED_MCHUNKS;
 
@@ -1542,11 +1568,19 @@ cudaError_t launch_coarse_average(const float4* fields, const uint32_t* cellw, u
   const uint32_t n = cx * cy * cz;
   // A warp's fixed part (the box's limits, one FP64 division) is worth 64 or so cells, so
   // small boxes share a warp; above 256 cells the loads of 8 lanes are too few in
-  // flight: 67 cells a box 19 us with 8 lanes, 49 with 32; 512 cells 235 and 185; 15360 cells 3530 and 1065.
-  const bool wide = (uint64_t)nx * ny * nz > (uint64_t)n * 256;
-  const uint32_t per = wide ? 4 : 16;
-  auto k = wide ? coarse_average_kernel<32> : coarse_average_kernel<8>;
-  k<<<(n + per - 1) / per, 128, 0, s>>>(fields, cellw, nx, ny, nz, coarse, cx, cy, cz);
+  // flight: 67 cells a box 19 us with 8 lanes, 49 with 32; 512 cells 235 and 185; 15360
+  // cells 3530 and 1065.  Below 10 cells a thread to a box is faster (512x192x160 with the
+  // copy to the host: 4 cells 1273 us, with 8 lanes 1982; 8 cells 805 and 1058; 12 cells
+  // 814 and 766).
+  const uint64_t cells = (uint64_t)nx * ny * nz;
+  if (cells < (uint64_t)n * 10) {
+    coarse_average_small_kernel<<<(n + 127) / 128, 128, 0, s>>>(fields, cellw, nx, ny, nz, coarse, cx, cy, cz);
+  } else {
+    const bool wide = cells > (uint64_t)n * 256;
+    const uint32_t per = wide ? 4 : 16;
+    auto k = wide ? coarse_average_kernel<32> : coarse_average_kernel<8>;
+    k<<<(n + per - 1) / per, 128, 0, s>>>(fields, cellw, nx, ny, nz, coarse, cx, cy, cz);
+  }
   return cudaGetLastError();
 }
 

@@ -1,6 +1,6 @@
 """The coarse box average at the edges of its integer sums, against exact means: boxes of
 2048, 4095, 4096 and more cells (the largest that are summed in integers, and the first in
-FP64), values over 60 binades of both signs, and infinities and NaN, whose boxes are
+FP64) and of fewer than ten (a thread to each), values over 60 binades of both signs, and infinities and NaN, whose boxes are
 summed in FP64 beside boxes of the same warp that are not."""
 import math
 
@@ -30,7 +30,7 @@ def averages(dims, coarse, fields, solid):
 
 @pytest.mark.parametrize("dims,coarse", [
     ((32, 8, 8), (1, 1, 1)), ((65, 9, 7), (1, 1, 1)), ((32, 16, 8), (1, 1, 1)), ((683, 3, 2), (1, 1, 1)),
-    ((96, 32, 8), (3, 2, 1)), ((40, 12, 9), (10, 4, 3)),
+    ((96, 32, 8), (3, 2, 1)), ((40, 12, 9), (10, 4, 3)), ((40, 12, 9), (20, 6, 9)), ((41, 13, 9), (41, 7, 3)),
 ])
 @pytest.mark.parametrize("spread", [0, 60])
 def test_means(wt_lib, dims, coarse, spread):
@@ -48,9 +48,9 @@ def test_means(wt_lib, dims, coarse, spread):
             assert abs(got[at][k] - ref) <= 2.0 ** -24 * abs(ref) + max(2.0 ** -48, len(cells) * 2.0 ** -53) * top
 
 
-@pytest.mark.parametrize("dims,coarse", [((40, 12, 9), (10, 4, 3)), ((96, 32, 24), (3, 2, 3))])
+@pytest.mark.parametrize("dims,coarse", [((40, 12, 9), (10, 4, 3)), ((96, 32, 24), (3, 2, 3)), ((40, 12, 9), (10, 12, 9))])
 def test_infinities_and_nan(wt_lib, dims, coarse):
-    """Eight and 32 lanes to a box; some boxes of every warp hold a special value."""
+    """Eight and 32 lanes to a box, and one; some boxes of every warp hold a special value."""
     rng = np.random.default_rng(3)
     nx, ny, nz = dims
     v = rng.normal(size=(nz, ny, nx, 4)).astype(np.float32)
