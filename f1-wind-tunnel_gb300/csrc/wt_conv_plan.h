@@ -226,7 +226,10 @@ bool plan_wgrad(const wt_conv_shape& s, uint32_t splits, WgradArgs& p, uint32_t&
   // voxels that follow one another in the grid, in their order, and the sums the same
   // bits as those of a plain walk over the voxels (a training run amplifies the last bit:
   // Adam's first steps divide gradients by themselves).  There the tile's rows shrink
-  // until it fits, elsewhere its groups.  A tile of one group that is over a half SM is
+  // until it fits, elsewhere its groups.  (Rows of 5 to 7 groups would fit the tables too:
+  // whole, 16x24x24 rows of 40 to 56 took 310 to 400 us instead of 397 to 523 with 64
+  // channels and 779 to 1002 instead of 529 to 699 with 128 to 64, and were not equal in
+  // their bits where the tile's rows had to shrink.)  A tile of one group that is over a half SM is
   // taken all the same; 104 channels and more on both sides are over the whole of it
   // and take 14 rows.
   const bool eight = p.groups == 8 && p.w % 8 == 0, whole = eight || (p.groups <= 4 && p.w % 8 == 0);
