@@ -621,7 +621,7 @@ __device__ __forceinline__ void step_tile(const StepArgs& a, const Ofs& ofs, For
     // ---------------------------------------------------------------- forces
     // Blocks with force links and face rows set the latency of a step: a lattice of any
     // size waited 6 us for the links' dependent flag loads and the FP64 trees of all
-    // nine sums, and 3 us for the faces' serial loads.  Group in the cell word, trees per
+    // nine sums, and 3 us for the faces' serial loads.  Group in the cell word, sums per
     // group present and loads ahead of the boundary cases: 168x50x38 f32 18.5 -> 14.1 us
     // a step, 128x48x40 f16 15.6 -> 9.0, 256x96x80 f32 / f16 56.6 / 42.9 -> 53.3 / 37.5,
     // 512x192x160 f16 315 -> 301.
@@ -737,13 +737,14 @@ __device__ __forceinline__ void step_tile(const StepArgs& a, const Ofs& ofs, For
   const int32_t slot = __ldg(a.block_slot + blk);
   if (slot < 0) return;  // no force-carrying link in this block: no barrier, no record
   // The warps' sums: multiples of 2^-54 in 64-bit integers, or (s_fp) the bits of FP64
-  // sums where a cell's force is 2 or more or below 2^-31.
+  // sums where a cell's force is 2 or more (bf16: or below 2^-31).
   __shared__ long long s_i[9][8];
   __shared__ int32_t s_r[6][8];
   __shared__ uint8_t s_fp[3][8];
-  // Per group with a force in this warp (mostly one or none).  Forces from 2^-31 (and
-  // so multiples of 2^-54; those of 16-bit populations near rest can be smaller) to 2
-  // are summed exactly, as three limbs by one reduction instruction each: an
+  // Per group with a force in this warp (mostly one or none).  Forces below 2 are
+  // multiples of 2^-54 (f32 populations give multiples of 2^-29, f16 ones of 2^-37, bf16
+  // ones from 2^-31 on; smaller bf16 forces take the FP64 sums) and are
+  // summed exactly, as three limbs by one reduction instruction each: an
   // FP64 tree of three sums takes fifteen additions at 1/64 of
   // the FP32 rate.  us per step: 128x48x40 f16 9.0 -> 7.9, 168x50x38 f32 14.1 -> 13.5,
   // 256x96x80 f32 53.3 -> 52.2, f16 unchanged from 256x96x80 on.  (Half the shared
@@ -763,9 +764,11 @@ __device__ __forceinline__ void step_tile(const StepArgs& a, const Ofs& ofs, For
       s_r[2 * g][warp] = (int32_t)sx;
       s_r[2 * g + 1][warp] = (int32_t)sy;
     }
-    // magnitudes as bits: below 2, and from 2^-31 on or zero
-    const uint32_t m0 = __float_as_uint(fg[0]) & 0x7fffffffu, m1 = __float_as_uint(fg[1]) & 0x7fffffffu, m2 = __float_as_uint(fg[2]) & 0x7fffffffu;
-    const bool exact = max(max(m0, m1), m2) < 0x40000000u && min(min(m0 - 1u, m1 - 1u), m2 - 1u) >= 0x30000000u - 1u;
+    bool exact = fabsf(fg[0]) < 2.0f && fabsf(fg[1]) < 2.0f && fabsf(fg[2]) < 2.0f;
+    if constexpr (St::id == WT_STORE_BF16) {  // and from 2^-31 on or zero, as bits
+      const uint32_t m0 = __float_as_uint(fg[0]) & 0x7fffffffu, m1 = __float_as_uint(fg[1]) & 0x7fffffffu, m2 = __float_as_uint(fg[2]) & 0x7fffffffu;
+      exact = exact && min(min(m0 - 1u, m1 - 1u), m2 - 1u) >= 0x30000000u - 1u;
+    }
     if (__all_sync(0xffffffffu, exact)) {
 #pragma unroll
       for (int q = 0; q < 3; q++) {
