@@ -150,10 +150,11 @@ __device__ __noinline__ float sd_ellipsoid(const float4* q, V3 pw) {
   const float k1 = len3(v3(dv(p.x, q2.x), dv(p.y, q2.y), dv(p.z, q2.z)));
   return dv(k0 * (k0 - 1.0f), mx(k1, 1e-5f));
 }
-__device__ __noinline__ float sd_cyl_z(V3 p, float r, float hz) {
+__device__ float sd_cyl_z(V3 p, float r, float hz) {
   const float dx = len2(v2(p.x, p.y)) - r, dz = ab(p.z) - hz;
   return mn(mx(dx, dz), 0.0f) + len2(v2(mx(dx, 0.0f), mx(dz, 0.0f)));
 }
+__device__ __noinline__ float sd_cyl(V3 p, float r, float hz) { return sd_cyl_z(p, r, hz); }
 __device__ __noinline__ float sd_wing_z(const float4* q, V3 p) {
   const float4 q0 = q[0], q1 = q[1], q2 = q[2];
   const float z1 = q1.z, rise = q1.w;
@@ -315,9 +316,9 @@ __device__ V2 sd_f1(const Scene& S, V3 pw) {
     const float hw = w ? RHW26 : FHW26, inboard = w ? 0.08f : 0.10f;
     res = op_u(res, v2(sd_tyre(pworld, c, hw), 2.0f));
     const V3 q = pworld - c;
-    const float cover = mn(sd_cyl_z(q, 0.234f, hw - 0.028f), sd_cyl_z(q - v3(0.0f, 0.0f, hw - 0.02f), 0.045f, 0.02f));
+    const float cover = mn(sd_cyl(q, 0.234f, hw - 0.028f), sd_cyl(q - v3(0.0f, 0.0f, hw - 0.02f), 0.045f, 0.02f));
     res = op_u(res, v2(cover, 9.0f));
-    const float duct = sd_cyl_z(pworld - v3(c.x, c.y, c.z - hw - inboard * 0.5f), 0.17f, inboard * 0.5f);
+    const float duct = sd_cyl(pworld - v3(c.x, c.y, c.z - hw - inboard * 0.5f), 0.17f, inboard * 0.5f);
     res = op_u(res, v2(mn(duct, sd_rb(F.box[B_DUCT + w], pworld)), 10.0f));
   }
   return res;
