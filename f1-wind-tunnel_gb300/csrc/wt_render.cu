@@ -50,7 +50,8 @@ __device__ __forceinline__ ushort4 pack(float r, float g, float b, float a) {
 // tables and without the parts that cannot matter (wt_scene.cuh), 1280x720 of the F1:
 // 3.15 -> 1.81 ms; issue slots used 15 -> 27 %, instruction cache hits 51 -> 76 %.
 template <bool MESH>
-__global__ void __launch_bounds__(64, 16) scene_kernel(const __grid_constant__ Scene S, const SceneArgs a) {
+__global__ void __launch_bounds__(64, 16) scene_kernel(const __grid_constant__ SceneParam P, const SceneArgs a) {
+  const Scene S = scene_of(P);
   const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t y = blockIdx.y * blockDim.y + threadIdx.y;
   if (x >= a.w || y >= a.h) return;
@@ -397,7 +398,7 @@ dim3 tiles(uint32_t w, uint32_t h, dim3 b) { return dim3((w + b.x - 1) / b.x, (h
 }  // namespace
 
 cudaError_t launch_render_scene(const SceneArgs& a, cudaStream_t s) {
-  const Scene S = make_scene(a.shape, a.car);
+  const SceneParam S = make_scene(a.shape, a.car);
   const dim3 b(8, 8);
   if (a.mesh_mode != 0u) scene_kernel<true><<<tiles(a.w, a.h, b), b, 0, s>>>(S, a);
   else scene_kernel<false><<<tiles(a.w, a.h, b), b, 0, s>>>(S, a);

@@ -49,15 +49,25 @@ struct F1Tables {
   float ep[5];         // front endplate: centre x, y, half x, y, radius
 };
 
-// Shape plus host-computed shape-wide constants.
+// Shape plus host-computed shape-wide constants.  A kernel has them as a copy of its own,
+// as the W17's distance likes them, and the tables in its parameter block (SceneParam).
 struct Scene {
-  F1Tables f1;                // kind 0
+  const F1Tables* f1;         // kind 0; set by the kernel
   wt_shape s;
   CarView car;                // the W17 model (kind 5)
   float rake_c, rake_s;       // cos/sin of the rake angle (f1.ts:37-40)
   float rear_c, rear_s;       // cos/sin of the rear main-plane angle after variant offsets (f1.ts:274)
   float ang_m, ang_f, chord_m, chord_f, rise_m, ep_hx, ep_hy;  // rear-wing variant (f1.ts:260-272)
 };
+struct SceneParam {
+  Scene s;
+  F1Tables f1;
+};
+__host__ __device__ __forceinline__ Scene scene_of(const SceneParam& P) {
+  Scene S = P.s;
+  S.f1 = &P.f1;
+  return S;
+}
 
 constexpr float DEG = 0.017453292f, FA = 1.0f, RA = 4.6f, WR = 0.36f, FWZ = 0.84f, FHW = 0.152f, RWZ = 0.80f,
                 RHW = 0.20f, RA26 = 4.4f, WR26 = 0.355f, FHW26 = 0.14f, RHW26 = 0.1875f, BODY_X = 0.9444444f,
@@ -265,7 +275,7 @@ __device__ float sd_floor(const F1Tables& F, V3 p, float b, float near) {
   return d;
 }
 __device__ V2 sd_f1(const Scene& S, V3 pw) {
-  const F1Tables& F = S.f1;
+  const F1Tables& F = *S.f1;
   const V3 pworld = v3(pw.x, pw.y, ab(pw.z));
   const V3 p = body_frame(S, pworld);
   const float b = S.s.ride_h;
@@ -516,8 +526,7 @@ uint32_t host_variant(float v) {  // u32(v + 0.5), saturating
   return (t == t && t > 0.0f) ? (t >= 4294967296.0f ? 4294967295u : (uint32_t)t) : 0u;
 }
 // The parts of f1.ts:42-320.
-void f1_tables(Scene& S) {
-  F1Tables& F = S.f1;
+void f1_tables(const Scene& S, F1Tables& F) {
   const float b = S.s.ride_h, yw = 0.19f + b * 0.45f, yr = b + 0.80f, ff = S.s.front_flap;
   auto f4 = [](float x, float y, float z, float w) { return make_float4(x, y, z, w); };
   auto at = [&](float x, float y, float z) { return v3(x, b + y, z); };
@@ -687,8 +696,9 @@ void f1_tables(Scene& S) {
 }
 
 // Shape plus its shape-wide constants.
-Scene make_scene(const wt_shape& shape, const CarView& car = CarView{}) {
-  Scene S;
+SceneParam make_scene(const wt_shape& shape, const CarView& car = CarView{}) {
+  SceneParam P;
+  Scene& S = P.s;
   S.s = shape;
   S.car = car;
   // Shape-wide constants, evaluated once (same functions and operation order as per cell).
@@ -709,9 +719,10 @@ Scene make_scene(const wt_shape& shape, const CarView& car = CarView{}) {
   }
   S.rear_c = wtm::cosf(S.ang_m);
   S.rear_s = wtm::sinf(S.ang_m);
-  S.f1 = F1Tables{};
-  if (shape.kind == WT_KIND_F1) f1_tables(S);
-  return S;
+  S.f1 = nullptr;
+  P.f1 = F1Tables{};
+  if (shape.kind == WT_KIND_F1) f1_tables(S, P.f1);
+  return P;
 }
 
 }  // namespace

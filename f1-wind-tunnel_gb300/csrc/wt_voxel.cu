@@ -22,8 +22,9 @@
 namespace wt {
 namespace {
 
-__global__ void voxelize_kernel(const __grid_constant__ Scene S, uint32_t nx, uint32_t ny, uint32_t nz, float ox, float oy, float oz, float h,
+__global__ void voxelize_kernel(const __grid_constant__ SceneParam P, uint32_t nx, uint32_t ny, uint32_t nz, float ox, float oy, float oz, float h,
                                 uint8_t* __restrict__ solid, float* __restrict__ emit) {
+  const Scene S = scene_of(P);
   const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t y = blockIdx.y * blockDim.y + threadIdx.y;
   const uint32_t z = blockIdx.z;
@@ -182,8 +183,9 @@ __global__ void solid_from_u32_kernel(const uint32_t* __restrict__ in, uint8_t* 
 }  // namespace
 
 // Scene distance at the cell centres of `grid` (the first component of sceneSdf).
-__global__ void sdf_sample_kernel(const __grid_constant__ Scene S, uint32_t nx, uint32_t ny, uint32_t nz, float ox, float oy, float oz,
+__global__ void sdf_sample_kernel(const __grid_constant__ SceneParam P, uint32_t nx, uint32_t ny, uint32_t nz, float ox, float oy, float oz,
                                   float h, float* __restrict__ out) {
+  const Scene S = scene_of(P);
   const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t y = blockIdx.y * blockDim.y + threadIdx.y;
   const uint32_t z = blockIdx.z;
@@ -194,7 +196,7 @@ __global__ void sdf_sample_kernel(const __grid_constant__ Scene S, uint32_t nx, 
 
 
 cudaError_t launch_sdf_sample(const wt_shape& shape, const wt_grid& grid, float* out, cudaStream_t s) {
-  const Scene S = make_scene(shape);
+  const SceneParam S = make_scene(shape);
   const dim3 block(32, 4, 1);
   const dim3 g((grid.nx + 31) / 32, (grid.ny + 3) / 4, grid.nz);
   sdf_sample_kernel<<<g, block, 0, s>>>(S, grid.nx, grid.ny, grid.nz, grid.origin[0], grid.origin[1], grid.origin[2],
@@ -204,7 +206,7 @@ cudaError_t launch_sdf_sample(const wt_shape& shape, const wt_grid& grid, float*
 
 cudaError_t launch_voxelize(const wt_shape& shape, const CarView& car, const wt_grid& grid, uint8_t* solid, float* emit,
                             cudaStream_t s) {
-  const Scene S = make_scene(shape, car);
+  const SceneParam S = make_scene(shape, car);
   const dim3 block(32, 4, 1);
   const dim3 g((grid.nx + 31) / 32, (grid.ny + 3) / 4, grid.nz);
   voxelize_kernel<<<g, block, 0, s>>>(S, grid.nx, grid.ny, grid.nz, grid.origin[0], grid.origin[1], grid.origin[2],

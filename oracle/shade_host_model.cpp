@@ -115,7 +115,8 @@ void wthm_render(const void* shape, const void* cam_p, const void* look_p, const
   a.fill_b = f3n(0.6f, 0.35f, 0.7f);
   a.w = w; a.h = hgt;
   a.car = g_car;
-  const Scene S = make_scene(a.shape, g_car);
+  const SceneParam P = make_scene(a.shape, g_car);
+  const Scene S = scene_of(P);
   for (uint32_t y = y0; y < y1 && y < hgt; y++)
     for (uint32_t x = 0; x < w; x++) {
       const float4 c = a.mesh_mode != 0u ? render_pixel<true>(S, a, x, y) : render_pixel<false>(S, a, x, y);
@@ -128,7 +129,8 @@ void wthm_render(const void* shape, const void* cam_p, const void* look_p, const
 void wthm_scene_sdf(const void* shape, const float* pts, uint32_t n, float* out) {
   wt_shape sh;
   memcpy(&sh, shape, sizeof sh);
-  const Scene S = make_scene(sh, g_car);
+  const SceneParam P = make_scene(sh, g_car);
+  const Scene S = scene_of(P);
   for (uint32_t k = 0; k < n; k++) {
     const V2 r = scene_sdf(S, v3(pts[3 * k], pts[3 * k + 1], pts[3 * k + 2]));
     out[2 * k] = r.x;
