@@ -139,7 +139,7 @@ __device__ V2 box_hit(V3 ro, V3 rd, V3 bmin, V3 bmax) {
 // One out-of-line copy of the scene SDF for the whole pass: the ray march,
 // normal, occlusion, shadow and reflection taps all call it, and inlining it
 // at each site multiplies the code past the instruction cache.
-__device__ __noinline__ V2 sdf(const Scene& S, V3 p) { return scene_sdf(S, p); }
+__device__ __noinline__ V2 sdf(const Scene& S, V3 p) { return scene_sdf(S, *S.f1, p); }
 
 
 // march (render-wgsl.ts:68-79)

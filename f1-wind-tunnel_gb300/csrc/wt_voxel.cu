@@ -24,14 +24,14 @@ namespace {
 
 __global__ void voxelize_kernel(const __grid_constant__ SceneParam P, uint32_t nx, uint32_t ny, uint32_t nz, float ox, float oy, float oz, float h,
                                 uint8_t* __restrict__ solid, float* __restrict__ emit) {
-  const Scene S = scene_of(P);
+  const Scene& S = P.s;
   const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t y = blockIdx.y * blockDim.y + threadIdx.y;
   const uint32_t z = blockIdx.z;
   if (x >= nx || y >= ny) return;
   const uint32_t idx = x + nx * (y + ny * z);
   const V3 p = v3(ox + ((float)x + 0.5f) * h, oy + ((float)y + 0.5f) * h, oz + ((float)z + 0.5f) * h);
-  V2 r = scene_sdf(S, p);
+  V2 r = scene_sdf(S, P.f1, p);
   const bool w17 = S.s.kind == WT_KIND_W17 && S.car.body != nullptr;
   // the W17's cooling ducts are carved out of its body (wgsl.ts:313) and marked
   // with emission -1 (wgsl.ts:319-320): the step relaxes the air there
@@ -185,13 +185,12 @@ __global__ void solid_from_u32_kernel(const uint32_t* __restrict__ in, uint8_t* 
 // Scene distance at the cell centres of `grid` (the first component of sceneSdf).
 __global__ void sdf_sample_kernel(const __grid_constant__ SceneParam P, uint32_t nx, uint32_t ny, uint32_t nz, float ox, float oy, float oz,
                                   float h, float* __restrict__ out) {
-  const Scene S = scene_of(P);
   const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t y = blockIdx.y * blockDim.y + threadIdx.y;
   const uint32_t z = blockIdx.z;
   if (x >= nx || y >= ny) return;
   const V3 p = v3(ox + ((float)x + 0.5f) * h, oy + ((float)y + 0.5f) * h, oz + ((float)z + 0.5f) * h);
-  out[x + nx * (y + ny * z)] = scene_sdf(S, p).x;
+  out[x + nx * (y + ny * z)] = scene_sdf(P.s, P.f1, p).x;
 }
 
 

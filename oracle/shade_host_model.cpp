@@ -132,7 +132,7 @@ void wthm_scene_sdf(const void* shape, const float* pts, uint32_t n, float* out)
   const SceneParam P = make_scene(sh, g_car);
   const Scene S = scene_of(P);
   for (uint32_t k = 0; k < n; k++) {
-    const V2 r = scene_sdf(S, v3(pts[3 * k], pts[3 * k + 1], pts[3 * k + 2]));
+    const V2 r = scene_sdf(S, P.f1, v3(pts[3 * k], pts[3 * k + 1], pts[3 * k + 2]));
     out[2 * k] = r.x;
     out[2 * k + 1] = r.y;
   }
